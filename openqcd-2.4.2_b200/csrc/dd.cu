@@ -26,8 +26,10 @@
 // host copy), an all-gather callback moves the reduction partials.  No
 // kernel waits on another rank.
 #include "lib.h"
+#include "pairs.cuh"
 #include <algorithm>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace qcd {
@@ -46,16 +48,15 @@ __global__ void k_dd_pack(Geom g, DDGeom dg, const void *__restrict__ t, const v
   face_site(g, side, f, chunk, s, n, y);
   const spinor<R> v = Store<R>::load_spinor(t, chunk, s, g.vbh);
   vec3<R> a, b;
-  if (side == 0) {
+  if constexpr (sizeof(R) == 4) {
+    using LP = typename std::conditional<L12 != 0, EoTwoRow, EoFull>::type;
+    eo_face_send<LP>(side, v, u, g.vbh, chunk, s, dg.x0off + g.L[0] - 1 == dg.N0 - 1, a, b);
+  } else if (side == 0) {
     dd_proj_fwd<R>(v, a, b);
-    Half<R>::store(dn, F, f, a, b);
   } else {
-    su3<R> uu;
-    if constexpr (L12 != 0) uu = load_link12(u, chunk, 0, s, g.vbh, dg.x0off + g.L[0] - 1 == dg.N0 - 1);
-    else uu = Store<R>::load_link(u, chunk, 0, s, g.vbh);
-    dd_proj_bwd<R>(uu, v, a, b);
-    Half<R>::store(up, F, f, a, b);
+    dd_proj_bwd<R>(Store<R>::load_link(u, chunk, 0, s, g.vbh), v, a, b);
   }
+  Half<R>::store(side == 0 ? dn : up, F, f, a, b);
 }
 
 int dd_exchange(Ctx &c, size_t bytes, cudaStream_t st) {

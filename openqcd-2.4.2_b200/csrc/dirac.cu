@@ -1,7 +1,7 @@
 // Wilson-Dirac operator kernels (full, even/odd pieces, Dwhat) in FP64 and
 // FP32 on the block-major layout of qcd.cuh.
 //
-// One templated kernel covers every operator of the reference's
+// One templated form (FP64: dirac_body, FP32: pair_body) covers every operator of the reference's
 // modules/dirac/Dw_dble.c and modules/dirac/Dw.c.  Per site x of the selected
 // parity it forms
 //     acc  = (A(x) + i mu_x gamma5) s(x)                    if OP_SW
@@ -17,9 +17,11 @@
 //     Dweo  : even,      HOPSUB|ACC        (Dw_dble.c:1705, subtracts from r)
 //     Dwhat : odd HOP|INV into a scratch field, then even SW|HOPSUB
 //                                          (Dw_dble.c:1792)
-// It is a pure gather: each thread reads the spinors of its 8 neighbours and
-// the 8 links that touch its site, and writes only its own site.
+// It is a pure gather: each thread (FP64) or pair of lanes (FP32) reads the
+// spinors of its 8 neighbours and the 8 links that touch its site, and writes
+// only its own site.
 #include "lib.h"
+#include "pairs.cuh"
 #include "tma.cuh"
 #include <algorithm>
 
@@ -63,26 +65,6 @@ __device__ __forceinline__ spinor<double> apply_sw_site_cs(const void *sw, int c
   return out;
 }
 
-// FP64: SW read and output written with the evict-first policy; FP32 as is
-template <typename R> struct DwIO {
-  __device__ __forceinline__ static spinor<R> sw(const void *m, int chunk, int s, int vbh, R mu, const spinor<R> &in) {
-    return apply_sw_site<R>(m, chunk, s, vbh, mu, in);
-  }
-  __device__ __forceinline__ static void store(void *r, int chunk, int s, int vbh, const spinor<R> &v) {
-    Store<R>::store_spinor(r, chunk, s, vbh, v);
-  }
-};
-__device__ __forceinline__ void store_spinor_cs(double2 *base, int chunk, int s, int vbh, const spinor<double> &r);
-template <> struct DwIO<double> {
-  __device__ __forceinline__ static spinor<double> sw(const void *m, int chunk, int s, int vbh, double mu,
-                                                      const spinor<double> &in) {
-    return apply_sw_site_cs(m, chunk, s, vbh, mu, in);
-  }
-  __device__ __forceinline__ static void store(void *r, int chunk, int s, int vbh, const spinor<double> &v) {
-    store_spinor_cs((double2 *)r, chunk, s, vbh, v);
-  }
-};
-
 __device__ __forceinline__ void store_spinor_cs(double2 *base, int chunk, int s, int vbh, const spinor<double> &r) {
   double2 *p = base + (size_t)chunk * 12 * vbh + s;
 #pragma unroll
@@ -96,24 +78,16 @@ __device__ __forceinline__ void store_spinor_cs(double2 *base, int chunk, int s,
 // RHALF / THALF = 1: the output r / the hop field t is a half-field holding
 // only the odd chunks (chunk index counted from the first odd chunk).
 // Resident CTAs per SM asked of the compiler: the FP64 kernel keeps 255
-// registers (more CTAs made it spill and run slower), the FP32 kernel runs
-// 4 CTAs per SM at 128 registers (3 CTAs were 14 % faster than 2 on B200;
-// with the 12-real link reads 4 are 5-7 % faster than 3: Dw 0.3006 against
-// 0.3218 ms at 32^3x64, 1.58 against 1.67 ms at 48^3x96).
+// registers (more CTAs made it spill and run slower).
 #ifndef DW_MINB64
 #define DW_MINB64 1
-#endif
-#ifndef DW_MINB32
-#define DW_MINB32 4
 #endif
 #ifndef DW_UNROLL
 #define DW_UNROLL 4
 #endif
 constexpr int kDwUnroll = DW_UNROLL;
 
-// L12 = 1 (FP32 only): the links are read as 12 reals (load_link12), the
-// time links at x0 = N0-1 with the boundary sign.
-template <typename R, int OPS, int PAR, int RHALF, int THALF, int L12, int DD>
+template <typename R, int OPS, int PAR, int RHALF, int THALF, int DD>
 __device__ __forceinline__ void dirac_body(const Geom &g, const DDGeom &dg, int i, const void *__restrict__ s,
                                            const void *__restrict__ t, void *r, const void *__restrict__ u,
                                            const void *__restrict__ sw, const void *__restrict__ swinv, R mu_e,
@@ -140,7 +114,7 @@ __device__ __forceinline__ void dirac_body(const Geom &g, const DDGeom &dg, int 
   spinor<R> acc;
   if (OPS & OP_SW) {
     spinor<R> in = Store<R>::load_spinor(s, chunk, si, g.vbh);
-    acc = DwIO<R>::sw(sw, chunk, si, g.vbh, p == 0 ? mu_e : mu_o, in);
+    acc = apply_sw_site_cs(sw, chunk, si, g.vbh, p == 0 ? mu_e : mu_o, in);
   } else {
     szero(acc);
   }
@@ -149,39 +123,31 @@ __device__ __forceinline__ void dirac_body(const Geom &g, const DDGeom &dg, int 
     spinor<R> h;
     szero(h);
     if constexpr (DD == 0) {
-      const int x0 = x.n[0] * g.bs[0] + x.y[0];
 #pragma unroll kDwUnroll
       for (int mu = 0; mu < 4; mu++) {
         int c2, s2;
         site_nbr(g, x, mu, +1, c2, s2);
         {
           spinor<R> sp = Store<R>::load_spinor(t, THALF ? c2 - g.nbl : c2, s2, g.vbh);
-          su3<R> uu;
-          if constexpr (L12 != 0) uu = load_link12(u, chunk, mu, si, g.vbh, mu == 0 && x0 == g.L[0] - 1);
-          else uu = Store<R>::load_link(u, chunk, mu, si, g.vbh);
+          const su3<R> uu = Store<R>::load_link(u, chunk, mu, si, g.vbh);
           hop_fwd<R>(mu, uu, sp, h);
         }
         site_nbr(g, x, mu, -1, c2, s2);
         {
           spinor<R> sm = Store<R>::load_spinor(t, THALF ? c2 - g.nbl : c2, s2, g.vbh);
-          su3<R> uu;
-          if constexpr (L12 != 0) uu = load_link12(u, c2, mu, s2, g.vbh, mu == 0 && x0 == 0);
-          else uu = Store<R>::load_link(u, c2, mu, s2, g.vbh);
+          const su3<R> uu = Store<R>::load_link(u, c2, mu, s2, g.vbh);
           hop_bwd<R>(mu, uu, sm, h);
         }
       }
     } else {
-      // domain decomposition: global time coordinate, and the x0-neighbours
-      // across the rank boundary from the faces
-      const int x0 = dg.x0off + x.n[0] * g.bs[0] + x.y[0];
+      // domain decomposition: the x0-neighbours across the rank boundary from
+      // the faces
       const bool up = x.n[0] + 1 == g.nb[0] && x.y[0] + 1 == g.bs[0];
       const bool dn = x.n[0] == 0 && x.y[0] == 0;
 #pragma unroll kDwUnroll
       for (int mu = 0; mu < 4; mu++) {
         int c2, s2;
-        su3<R> uu;
-        if constexpr (L12 != 0) uu = load_link12(u, chunk, mu, si, g.vbh, mu == 0 && x0 == dg.N0 - 1);
-        else uu = Store<R>::load_link(u, chunk, mu, si, g.vbh);
+        const su3<R> uu = Store<R>::load_link(u, chunk, mu, si, g.vbh);
         if (mu == 0 && up) {
           vec3<R> h0, h1;
           Half<R>::load(dg.hup, face_sites(g), face_index_of(g, x.n, x.y), h0, h1);
@@ -198,15 +164,13 @@ __device__ __forceinline__ void dirac_body(const Geom &g, const DDGeom &dg, int 
         } else {
           site_nbr(g, x, mu, -1, c2, s2);
           spinor<R> sm = Store<R>::load_spinor(t, THALF ? c2 - g.nbl : c2, s2, g.vbh);
-          su3<R> ub;
-          if constexpr (L12 != 0) ub = load_link12(u, c2, mu, s2, g.vbh, mu == 0 && x0 == 0);
-          else ub = Store<R>::load_link(u, c2, mu, s2, g.vbh);
+          const su3<R> ub = Store<R>::load_link(u, c2, mu, s2, g.vbh);
           hop_bwd<R>(mu, ub, sm, h);
         }
       }
     }
     sscale<R>(h, (R)-0.5);
-    if (OPS & OP_INV) h = DwIO<R>::sw(swinv, chunk, si, g.vbh, (R)0, h);
+    if (OPS & OP_INV) h = apply_sw_site_cs(swinv, chunk, si, g.vbh, 0.0, h);
     if (OPS & OP_HOP) sadd(acc, h);
     else ssub(acc, h);
   }
@@ -215,36 +179,169 @@ __device__ __forceinline__ void dirac_body(const Geom &g, const DDGeom &dg, int 
   if (OPS & OP_SUB) {   // r = sub - acc (the residual update of a preconditioner)
     spinor<R> v = Store<R>::load_spinor(sub, rchunk, si, g.vbh);
     ssub(v, acc);
-    DwIO<R>::store(r, rchunk, si, g.vbh, v);
+    store_spinor_cs((double2 *)r, rchunk, si, g.vbh, v);
   } else if (OPS & OP_ACC) {
     spinor<R> old = Store<R>::load_spinor_rw(r, rchunk, si, g.vbh);
     sadd(old, acc);
     Store<R>::store_spinor(r, rchunk, si, g.vbh, old);
   } else {
-    DwIO<R>::store(r, rchunk, si, g.vbh, acc);
+    store_spinor_cs((double2 *)r, rchunk, si, g.vbh, acc);
   }
 }
 
 
-// The operator kernels: without domain decomposition the parameter list of
-// the single-GPU kernel stays as it was (a larger one made the compiler
-// spill in the FP32 operator); the DD twin takes the slab's geometry.
-template <typename R, int OPS, int PAR, int RHALF = 0, int THALF = 0, int L12 = 0>
-__global__ void __launch_bounds__(128, sizeof(R) == 8 ? DW_MINB64 : DW_MINB32)
+// ------------------------------------------------------------------------
+// The FP32 operators, two lanes per site (pairs.cuh): a warp takes 16 sites
+// of one parity of a block, warp w of a launch parity w & 1 when both are
+// done.
+//
+// Bound by the latency of the gathers.  Against one thread per site (the same
+// 128 registers and 16 warps per SM) a lane's chain is half as long and its
+// four hops' loads are in flight together: Dw on 32^3x64 335 -> 275 us (5.1
+// TB/s of the 672 algorithmic bytes per site), on 48x24^3 with 6^4 blocks 107.6
+// -> 94.5 us, on 8^4 8.2 -> 4.1 us; five CTAs per SM (96 registers) 312 and
+// 98.8 us, six (80) 294 and 94.3 us.
+#ifndef DW_MINB32
+#define DW_MINB32 4
+#endif
+template <int OPS, int PAR, class LP, int DD>
+__device__ __forceinline__ void pair_body(const Geom &g, const DDGeom &dg, int w, const float4 *__restrict__ s,
+                                          const float4 *__restrict__ t, float4 *r, const void *__restrict__ u,
+                                          const void *__restrict__ sw, const void *__restrict__ swinv, float mu_e,
+                                          float mu_o, const int *__restrict__ sched, const float4 *__restrict__ sub) {
+  const int lane = threadIdx.x & 31, vbh = g.vbh, tpb = (vbh + 15) >> 4;
+  const int p = PAR == 2 ? w & 1 : PAR, wb = PAR == 2 ? w >> 1 : w;
+  int blk = wb / tpb;
+  const int s0 = (wb - blk * tpb) * 16 + (lane & 15);
+  if (sched) blk = __ldg(sched + blk);
+  // lanes beyond the last site work on it again (every lane takes part in
+  // the exchange) and store nothing
+  const bool act = s0 < vbh;
+  const int si = act ? s0 : vbh - 1;
+  Site x;
+  site_decode(g, p, blk, si, x);
+  const int chunk = p * g.nbl + blk;
+  const EoRole ro = eo_role(g, lane >> 4);
+  const size_t own = ((size_t)chunk * 6 + 3 * ro.role) * vbh + si;   // this role's chirality of a field
+  cpx<float> acc[6], h[6];
+  if (OPS & (OP_HOP | OP_HOPSUB)) {
+    // the two directions of the role: coordinates and blocks
+    const int ya = ro.role ? x.y[2] : x.y[0], yb = ro.role ? x.y[1] : x.y[3];
+    const int na = ro.role ? x.n[2] : x.n[0], nba = ro.role ? g.nb[2] : g.nb[0], bsta = ro.role ? g.bstr[2] : g.bstr[0];
+    const int nb = ro.role ? x.n[1] : x.n[3], nbb = ro.role ? g.nb[1] : g.nb[3], bstb = ro.role ? g.bstr[1] : 1;
+    auto fwd = [&](int y, int n, int nbk, int bstr, int bs, int str, int &c2, int &s2) {
+      const bool in = y + 1 < bs;
+      s2 = (in ? x.l + str : x.l - (bs - 1) * str) >> 1;
+      c2 = (1 - p) * g.nbl + blk + (in ? 0 : (n + 1 < nbk ? bstr : -(nbk - 1) * bstr));
+    };
+    auto bwd = [&](int y, int n, int nbk, int bstr, int bs, int str, int &c2, int &s2) {
+      const bool in = y > 0;
+      s2 = (in ? x.l - str : x.l + (bs - 1) * str) >> 1;
+      c2 = (1 - p) * g.nbl + blk + (in ? 0 : (n > 0 ? -bstr : (nbk - 1) * bstr));
+    };
+    // global time coordinate: the time links at x0 = N0-1 carry the boundary sign
+    const int x0 = (DD ? dg.x0off : 0) + x.n[0] * g.bs[0] + x.y[0], xlast = (DD ? dg.N0 : g.L[0]) - 1;
+    Pair3 up, lo;
+#pragma unroll
+    for (int k = 0; k < 3; k++) up.re[k] = up.im[k] = lo.re[k] = lo.im[k] = make_float2(0.0f, 0.0f);
+    int c2, s2;
+    if (DD && ro.role == 0 && na + 1 == nba && ya + 1 == ro.bsa) {
+      eo_face_fwd<LP>(dg.hup, face_sites(g), face_index_of(g, x.n, x.y), u, vbh, chunk, si, x0 == xlast, up, lo);
+    } else {
+      fwd(ya, na, nba, bsta, ro.bsa, ro.stra, c2, s2);
+      eo_field_hop<0, 0, LP>(ro, t, u, vbh, c2, s2, chunk, ro.mua, si, ro.s, ro.role == 0 && x0 == xlast, up, lo);
+    }
+    if (DD && ro.role == 0 && na == 0 && ya == 0) {
+      eo_face_bwd(dg.hdn, face_sites(g), face_index_of(g, x.n, x.y), up, lo);
+    } else {
+      bwd(ya, na, nba, bsta, ro.bsa, ro.stra, c2, s2);
+      eo_field_hop<0, 1, LP>(ro, t, u, vbh, c2, s2, c2, ro.mua, s2, -ro.s, ro.role == 0 && x0 == 0, up, lo);
+    }
+    fwd(yb, nb, nbb, bstb, ro.bsb, ro.strb, c2, s2);
+    eo_field_hop<1, 0, LP>(ro, t, u, vbh, c2, s2, chunk, ro.mub, si, ro.t, false, up, lo);
+    bwd(yb, nb, nbb, bstb, ro.bsb, ro.strb, c2, s2);
+    eo_field_hop<1, 1, LP>(ro, t, u, vbh, c2, s2, c2, ro.mub, s2, -ro.t, false, up, lo);
+    if (DD) __syncwarp();
+    eo_exchange(ro.role, up, lo, h);
+#pragma unroll
+    for (int i = 0; i < 6; i++) h[i] = mk<float>(-0.5f * h[i].re, -0.5f * h[i].im);
+    if (OPS & OP_INV) {
+      cpx<float> q[6];
+      float m[36];
+      Store<float>::load_pauli(swinv, chunk, ro.role, si, vbh, m);
+      eo_pauli(0.0f, m, h, q);
+#pragma unroll
+      for (int i = 0; i < 6; i++) h[i] = q[i];
+    }
+  }
+  if (OPS & OP_SW) {
+    cpx<float> in[6];
+    eo_load(s + own, vbh, in);
+    float m[36];
+    Store<float>::load_pauli(sw, chunk, ro.role, si, vbh, m);
+    const float mu = p == 0 ? mu_e : mu_o;
+    eo_pauli(ro.role ? -mu : mu, m, in, acc);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 6; i++) acc[i] = mk<float>(0.0f, 0.0f);
+  }
+  if (OPS & (OP_HOP | OP_HOPSUB)) {
+    const float sg = (OPS & OP_HOP) ? 1.0f : -1.0f;
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+      acc[i] = mk<float>(fmaf(sg, h[i].re, acc[i].re), fmaf(sg, h[i].im, acc[i].im));
+    }
+  }
+  if (!act) return;
+  if (OPS & (OP_SUB | OP_ACC)) {   // r = sub - acc (the residual update of a preconditioner), r += acc
+    cpx<float> v[6];
+    eo_load(((OPS & OP_SUB) ? sub : (const float4 *)r) + own, vbh, v);
+    const float sg = (OPS & OP_SUB) ? -1.0f : 1.0f;
+#pragma unroll
+    for (int i = 0; i < 6; i++) acc[i] = mk<float>(fmaf(sg, acc[i].re, v[i].re), fmaf(sg, acc[i].im, v[i].im));
+  }
+  eo_store(r + own, vbh, acc);
+}
+
+// CTAs of four warps for nblk blocks (a multiple of eight in every use, since
+// every lattice direction has an even number of blocks: no warp is left over)
+static unsigned pair_grid(const Geom &g, int par, int nblk) {
+  return (unsigned)(((g.vbh + 15) / 16) * nblk * (par == 2 ? 2 : 1) / 4);
+}
+__device__ __forceinline__ int pair_warp(int cta) { return cta * 4 + (threadIdx.x >> 5); }
+
+template <int OPS, int PAR, class LP>
+__global__ void __launch_bounds__(128, DW_MINB32)
+    dirac_pair_kernel(Geom g, const float4 *__restrict__ s, const float4 *__restrict__ t, float4 *r,
+                      const void *__restrict__ u, const void *__restrict__ sw, const void *__restrict__ swinv,
+                      float mu_e, float mu_o, const int *__restrict__ sched, const float4 *__restrict__ sub) {
+  pair_body<OPS, PAR, LP, 0>(g, DDGeom{0, 0, nullptr, nullptr}, pair_warp(blockIdx.x), s, t, r, u, sw, swinv, mu_e, mu_o,
+                             sched, sub);
+}
+template <int OPS, int PAR, class LP>
+__global__ void __launch_bounds__(128, DW_MINB32)
+    dirac_pair_dd_kernel(Geom g, DDGeom dg, const float4 *__restrict__ s, const float4 *__restrict__ t, float4 *r,
+                         const void *__restrict__ u, const void *__restrict__ sw, const void *__restrict__ swinv,
+                         float mu_e, float mu_o, const int *__restrict__ sched) {
+  pair_body<OPS, PAR, LP, 1>(g, dg, pair_warp(blockIdx.x), s, t, r, u, sw, swinv, mu_e, mu_o, sched, nullptr);
+}
+
+// The direct FP64 kernels (the DD twin takes the slab's geometry)
+template <typename R, int OPS, int PAR, int RHALF = 0, int THALF = 0>
+__global__ void __launch_bounds__(128, DW_MINB64)
     dirac_kernel(Geom g, const void *__restrict__ s, const void *__restrict__ t, void *r, const void *__restrict__ u,
                  const void *__restrict__ sw, const void *__restrict__ swinv, R mu_e, R mu_o,
                  const int *__restrict__ sched, const void *__restrict__ sub) {
-  dirac_body<R, OPS, PAR, RHALF, THALF, L12, 0>(g, DDGeom{0, 0, nullptr, nullptr}, blockIdx.x * blockDim.x + threadIdx.x,
-                                                s, t, r, u, sw, swinv, mu_e, mu_o,
-                                                sched, sub);
+  dirac_body<R, OPS, PAR, RHALF, THALF, 0>(g, DDGeom{0, 0, nullptr, nullptr}, blockIdx.x * blockDim.x + threadIdx.x, s,
+                                           t, r, u, sw, swinv, mu_e, mu_o, sched, sub);
 }
-template <typename R, int OPS, int PAR, int L12>
-__global__ void __launch_bounds__(128, sizeof(R) == 8 ? DW_MINB64 : DW_MINB32)
+template <typename R, int OPS, int PAR>
+__global__ void __launch_bounds__(128, DW_MINB64)
     dirac_dd_kernel(Geom g, DDGeom dg, const void *__restrict__ s, const void *__restrict__ t, void *r,
                     const void *__restrict__ u, const void *__restrict__ sw, const void *__restrict__ swinv, R mu_e,
                     R mu_o, const int *__restrict__ sched) {
-  dirac_body<R, OPS, PAR, 0, 0, L12, 1>(g, dg, blockIdx.x * blockDim.x + threadIdx.x, s, t, r, u, sw, swinv, mu_e,
-                                        mu_o, sched, nullptr);
+  dirac_body<R, OPS, PAR, 0, 0, 1>(g, dg, blockIdx.x * blockDim.x + threadIdx.x, s, t, r, u, sw, swinv, mu_e, mu_o,
+                                   sched, nullptr);
 }
 
 // ------------------------------------------------------------------------
@@ -371,7 +468,7 @@ __device__ __forceinline__ void staged_tile(const Geom &g, int PAR_, int t, int 
 // 0.69 ms at 32^3x64, DRAM reads 4.35 GB against 3.36 GB per launch (the
 // prefetched lines were partly evicted before use).
 // Several systems of the batched solvers (SAP_MS at most): r_j = sub_j -
-// Dw(mu_j) s_j, FP32, in one launch whose CTAs of one tile of 128 sites
+// Dw(mu_j) s_j, FP32, in one launch whose CTAs of one tile of sites
 // are adjacent (CTA x: tile x / n, system x % n), so the links and SW
 // matrices of a tile serve every system while they are in L2.
 struct DwSys {
@@ -380,11 +477,11 @@ struct DwSys {
   const void *sub[SAP_MS];
   float mu[SAP_MS];
 };
-template <int L12>
+template <class LP>
 __global__ void __launch_bounds__(128, DW_MINB32)
     dirac_sys_kernel(Geom g, DwSys f, int n, const void *__restrict__ u, const void *__restrict__ sw, int eoflg,
                      const int *__restrict__ sched) {
-  const int j = blockIdx.x % n, i = (blockIdx.x / n) * blockDim.x + threadIdx.x;
+  const int j = blockIdx.x % n;
   // selected without indexing the parameter arrays by a variable (which
   // would copy them to local memory)
   const void *s = f.s[0], *sb = f.sub[0];
@@ -398,8 +495,9 @@ __global__ void __launch_bounds__(128, DW_MINB32)
       sb = f.sub[q];
       mu = f.mu[q];
     }
-  dirac_body<float, OP_SW | OP_HOP | OP_SUB, 2, 0, 0, L12, 0>(g, DDGeom{0, 0, nullptr, nullptr}, i, s, s, r, u, sw,
-                                                               nullptr, mu, eoflg ? 0.0f : mu, sched, sb);
+  pair_body<OP_SW | OP_HOP | OP_SUB, 2, LP, 0>(g, DDGeom{0, 0, nullptr, nullptr}, pair_warp(blockIdx.x / n),
+                                               (const float4 *)s, (const float4 *)s, (float4 *)r, u, sw, nullptr, mu,
+                                               eoflg ? 0.0f : mu, sched, (const float4 *)sb);
 }
 
 template <int OPS, int PAR, int DD>
@@ -564,19 +662,34 @@ static void launch_staged(const Ctx &c, const DDGeom &dg, const void *s, const v
         mu_o, c.sched, tpc, ntiles, c.d_kerr);
 }
 
-template <typename R, int OPS, int PAR, int L12, int DD>
-static void launch_plain(const Ctx &c, const DDGeom &dg, const void *s, const void *t, void *r, const void *u,
-                         R mu_e, R mu_o, cudaStream_t st) {
+template <int OPS, int PAR, int DD>
+static void launch_plain(const Ctx &c, const DDGeom &dg, const void *s, const void *t, void *r, double mu_e,
+                         double mu_o, cudaStream_t st) {
   const Geom &g = c.g;
-  const void *sw = sizeof(R) == 8 ? (const void *)c.swd : (const void *)c.sw32;
-  const void *swinv = sizeof(R) == 8 ? (const void *)c.swd_inv : (const void *)c.sw32_inv;
   const int n = PAR == 2 ? g.vol : g.volh, threads = 128;
   if (DD)
-    dirac_dd_kernel<R, OPS, PAR, L12><<<(n + threads - 1) / threads, threads, 0, st>>>(g, dg, s, t, r, u, sw, swinv,
-                                                                                      mu_e, mu_o, c.sched);
+    dirac_dd_kernel<double, OPS, PAR><<<(n + threads - 1) / threads, threads, 0, st>>>(g, dg, s, t, r, c.ud, c.swd,
+                                                                                      c.swd_inv, mu_e, mu_o, c.sched);
   else
-    dirac_kernel<R, OPS, PAR, 0, 0, L12><<<(n + threads - 1) / threads, threads, 0, st>>>(
-        g, s, t, r, u, sw, swinv, mu_e, mu_o, c.sched, nullptr);
+    dirac_kernel<double, OPS, PAR><<<(n + threads - 1) / threads, threads, 0, st>>>(g, s, t, r, c.ud, c.swd, c.swd_inv,
+                                                                                   mu_e, mu_o, c.sched, nullptr);
+}
+
+// the FP32 operators on the listed blocks (all of them in the order sched),
+// with the links u read by LP
+template <int OPS, int PAR, class LP>
+static void launch_pairs(const Ctx &c, const DDGeom *dg, const void *s, const void *t, void *r, const void *u,
+                         float mu_e, float mu_o, const int *sched, int nblk, const void *sub, cudaStream_t st) {
+  const unsigned nb = pair_grid(c.g, PAR, nblk);
+  if constexpr (!(OPS & OP_SUB)) {
+    if (dg) {
+      dirac_pair_dd_kernel<OPS, PAR, LP><<<nb, 128, 0, st>>>(c.g, *dg, (const float4 *)s, (const float4 *)t, (float4 *)r,
+                                                            u, c.sw32, c.sw32_inv, mu_e, mu_o, sched);
+      return;
+    }
+  }
+  dirac_pair_kernel<OPS, PAR, LP><<<nb, 128, 0, st>>>(c.g, (const float4 *)s, (const float4 *)t, (float4 *)r, u, c.sw32,
+                                                     c.sw32_inv, mu_e, mu_o, sched, (const float4 *)sub);
 }
 
 // With domain decomposition the operators that hop (all but Dwee, Dwoo)
@@ -593,21 +706,15 @@ static void launch(const Ctx &c, const void *s, const void *t, void *r, R mu_e, 
   const bool dd = HOPS && dd_on(c);
   if (dd && dd_faces(const_cast<Ctx &>(c), sizeof(R) == 8 ? 64 : 32, t, u12 ? u12 : u, u12 != nullptr, st, g))
     return;
-  if (sizeof(R) == 8 && !(OPS & OP_ACC) && (OPS & (OP_SW | OP_INV)) && c.dw_staged && c.d_kerr) {
-    if (dd) launch_staged<OPS, PAR, 1>(c, g, s, t, r, (double)mu_e, (double)mu_o, st);
-    else launch_staged<OPS, PAR, 0>(c, g, s, t, r, (double)mu_e, (double)mu_o, st);
-    return;
-  }
   if constexpr (sizeof(R) == 4) {
-    if (u12) {
-      if (dd) launch_plain<R, OPS, PAR, 1, 1>(c, g, s, t, r, u12, mu_e, mu_o, st);
-      else launch_plain<R, OPS, PAR, 1, 0>(c, g, s, t, r, u12, mu_e, mu_o, st);
-      return;
-    }
-  }
-  {
-    if (dd) launch_plain<R, OPS, PAR, 0, 1>(c, g, s, t, r, u, mu_e, mu_o, st);
-    else launch_plain<R, OPS, PAR, 0, 0>(c, g, s, t, r, u, mu_e, mu_o, st);
+    if (u12) launch_pairs<OPS, PAR, EoTwoRow>(c, dd ? &g : nullptr, s, t, r, u12, mu_e, mu_o, c.sched, c.g.nbl, nullptr, st);
+    else launch_pairs<OPS, PAR, EoFull>(c, dd ? &g : nullptr, s, t, r, u, mu_e, mu_o, c.sched, c.g.nbl, nullptr, st);
+  } else if (!(OPS & OP_ACC) && (OPS & (OP_SW | OP_INV)) && c.dw_staged && c.d_kerr) {
+    if (dd) launch_staged<OPS, PAR, 1>(c, g, s, t, r, mu_e, mu_o, st);
+    else launch_staged<OPS, PAR, 0>(c, g, s, t, r, mu_e, mu_o, st);
+  } else {
+    if (dd) launch_plain<OPS, PAR, 1>(c, g, s, t, r, mu_e, mu_o, st);
+    else launch_plain<OPS, PAR, 0>(c, g, s, t, r, mu_e, mu_o, st);
   }
 }
 
@@ -648,18 +755,14 @@ int dirac_dw_blocks(const Ctx &c, R mu, const void *s, void *r, const int *block
     dirac_staged_kernel<OPS, 2><<<ntiles, DWT_TS, DWT_SMEM, st>>>(
         c.g, (const double2 *)s, (const double2 *)s, (double2 *)r, (const double2 *)c.ud, (const double2 *)c.swd,
         (double)mu, (double)muo, blocks, tpc, ntiles, c.d_kerr);
+  } else if constexpr (sizeof(R) == 4) {
+    if (const void *u12 = links12(const_cast<Ctx &>(c), st))
+      launch_pairs<OPS, 2, EoTwoRow>(c, nullptr, s, s, r, u12, mu, muo, blocks, nblk, nullptr, st);
+    else
+      launch_pairs<OPS, 2, EoFull>(c, nullptr, s, s, r, c.u32, mu, muo, blocks, nblk, nullptr, st);
   } else {
-    const void *u = sizeof(R) == 8 ? (const void *)c.ud : (const void *)c.u32;
-    const void *sw = sizeof(R) == 8 ? (const void *)c.swd : (const void *)c.sw32;
     const int threads = 128, n = nblk * c.g.vb;
-    if constexpr (sizeof(R) == 4) {
-      if (const void *u12 = links12(const_cast<Ctx &>(c), st)) {
-        dirac_kernel<R, OPS, 2, 0, 0, 1><<<(n + threads - 1) / threads, threads, 0, st>>>(
-            c.g, s, s, r, u12, sw, nullptr, mu, muo, blocks, nullptr);
-        return cudaGetLastError() == cudaSuccess ? 0 : -2;
-      }
-    }
-    dirac_kernel<R, OPS, 2><<<(n + threads - 1) / threads, threads, 0, st>>>(c.g, s, s, r, u, sw, nullptr, mu, muo,
+    dirac_kernel<R, OPS, 2><<<(n + threads - 1) / threads, threads, 0, st>>>(c.g, s, s, r, c.ud, c.swd, nullptr, mu, muo,
                                                                             blocks, nullptr);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -689,22 +792,14 @@ int dirac_multi32(const Ctx &c, int n, float mu, void *const *sv, void *const *r
   // registers, 8 warps per SM) took 13.0 ms for four fields at 48^3x96 with
   // 6^4 blocks against 6.9 ms for four single-field launches
   const float muo = c.eoflg ? 0.0f : mu;
-  const int threads = 128, nn = c.g.vol;
-  const unsigned nb = (unsigned)((nn + threads - 1) / threads);
   const void *u12 = links12(const_cast<Ctx &>(c), st);
+  constexpr int OPS = OP_SW | OP_HOP;
   for (int j = 0; j < n; j++) {
-    if (subv && u12)
-      dirac_kernel<float, OP_SW | OP_HOP | OP_SUB, 2, 0, 0, 1><<<nb, threads, 0, st>>>(
-          c.g, sv[j], sv[j], rv[j], u12, c.sw32, nullptr, mu, muo, c.sched, subv[j]);
-    else if (subv)
-      dirac_kernel<float, OP_SW | OP_HOP | OP_SUB, 2><<<nb, threads, 0, st>>>(
-          c.g, sv[j], sv[j], rv[j], c.u32, c.sw32, nullptr, mu, muo, c.sched, subv[j]);
-    else if (u12)
-      dirac_kernel<float, OP_SW | OP_HOP, 2, 0, 0, 1><<<nb, threads, 0, st>>>(c.g, sv[j], sv[j], rv[j], u12, c.sw32,
-                                                                             nullptr, mu, muo, c.sched, nullptr);
-    else
-      dirac_kernel<float, OP_SW | OP_HOP, 2><<<nb, threads, 0, st>>>(c.g, sv[j], sv[j], rv[j], c.u32, c.sw32, nullptr,
-                                                                    mu, muo, c.sched, nullptr);
+    const void *b = subv ? subv[j] : nullptr;
+    if (b && u12) launch_pairs<OPS | OP_SUB, 2, EoTwoRow>(c, nullptr, sv[j], sv[j], rv[j], u12, mu, muo, c.sched, c.g.nbl, b, st);
+    else if (b) launch_pairs<OPS | OP_SUB, 2, EoFull>(c, nullptr, sv[j], sv[j], rv[j], c.u32, mu, muo, c.sched, c.g.nbl, b, st);
+    else if (u12) launch_pairs<OPS, 2, EoTwoRow>(c, nullptr, sv[j], sv[j], rv[j], u12, mu, muo, c.sched, c.g.nbl, b, st);
+    else launch_pairs<OPS, 2, EoFull>(c, nullptr, sv[j], sv[j], rv[j], c.u32, mu, muo, c.sched, c.g.nbl, b, st);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -721,11 +816,10 @@ int dirac_sys32(const Ctx &c, int n, const float *mu, void *const *sv, void *con
     f.sub[j] = subv[k];
     f.mu[j] = mu[k];
   }
-  const int threads = 128;
-  const unsigned nb = (unsigned)((c.g.vol + threads - 1) / threads) * n;
+  const unsigned nb = pair_grid(c.g, 2, c.g.nbl) * n;
   const void *u12 = links12(const_cast<Ctx &>(c), st);
-  if (u12) dirac_sys_kernel<1><<<nb, threads, 0, st>>>(c.g, f, n, u12, c.sw32, c.eoflg, c.sched);
-  else dirac_sys_kernel<0><<<nb, threads, 0, st>>>(c.g, f, n, c.u32, c.sw32, c.eoflg, c.sched);
+  if (u12) dirac_sys_kernel<EoTwoRow><<<nb, 128, 0, st>>>(c.g, f, n, u12, c.sw32, c.eoflg, c.sched);
+  else dirac_sys_kernel<EoFull><<<nb, 128, 0, st>>>(c.g, f, n, c.u32, c.sw32, c.eoflg, c.sched);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

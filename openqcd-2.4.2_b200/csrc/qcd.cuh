@@ -328,19 +328,20 @@ template <> struct Store<float> {
   }
 };
 
-// FP32 link stored as its first two rows (12 reals, planes
-// ((chunk*4 + mu)*6 + k)*vbh + s); the third row is rebuilt as the complex
+// FP32 link stored as its first two rows (12 reals, three float4 planes of
+// two complex entries each, ((chunk*4 + mu)*3 + j)*vbh + s); the third row is rebuilt as the complex
 // conjugate of the cross product of the first two, exact for SU(3), and
 // negated for a link that carries the antiperiodic time-boundary sign
 // (neg).  The library checks every link for this relation, with the sign
 // its position implies, before it reads 12-real links.
 __device__ __forceinline__ su3<float> load_link12(const void *base, int chunk, int mu, int s, int vbh, bool neg) {
-  const float2 *p = (const float2 *)base + ((size_t)chunk * 4 + mu) * 6 * vbh + s;
+  const float4 *p = (const float4 *)base + ((size_t)chunk * 4 + mu) * 3 * vbh + s;
   su3<float> r;
 #pragma unroll
-  for (int k = 0; k < 6; k++) {
-    const float2 v = __ldg(p + (size_t)k * vbh);
-    r.e[k] = mk<float>(v.x, v.y);
+  for (int j = 0; j < 3; j++) {
+    const float4 v = __ldg(p + (size_t)j * vbh);
+    r.e[2 * j] = mk<float>(v.x, v.y);
+    r.e[2 * j + 1] = mk<float>(v.z, v.w);
   }
   const float sg = neg ? -1.0f : 1.0f;
 #pragma unroll

@@ -16,14 +16,14 @@
 // update_flds1/2; sap.c:740-767, blk_solv.c:1153, sap.c:618-716);
 // k_sap_blocks_plain the plain one (isolv=0: blk_mres, update_flds0;
 // blk_solv.c:1117, sap.c:592).  One CTA owns one block: the fields that
-// neighbouring sites read (the current even residual, the odd intermediate,
-// the even solution) live in shared memory as 24 planes of vbh floats, the
-// Dhat image of the residual stays in registers, links and SW matrices come
-// through the L1 cache.  Fields that only their own site reads (the odd
-// start vector of the eo solve, the solution of the plain solve) are kept in
-// the phi output field, so that blocks of up to 768 sites per parity (6^4
-// blocks among them) fit into shared memory.
+// neighbouring sites read (the current even residual, the odd intermediate)
+// live in shared memory, links and SW matrices come through the L1 cache.
+// Fields that only their own site reads (the odd start vector of the eo
+// solve, the solution of the plain solve) are kept in registers or in the
+// output fields, so that blocks of up to 768 sites per parity (6^4 blocks
+// among them) fit into shared memory.
 #include "lib.h"
+#include "pairs.cuh"
 #include <cstring>
 #include <cuda_fp16.h>
 
@@ -80,15 +80,14 @@ __device__ __forceinline__ int block_of_colour(const Geom &g, int h, int colour)
   return q + (((n[0] + n[1] + n[2] + n[3]) & 1) != colour);
 }
 
-// Storage policies of the block solver.  All keep the block work vectors
-// in shared memory as 6 float4 planes (plane j at sm[4*(j*ld + s)], the
-// complex components 2j and 2j+1 of site s: one 16-byte access per pair);
-// SapF32
-// reads the FP32 links and Pauli matrices, SapF16 FP16 copies of them (links
-// as __half2 planes, Pauli matrices as uint2 planes of four halves), with
-// all arithmetic in FP32.  (FP16 work vectors were tried: their rounding,
-// relative to each cycle's input residual, is of the size of the residual
-// reduction of five cycles and cost half as many GCR iterations again.)
+// Storage policies of the SW matrices: SapF32 reads FP32 Pauli matrices,
+// SapF16 FP16 copies of them (uint2 planes of four halves), with all
+// arithmetic in FP32; the links have theirs in pairs.cuh.  The plain block
+// solver (SapF32) keeps its work vectors in shared memory as 6 float4 planes
+// (plane j at sm[4*(j*ld + s)], the complex components 2j and 2j+1 of site s).
+// (FP16 work vectors were tried: their rounding, relative to each cycle's
+// input residual, is of the size of the residual reduction of five cycles
+// and cost half as many GCR iterations again.)
 struct SapF32 {
   using T = float;
   static constexpr int NP = 24;
@@ -116,87 +115,21 @@ struct SapF32 {
   __device__ __forceinline__ static su3<float> link(const void *u, int chunk, int mu, int s, int vbh) {
     return Store<float>::load_link(u, chunk, mu, s, vbh);
   }
-  // a link of the block-boundary hops (18 reals: the time-boundary sign is stored)
-  __device__ __forceinline__ static su3<float> blink(const void *u, int chunk, int mu, int s, int vbh, bool) {
-    return link(u, chunk, mu, s, vbh);
-  }
-  __device__ __forceinline__ static spinor<float> sw(const void *m, int chunk, int s, int vbh, float mu,
-                                                     const spinor<float> &in) {
-    return apply_sw_site<float>(m, chunk, s, vbh, mu, in);
+  __device__ __forceinline__ static void pauli(const void *m, int chunk, int half, int s, int vbh, float (&u)[36]) {
+    Store<float>::load_pauli(m, chunk, half, s, vbh, u);
   }
 };
 
 struct SapF16 {
-  using T = float;
-  static constexpr int NP = 24;
-  __device__ __forceinline__ static spinor<float> sm_load(const float *sm, int ld, int s) {
-    return SapF32::sm_load(sm, ld, s);
-  }
-  __device__ __forceinline__ static void sm_store(float *sm, int ld, int s, const spinor<float> &v) {
-    SapF32::sm_store(sm, ld, s, v);
-  }
-  __device__ __forceinline__ static su3<float> link(const void *u, int chunk, int mu, int s, int vbh) {
-    const __half2 *p = (const __half2 *)u + ((size_t)chunk * 4 + mu) * 9 * vbh + s;
-    su3<float> r;
+  __device__ __forceinline__ static void pauli(const void *m, int chunk, int half, int s, int vbh, float (&u)[36]) {
+    const uint2 *p = (const uint2 *)m + ((size_t)chunk * 18 + 9 * half) * vbh + s;
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-      const float2 f = __half22float2(__ldg(p + (size_t)k * vbh));
-      r.e[k] = mk<float>(f.x, f.y);
+    for (int j = 0; j < 9; j++) {
+      uint2 v = __ldg(p + (size_t)j * vbh);
+      const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+      const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+      u[4 * j] = a.x; u[4 * j + 1] = a.y; u[4 * j + 2] = b.x; u[4 * j + 3] = b.y;
     }
-    return r;
-  }
-  __device__ __forceinline__ static su3<float> blink(const void *u, int chunk, int mu, int s, int vbh, bool) {
-    return link(u, chunk, mu, s, vbh);
-  }
-  __device__ __forceinline__ static spinor<float> sw(const void *m, int chunk, int s, int vbh, float mu,
-                                                     const spinor<float> &in) {
-    spinor<float> out;
-    float u[36];
-    cpx<float> w[6], r[6];
-#pragma unroll
-    for (int half = 0; half < 2; half++) {
-      const uint2 *p = (const uint2 *)m + ((size_t)chunk * 18 + 9 * half) * vbh + s;
-#pragma unroll
-      for (int j = 0; j < 9; j++) {
-        uint2 v = __ldg(p + (size_t)j * vbh);
-        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-        u[4 * j] = a.x; u[4 * j + 1] = a.y; u[4 * j + 2] = b.x; u[4 * j + 3] = b.y;
-      }
-      weyl_get(in, half, w);
-      mul_pauli<float>(half == 0 ? mu : -mu, u, w, r);
-      weyl_put(out, half, r);
-    }
-    return out;
-  }
-};
-
-// FP32 with the links stored as their first two rows (12 reals, planes
-// ((chunk*4 + mu)*6 + k)*vbh + s) and the third row rebuilt as the complex
-// conjugate of the cross product of the first two, exact for SU(3).  The
-// hops inside a block never use the time-boundary links that carry the
-// antiperiodic sign (a block does not wrap); the block-boundary hops give
-// the sign by position (load_link12).  The library checks every link for
-// the relation, with that sign, before it selects this policy.
-struct SapF32R {
-  using T = float;
-  static constexpr int NP = 24;
-  __device__ __forceinline__ static spinor<float> sm_load(const float *sm, int ld, int s) {
-    return SapF32::sm_load(sm, ld, s);
-  }
-  __device__ __forceinline__ static void sm_store(float *sm, int ld, int s, const spinor<float> &v) {
-    SapF32::sm_store(sm, ld, s, v);
-  }
-  __device__ __forceinline__ static su3<float> link(const void *u, int chunk, int mu, int s, int vbh) {
-    return load_link12(u, chunk, mu, s, vbh, false);
-  }
-  // a link of the block-boundary hops, which may carry the time-boundary sign
-  __device__ __forceinline__ static su3<float> blink(const void *u, int chunk, int mu, int s, int vbh, bool neg) {
-    return load_link12(u, chunk, mu, s, vbh, neg);
-  }
-  __device__ __forceinline__ static spinor<float> sw(const void *m, int chunk, int s, int vbh, float mu,
-                                                     const spinor<float> &in) {
-    return apply_sw_site<float>(m, chunk, s, vbh, mu, in);
   }
 };
 
@@ -238,149 +171,330 @@ __device__ __forceinline__ spinor<float> block_hop(const SapArgs &a, int p, int 
   return h;
 }
 
-// v = the block's sums of v, the same in every thread (the warps' partial
-// sums added in warp order by each thread), with one barrier.  The callers
-// separate two reductions by other barriers, so red is never overwritten
-// while a thread still reads it.
-template <int NC>
-__device__ __forceinline__ void block_allreduce(double v[NC], double *red) {
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// v = the block's sums of the three values v, the same in every thread, with
+// one barrier.  The lanes of a warp first halve the set of values they carry
+// (four, one of them unused) while they halve the set of lanes, then sum
+// over the remaining lanes; every warp adds the warps' sums in the same
+// order.  The callers separate two reductions by other barriers, so red is
+// never overwritten while a thread still reads it.
+__device__ __forceinline__ double shfl_xor_d(double x, int o) { return __shfl_xor_sync(0xffffffffu, x, o); }
+__device__ __forceinline__ void block_allreduce3(double (&v)[3], double *red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
+  // lanes with bit 4 clear keep v[0], v[1], the others v[2]; then bit 3
+  const double a0 = shfl_xor_d(h16 ? v[0] : v[2], 16), a1 = shfl_xor_d(h16 ? v[1] : 0.0, 16);
+  const double x0 = (h16 ? v[2] : v[0]) + a0, x1 = (h16 ? 0.0 : v[1]) + a1;
+  double x = (h8 ? x1 : x0) + shfl_xor_d(h8 ? x0 : x1, 8);
 #pragma unroll
-  for (int k = 0; k < NC; k++) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  }
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NC; k++) red[k * 32 + w] = v[k];
+  for (int o = 4; o > 0; o >>= 1) x += shfl_xor_d(x, o);
+  if ((lane & 7) == 0) red[(lane >> 3) * 32 + w] = x;   // value lane / 8 of warp w
   __syncthreads();
+  double t = 0.0;
+  for (int j = lane & 7; j < nw; j += 8) t += red[(lane >> 3) * 32 + j];
 #pragma unroll
-  for (int k = 0; k < NC; k++) {
-    double t = 0.0;
-    for (int j = 0; j < nw; j++) t += red[k * 32 + j];
-    v[k] = t;
+  for (int o = 4; o > 0; o >>= 1) t += shfl_xor_d(t, o);
+#pragma unroll
+  for (int k = 0; k < 3; k++) v[k] = __shfl_sync(0xffffffffu, t, 8 * k);
+}
+
+// ------------------------------------------------------------------------
+// The even-odd block solver, two lanes per site (pairs.cuh).  In shared
+// memory a site's spinor is 9 float4 (144 bytes, free of bank conflicts for 8
+// consecutive sites): for each colour k the pairs (c1 c2), (c3 c4) and
+// (c4 c3), real parts then imaginary parts; the swapped copy lets both roles
+// load their lower components in the order of their projector.
+//
+// What bounds it: the shared-memory and L1 data path (half busy) and the
+// latency of the link and SW reads, at 8 to 16 warps per SM; HBM is far from
+// busy.  Against one thread per site (the form this replaces) a block of 4^4
+// has 8 warps instead of 4 and each works through half the chain.  One cycle
+// (nmr = 4: two launches each of this and the boundary kernel): 8^4 lattice 120
+// -> 70 us, 16^4 126 -> 78 us, 32^4 841 -> 760 us (4^4 blocks); 48x24^3 (6^4
+// blocks) 701 -> 664 us.  Tried and dropped: the links of the block copied into
+// shared memory at the start (their reads compete with the spinors' for the
+// same data path: 90.8 against 81.2 us on 8^4); the two half spinors as packed
+// FP32 pairs (fma.rn.f32x2 issues at half the rate: the same time within
+// 2 %); three CTAs of 256 threads per SM (80 registers, 3 % slower).
+constexpr int EO_SREC = 9;   // float4 of a spinor record
+
+template <int FI, int DAG>
+__device__ __forceinline__ void hop_pair(const float4 *rec, int lo_slot, const float (&u)[18], float gy, Pair3 &up,
+                                         Pair3 &lo) {
+  float2 hr[3], hi[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) hop_project<FI, DAG>(rec[3 * k], rec[3 * k + lo_slot], gy, hr[k], hi[k]);
+  hop_link<FI, DAG>(hr, hi, u, gy, up, lo);
+}
+
+// own chirality of the sum of the hops around site (p, s) within the block;
+// src: spinor records of parity 1-p.  Every lane of the warp takes part.
+template <class LP>
+__device__ __forceinline__ void eo_hop(const SapArgs &a, const EoRole &ro, int p, int blk, int s,
+                                       const float4 *src, cpx<float> (&o)[6]) {
+  const Geom &g = a.g;
+  int y[4];
+  unpack4(__ldg(g.lcoord + p * g.vbh + s), y);
+  const int l = y[0] * g.lstr[0] + y[1] * g.lstr[1] + y[2] * g.lstr[2] + y[3];
+  const int ya = ro.role ? y[2] : y[0], yb = ro.role ? y[1] : y[3];
+  const int chunk = p * g.nbl + blk, ochunk = (1 - p) * g.nbl + blk;
+  Pair3 up, lo;
+#pragma unroll
+  for (int k = 0; k < 3; k++) up.re[k] = up.im[k] = lo.re[k] = lo.im[k] = make_float2(0.0f, 0.0f);
+  // a neighbour outside the block is one of the eight zero records at index
+  // vbh8 (the one in the banks of the record it replaces), with any link: no
+  // branches, so that the loads of a hop overlap the arithmetic of the one
+  // before
+  const int slot = 1 + ro.role, vbh = g.vbh, vbh8 = (vbh + 7) & ~7;
+  const bool fa = ya + 1 < ro.bsa, ba = ya > 0, fb = yb + 1 < ro.bsb, bb = yb > 0;
+  int sfa = (l + ro.stra) >> 1, sba = (l - ro.stra) >> 1, sfb = (l + ro.strb) >> 1, sbb = (l - ro.strb) >> 1;
+  sfa = fa ? sfa : vbh8 + (sfa & 7);
+  sba = ba ? sba : vbh8 + (sba & 7);
+  sfb = fb ? sfb : vbh8 + (sfb & 7);
+  sbb = bb ? sbb : vbh8 + (sbb & 7);
+  float r0[LP::NRAW], r1[LP::NRAW], u[18];
+  LP::load(a.u, chunk, ro.mua, s, vbh, r0);
+  LP::load(a.u, ochunk, ro.mua, ba ? sba : s, vbh, r1);
+  LP::expand(r0, u);
+  hop_pair<0, 0>(src + sfa * EO_SREC, slot, u, ro.s, up, lo);
+  LP::load(a.u, chunk, ro.mub, s, vbh, r0);
+  LP::expand(r1, u);
+  hop_pair<0, 1>(src + sba * EO_SREC, slot, u, -ro.s, up, lo);
+  LP::load(a.u, ochunk, ro.mub, bb ? sbb : s, vbh, r1);
+  LP::expand(r0, u);
+  hop_pair<1, 0>(src + sfb * EO_SREC, slot, u, ro.t, up, lo);
+  LP::expand(r1, u);
+  hop_pair<1, 1>(src + sbb * EO_SREC, slot, u, -ro.t, up, lo);
+  eo_exchange(ro.role, up, lo, o);
+}
+
+// a chirality (6 components) of a spinor record and of a field
+__device__ __forceinline__ void eo_get(const float4 *rec, int role, cpx<float> (&v)[6]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const float4 q = rec[3 * k + role];
+    v[k] = mk<float>(q.x, q.z);
+    v[3 + k] = mk<float>(q.y, q.w);
+  }
+}
+__device__ __forceinline__ void eo_put(float4 *rec, int role, const cpx<float> (&v)[6]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    rec[3 * k + role] = make_float4(v[k].re, v[3 + k].re, v[k].im, v[3 + k].im);
+    if (role) rec[3 * k + 2] = make_float4(v[3 + k].re, v[k].re, v[3 + k].im, v[k].im);
+  }
+}
+// psi += phi on one chirality
+__device__ __forceinline__ void eo_add(float4 *f, int vbh, const cpx<float> (&v)[6]) {
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    float4 q = f[(size_t)j * vbh];
+    q.x += v[2 * j].re;
+    q.y += v[2 * j].im;
+    q.z += v[2 * j + 1].re;
+    q.w += v[2 * j + 1].im;
+    f[(size_t)j * vbh] = q;
   }
 }
 
-// The kernel runs as one loop over phases so that each heavy routine (the
-// odd-site hop, the even-site hop, the two SW products) has a single call
-// site; with separate set-up, MR and reconstruction code the kernel
-// overflowed the instruction cache.
+// rho += 1/2 h on one chirality
+__device__ __forceinline__ void eo_add_half(float4 *f, int vbh, const cpx<float> (&h)[6]) {
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    float4 q = f[(size_t)j * vbh];
+    q.x = fmaf(0.5f, h[2 * j].re, q.x);
+    q.y = fmaf(0.5f, h[2 * j].im, q.y);
+    q.z = fmaf(0.5f, h[2 * j + 1].re, q.z);
+    q.w = fmaf(0.5f, h[2 * j + 1].im, q.w);
+    f[(size_t)j * vbh] = q;
+  }
+}
+
+// r = (A + i m) w for one chirality of a site
+template <class P>
+__device__ __forceinline__ void eo_sw(const void *m, int chunk, int half, int s, int vbh, float mu,
+                                      const cpx<float> (&w)[6], cpx<float> (&r)[6]) {
+  float u[36];
+  P::pauli(m, chunk, half, s, vbh, u);
+  eo_pauli(half == 0 ? mu : -mu, u, w, r);
+}
+
+// Own chirality of the sum of the hops of phi into site (p, blk, s) across
+// the faces of its block (the block-boundary hop of the reference's
+// Dw_bnd/sap_com, as a gather); false if the site lies on no face of the
+// role's directions.  With domain decomposition the x0-neighbours across the
+// rank boundary are half spinors in the exchanged faces.
+template <class LP, int DD>
+__device__ __forceinline__ bool eo_cross(const SapArgs &a, const DDGeom &dg, const EoRole &ro, const float4 *phi,
+                                         int p, int blk, int s, cpx<float> (&o)[6]) {
+  const Geom &g = a.g;
+  Site x;
+  site_decode(g, p, blk, s, x);
+  const int chunk = p * g.nbl + blk;
+  const int ya = ro.role ? x.y[2] : x.y[0], yb = ro.role ? x.y[1] : x.y[3];
+  // global time coordinate: the time links at x0 = N0-1 carry the boundary sign
+  const int x0 = (DD ? dg.x0off : 0) + x.n[0] * g.bs[0] + x.y[0], xlast = (DD ? dg.N0 : g.L[0]) - 1;
+  Pair3 up, lo;
+#pragma unroll
+  for (int k = 0; k < 3; k++) up.re[k] = up.im[k] = lo.re[k] = lo.im[k] = make_float2(0.0f, 0.0f);
+  // chunk and site of the neighbour in the block across the face: block
+  // coordinate n of nb, step bstr, in-block stride str
+  auto across = [&](int n, int nb, int bstr, int bs, int str, int dir, int &c2, int &s2) {
+    int b = blk, l = x.l;
+    if (dir > 0) {
+      l -= (bs - 1) * str;
+      b += n + 1 < nb ? bstr : -(nb - 1) * bstr;
+    } else {
+      l += (bs - 1) * str;
+      b += n > 0 ? -bstr : (nb - 1) * bstr;
+    }
+    c2 = (1 - p) * g.nbl + b;
+    s2 = l >> 1;
+  };
+  const int na = ro.role ? x.n[2] : x.n[0], nba = ro.role ? g.nb[2] : g.nb[0], bsta = ro.role ? g.bstr[2] : g.bstr[0];
+  const int nb_ = ro.role ? x.n[1] : x.n[3], nbb = ro.role ? g.nb[1] : g.nb[3], bstb = ro.role ? g.bstr[1] : 1;
+  const bool fa = ya + 1 == ro.bsa, ba = ya == 0, fb = yb + 1 == ro.bsb, bb = yb == 0;
+  int c2, s2;
+  if (fa) {
+    if (DD && ro.role == 0 && na + 1 == nba) {
+      eo_face_fwd<LP>(dg.hup, face_sites(g), face_index_of(g, x.n, x.y), a.ub, g.vbh, chunk, s, x0 == xlast, up, lo);
+    } else {
+      across(na, nba, bsta, ro.bsa, ro.stra, +1, c2, s2);
+      eo_field_hop<0, 0, LP>(ro, phi, a.ub, g.vbh, c2, s2, chunk, ro.mua, s, ro.s, ro.role == 0 && x0 == xlast, up, lo);
+    }
+  }
+  if (ba) {
+    if (DD && ro.role == 0 && na == 0) {
+      eo_face_bwd(dg.hdn, face_sites(g), face_index_of(g, x.n, x.y), up, lo);
+    } else {
+      across(na, nba, bsta, ro.bsa, ro.stra, -1, c2, s2);
+      eo_field_hop<0, 1, LP>(ro, phi, a.ub, g.vbh, c2, s2, c2, ro.mua, s2, -ro.s, ro.role == 0 && x0 == 0, up, lo);
+    }
+  }
+  if (fb) {
+    across(nb_, nbb, bstb, ro.bsb, ro.strb, +1, c2, s2);
+    eo_field_hop<1, 0, LP>(ro, phi, a.ub, g.vbh, c2, s2, chunk, ro.mub, s, ro.t, false, up, lo);
+  }
+  if (bb) {
+    across(nb_, nbb, bstb, ro.bsb, ro.strb, -1, c2, s2);
+    eo_field_hop<1, 1, LP>(ro, phi, a.ub, g.vbh, c2, s2, c2, ro.mub, s2, -ro.t, false, up, lo);
+  }
+  __syncwarp();
+  eo_exchange(ro.role, up, lo, o);
+  const bool any = fa || ba || fb || bb;
+  return __shfl_xor_sync(0xffffffffu, (int)any, 16) || any;
+}
+
+// One CTA per block and system, NS sites per lane pair.
 //   step 0         : V = W = A_o^-1 rho_o ;  S1 = rho_e - D_eo W ; S0 = 0
 //                    (V is kept in phi_o until the last step)
 //   step 1..nmr    : W = A_o^-1 D_oe S1 ;  s2 = (A_e + i mu g5) S1 - D_eo W ;
 //                    z = (s2,S1)/|s2|^2 ; S0 += z S1 ; S1 -= z s2
-//   step nmr+1     : phi_o = V - A_o^-1 D_oe S0 ; phi_e = S0 ; psi += phi ;
-//                    rho_e = S1 ; rho_o = -i mu g5 phi_o (0 with the eo flag)
-template <int NS, class P, int MAXT, int MINB>
+//   after the last : rho_e = S1 ; phi_e = S0 ; S0 takes the place of S1
+//   step nmr+1     : phi_o = V - A_o^-1 D_oe S0 ; psi += phi ;
+//                    rho_o = -i mu g5 phi_o (0 with the eo flag)
+// S0 and s2 stay in registers with one site per lane pair; with more of them
+// S0 is kept in phi_e and s2 in rho_e (whose start value is used up in step 0).
+template <int NS, class LP, class P, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) k_sap_blocks_eo(SapArgs a) {
-  using T = typename P::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *smem = reinterpret_cast<T *>(smem_raw);
   const Geom &g = a.g;
-  const int ld = g.vbh;
-  T *S1 = smem, *W = smem + P::NP * ld, *S0 = smem + 2 * P::NP * ld;
-  __shared__ double red[3 * 32];
+  const int vbh = g.vbh;
+  const int nrec = ((vbh + 7) & ~7) + 8;   // records of a field, the zero records last
+  float4 *S1 = reinterpret_cast<float4 *>(smem_raw), *W = S1 + EO_SREC * nrec;
+  __shared__ double red[4 * 32];
   const SapSys y = sap_sys(a, blockIdx.x % a.nsys);
   const int blk = block_of_colour(g, blockIdx.x / a.nsys, a.colour);
   const int ce = blk, co = g.nbl + blk;
-  const int T_ = blockDim.x;
+  for (int i = threadIdx.x; i < 8 * EO_SREC; i += blockDim.x)
+    S1[EO_SREC * (nrec - 8) + i] = W[EO_SREC * (nrec - 8) + i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const EoRole ro = eo_role(g, lane >> 4);
+  // site k of a lane pair; lanes beyond the last site work on it again and
+  // store nothing
+  const int sa = wp * 16 + (lane & 15);
+  auto site = [&](int k, bool &act) {
+    const int s = sa + k * nw * 16;
+    act = s < vbh;
+    return act ? s : vbh - 1;
+  };
+  // a chirality of a field at (chunk, s): planes 3 role .. 3 role + 2
+  auto fld = [&](float4 *f, int chunk, int s) { return f + ((size_t)chunk * 6 + 3 * ro.role) * vbh + s; };
+  cpx<float> S0[6];
+#pragma unroll
+  for (int i = 0; i < 6; i++) S0[i] = mk<float>(0.0f, 0.0f);
   const int nmr = a.nmr;
   for (int step = 0; step <= nmr + 1; step++) {
     const bool last = step == nmr + 1;
     // ---- odd sites
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < NS; k++) {
-      int s = threadIdx.x + k * T_;
-      if (s < g.vbh) {
-        spinor<float> h;
-        if (step == 0) {
-          h = Store<float>::load_spinor_rw(y.rho, co, s, g.vbh);
-        } else {
-          h = block_hop<P>(a, 1, blk, s, last ? S0 : S1, ld);
-        }
-        spinor<float> t = P::sw(a.swinv, co, s, g.vbh, 0.0f, h);
-        if (step == 0) {
-          Store<float>::store_spinor(y.phi, co, s, g.vbh, t);
-          P::sm_store(W, ld, s, t);
-        } else if (!last) {
-          P::sm_store(W, ld, s, t);
-        } else {
-          // one field at a time, so that few spinors are live at once
-          spinor<float> ph = Store<float>::load_spinor_rw(y.phi, co, s, g.vbh);
-          ssub(ph, t);
-          Store<float>::store_spinor(y.phi, co, s, g.vbh, ph);
-          {
-            spinor<float> ps = Store<float>::load_spinor_rw(y.psi, co, s, g.vbh);
-            sadd(ps, ph);
-            Store<float>::store_spinor(y.psi, co, s, g.vbh, ps);
-          }
-          spinor<float> ro;
-          if (a.eoflg) {
-            szero(ro);
-          } else {
+      bool act;
+      const int s = site(k, act);
+      cpx<float> h[6], t[6];
+      if (step == 0) {
+        eo_load(fld(y.rho, co, s), vbh, h);
+      } else {
+        eo_hop<LP>(a, ro, 1, blk, s, S1, h);
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-              const float m = c < 2 ? -y.mu : y.mu;   // rho_o = i m phi_o
+        for (int i = 0; i < 6; i++) h[i] = mk<float>(-0.5f * h[i].re, -0.5f * h[i].im);
+      }
+      eo_sw<P>(a.swinv, co, ro.role, s, vbh, 0.0f, h, t);
+      if (!act) continue;
+      if (!last) {
+        if (step == 0) eo_store(fld(y.phi, co, s), vbh, t);
+        eo_put(W + s * EO_SREC, ro.role, t);
+      } else {
+        cpx<float> ph[6];
+        eo_load(fld(y.phi, co, s), vbh, ph);
+        // rho_o = i m phi_o with m = -mu on the upper, +mu on the lower chirality
+        const float m = a.eoflg ? 0.0f : (ro.role ? y.mu : -y.mu);
 #pragma unroll
-              for (int j = 0; j < 3; j++) ro.c[c].c[j] = mk<float>(-m * ph.c[c].c[j].im, m * ph.c[c].c[j].re);
-            }
-          }
-          Store<float>::store_spinor(y.rho, co, s, g.vbh, ro);
+        for (int i = 0; i < 6; i++) {
+          ph[i].re -= t[i].re;
+          ph[i].im -= t[i].im;
+          t[i] = a.eoflg ? mk<float>(0.0f, 0.0f) : mk<float>(-m * ph[i].im, m * ph[i].re);
         }
+        eo_store(fld(y.phi, co, s), vbh, ph);
+        eo_add(fld(y.psi, co, s), vbh, ph);
+        eo_store(fld(y.rho, co, s), vbh, t);
       }
     }
+    if (last) break;
     __syncthreads();
     // ---- even sites
-    if (last) {
-#pragma unroll
-      for (int k = 0; k < NS; k++) {
-        int s = threadIdx.x + k * T_;
-        if (s < g.vbh) {
-          const spinor<float> s0 = P::sm_load(S0, ld, s);
-          Store<float>::store_spinor(y.phi, ce, s, g.vbh, s0);
-          {
-            spinor<float> ps = Store<float>::load_spinor_rw(y.psi, ce, s, g.vbh);
-            sadd(ps, s0);
-            Store<float>::store_spinor(y.psi, ce, s, g.vbh, ps);
-          }
-          Store<float>::store_spinor(y.rho, ce, s, g.vbh, P::sm_load(S1, ld, s));
-        }
-      }
-      break;
-    }
-    spinor<float> s2[NS];
+    cpx<float> s2[6];
     double v[3] = {0.0, 0.0, 0.0};
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < NS; k++) {
-      int s = threadIdx.x + k * T_;
-      if (s < g.vbh) {
-        // base - (-1/2) H W as (2 base + H W) / 2 (exact scalings), with
-        // base = rho_e (step 0) or (A_e + i mu g5) S1: the hop accumulates
-        // straight into it, so no second spinor is live across the hop
-        spinor<float> b2;
-        if (step == 0) b2 = Store<float>::load_spinor_rw(y.rho, ce, s, g.vbh);
-        else b2 = P::sw(a.sw, ce, s, g.vbh, y.mu, P::sm_load(S1, ld, s));
-        sscale<float>(b2, 2.0f);
-        block_hop_acc<P>(a, 0, blk, s, W, ld, b2);
-        sscale<float>(b2, 0.5f);
-        if (step == 0) {
-          P::sm_store(S1, ld, s, b2);
-          spinor<float> z;
-          szero(z);
-          P::sm_store(S0, ld, s, z);
-        } else {
-          const spinor<float> s1 = P::sm_load(S1, ld, s);
-          s2[k] = b2;
+      bool act;
+      const int s = site(k, act);
+      cpx<float> b[6], s1[6];
+      eo_hop<LP>(a, ro, 0, blk, s, W, b);
+      if (step == 0) {
+        eo_load(fld(y.rho, ce, s), vbh, s1);
 #pragma unroll
-          for (int c = 0; c < 4; c++)
+        for (int i = 0; i < 6; i++) s1[i] = mk<float>(s1[i].re + 0.5f * b[i].re, s1[i].im + 0.5f * b[i].im);
+        if (act) {
+          eo_put(S1 + s * EO_SREC, ro.role, s1);
+          if (NS > 1) eo_store(fld(y.phi, ce, s), vbh, S0);
+        }
+        continue;
+      }
+      eo_get(S1 + s * EO_SREC, ro.role, s1);
+      eo_sw<P>(a.sw, ce, ro.role, s, vbh, y.mu, s1, s2);
 #pragma unroll
-            for (int j = 0; j < 3; j++) {
-              const cpx<float> x2 = s2[k].c[c].c[j], x1 = s1.c[c].c[j];
-              v[0] += (double)x2.re * x2.re + (double)x2.im * x2.im;
-              v[1] += (double)x2.re * x1.re + (double)x2.im * x1.im;
-              v[2] += (double)x2.re * x1.im - (double)x2.im * x1.re;
-            }
+      for (int i = 0; i < 6; i++) {
+        s2[i].re += 0.5f * b[i].re;
+        s2[i].im += 0.5f * b[i].im;
+      }
+      if (act) {
+        if (NS > 1) eo_store(fld(y.rho, ce, s), vbh, s2);
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+          const double xr = s2[i].re, xi = s2[i].im, yr = s1[i].re, yi = s1[i].im;
+          v[0] += xr * xr + xi * xi;
+          v[1] += xr * yr + xi * yi;
+          v[2] += xr * yi - xi * yr;
         }
       }
     }
@@ -390,38 +504,41 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sap_blocks_eo(SapArgs a) {
     }
     // MR coefficient (blk_solv.c:1153-1188): stop if |s2|^2 < 2 FLT_MIN;
     // every thread has the same sums and computes the same coefficient
-    block_allreduce<3>(v, red);
+    block_allreduce3(v, red);
     const float rr = (float)v[0];
-    if (rr < 2.0f * 1.17549435e-38f) {
-      step = nmr;   // go to the reconstruction step
-      continue;
-    }
-    const float ri = 1.0f / rr, zr = (float)v[1] * ri, zi = (float)v[2] * ri;
-#pragma unroll
+    const bool stop = rr < 2.0f * 1.17549435e-38f;
+    const float ri = 1.0f / rr, zr = stop ? 0.0f : (float)v[1] * ri, zi = stop ? 0.0f : (float)v[2] * ri;
+    const bool fin = stop || step == nmr;
+#pragma unroll 1
     for (int k = 0; k < NS; k++) {
-      int s = threadIdx.x + k * T_;
-      if (s < g.vbh) {
-        // plane by plane (two complex components), so that only s2 stays
-        // live across the update
-        float4 *v1 = reinterpret_cast<float4 *>(S1), *v0 = reinterpret_cast<float4 *>(S0);
+      bool act;
+      const int s = site(k, act);
+      if (!act) continue;
+      cpx<float> s1[6];
+      eo_get(S1 + s * EO_SREC, ro.role, s1);
+      if (NS > 1) {
+        eo_load(fld(y.phi, ce, s), vbh, S0);
+        eo_load(fld(y.rho, ce, s), vbh, s2);
+      }
+      if (!stop) {
 #pragma unroll
-        for (int jp = 0; jp < 6; jp++) {
-          float4 a1 = v1[jp * ld + s], a0 = v0[jp * ld + s];
-          const cpx<float> x2 = s2[k].c[(2 * jp) / 3].c[(2 * jp) % 3];
-          const cpx<float> y2 = s2[k].c[(2 * jp + 1) / 3].c[(2 * jp + 1) % 3];
-          a0.x += zr * a1.x - zi * a1.y;
-          a0.y += zr * a1.y + zi * a1.x;
-          a0.z += zr * a1.z - zi * a1.w;
-          a0.w += zr * a1.w + zi * a1.z;
-          a1.x -= zr * x2.re - zi * x2.im;
-          a1.y -= zr * x2.im + zi * x2.re;
-          a1.z -= zr * y2.re - zi * y2.im;
-          a1.w -= zr * y2.im + zi * y2.re;
-          v0[jp * ld + s] = a0;
-          v1[jp * ld + s] = a1;
+        for (int i = 0; i < 6; i++) {
+          S0[i].re += zr * s1[i].re - zi * s1[i].im;
+          S0[i].im += zr * s1[i].im + zi * s1[i].re;
+          s1[i].re -= zr * s2[i].re - zi * s2[i].im;
+          s1[i].im -= zr * s2[i].im + zi * s2[i].re;
         }
       }
+      if (NS > 1 || fin) eo_store(fld(y.phi, ce, s), vbh, S0);
+      if (fin) {
+        eo_store(fld(y.rho, ce, s), vbh, s1);
+        eo_add(fld(y.psi, ce, s), vbh, S0);
+        eo_put(S1 + s * EO_SREC, ro.role, S0);
+      } else {
+        eo_put(S1 + s * EO_SREC, ro.role, s1);
+      }
     }
+    if (fin) step = nmr;   // the reconstruction step is next
     __syncthreads();
   }
 }
@@ -438,7 +555,7 @@ __global__ void __launch_bounds__(256) k_sap_blocks_plain(SapArgs a) {
   const int ld = g.vbh;
   // planes: S1 even, S1 odd; the solution S0 accumulates in phi
   float *S1[2] = {smem, smem + 24 * ld};
-  __shared__ double red[3 * 32];
+  __shared__ double red[4 * 32];
   const SapSys y = sap_sys(a, blockIdx.x % a.nsys);
   const int blk = block_of_colour(g, blockIdx.x / a.nsys, a.colour);
   const int T = blockDim.x;
@@ -479,7 +596,7 @@ __global__ void __launch_bounds__(256) k_sap_blocks_plain(SapArgs a) {
             }
         }
       }
-    block_allreduce<3>(v, red);
+    block_allreduce3(v, red);
     const float rr = (float)v[0];
     if (rr < 2.0f * 1.17549435e-38f) break;
     const float ri = 1.0f / rr, zr = (float)v[1] * ri, zi = (float)v[2] * ri;
@@ -522,88 +639,44 @@ __global__ void __launch_bounds__(256) k_sap_blocks_plain(SapArgs a) {
 }
 
 // rho(y) -= D_{y,x} phi(x) for every site y of a block of colour 1-c and every
-// neighbour x of y in a (colour c) block: the block-boundary hop of the
-// reference's Dw_bnd/sap_com, as a gather.
-// 8 resident CTAs per SM (64 registers): two SAP cycles at 48^3x96 with 6^4
-// blocks 17.86 ms against 17.99 ms with the compiler's choice (80-87
-// registers, 6 CTAs); 12 CTAs (40 registers) spilled
-#ifndef SAP_BND_MINB
-#define SAP_BND_MINB 8
-#endif
-template <class P, int DD>
+// neighbour x of y in a (colour c) block.  Two lanes per site, as in the block
+// solver: against one thread per site a launch takes 4.8 instead of 9.7 us on
+// 8^4 and 6 instead of 9.7 us on 16^4 (5 CTAs per SM); on large lattices, where
+// the gather's bytes in flight count, 8 CTAs per SM of 64 registers are as
+// fast as one thread per site was (71 against 69 us on 32^4, 47 against 44 us on
+// 48x24^3 with 6^4 blocks; with 5 CTAs 76 and 54 us).
+template <class LP, int DD>
 __device__ __forceinline__ void sap_bnd_body(const SapArgs &a, const DDGeom &dg) {
   const Geom &g = a.g;
   const SapSys y = sap_sys(a, blockIdx.x % a.nsys);
-  size_t i = (blockIdx.x / a.nsys) * (size_t)blockDim.x + threadIdx.x;
-  if (i >= (size_t)(g.nbl / 2) * g.vb) return;
-  int h = (int)(i / g.vb), r = (int)(i % g.vb);
-  int p = r >= g.vbh, s = r - p * g.vbh;
-  int blk = block_of_colour(g, h, 1 - a.colour);
-  Site x;
-  site_decode(g, p, blk, s, x);
-  const int chunk = p * g.nbl + blk;
-  // global time coordinate: the time links at x0 = N0-1 carry the boundary sign
-  const int x0 = (DD ? dg.x0off : 0) + x.n[0] * g.bs[0] + x.y[0];
-  const int xlast = (DD ? dg.N0 : g.L[0]) - 1;
-  // DD: the x0-neighbour blocks across the rank boundary are on the other
-  // ranks; their hops come from the exchanged faces of phi
-  const bool dd_up = DD && x.n[0] + 1 == g.nb[0] && x.y[0] + 1 == g.bs[0];
-  const bool dd_dn = DD && x.n[0] == 0 && x.y[0] == 0;
-  spinor<float> hsum;
-  szero(hsum);
-  bool any = false;
-#pragma unroll
-  for (int mu = 0; mu < 4; mu++) {
-    if (crosses_block(g, x, mu, +1)) {
-      su3<float> uu = P::blink(a.ub, chunk, mu, s, g.vbh, mu == 0 && x0 == xlast);
-      if (mu == 0 && dd_up) {
-        vec3<float> h0, h1;
-        Half<float>::load(dg.hup, face_sites(g), face_index_of(g, x.n, x.y), h0, h1);
-        dd_hop_fwd<float>(uu, h0, h1, hsum);
-      } else {
-        int c2, s2;
-        site_nbr(g, x, mu, +1, c2, s2);
-        spinor<float> sp = Store<float>::load_spinor(y.phi, c2, s2, g.vbh);
-        hop_fwd<float>(mu, uu, sp, hsum);
-      }
-      any = true;
-    }
-    if (crosses_block(g, x, mu, -1)) {
-      if (mu == 0 && dd_dn) {
-        vec3<float> c0, c1;
-        Half<float>::load(dg.hdn, face_sites(g), face_index_of(g, x.n, x.y), c0, c1);
-        dd_hop_bwd<float>(c0, c1, hsum);
-      } else {
-        int c2, s2;
-        site_nbr(g, x, mu, -1, c2, s2);
-        spinor<float> sm = Store<float>::load_spinor(y.phi, c2, s2, g.vbh);
-        su3<float> uu = P::blink(a.ub, c2, mu, s2, g.vbh, mu == 0 && x0 == 0);
-        hop_bwd<float>(mu, uu, sm, hsum);
-      }
-      any = true;
-    }
-  }
-  if (!any) return;
-  sscale<float>(hsum, 0.5f);   // rho -= (-1/2) H phi
-  spinor<float> rr = Store<float>::load_spinor_rw(y.rho, chunk, s, g.vbh);
-  sadd(rr, hsum);
-  Store<float>::store_spinor(y.rho, chunk, s, g.vbh, rr);
+  const int lane = threadIdx.x & 31;
+  const EoRole ro = eo_role(g, lane >> 4);
+  const size_t n = (size_t)(g.nbl / 2) * g.vb;
+  size_t i = ((blockIdx.x / a.nsys) * (size_t)(blockDim.x >> 5) + (threadIdx.x >> 5)) * 16 + (lane & 15);
+  const bool act = i < n;
+  if (!act) i = n - 1;   // every lane takes part in the exchange
+  const int h = (int)(i / g.vb), r = (int)(i % g.vb);
+  const int p = r >= g.vbh, s = r - p * g.vbh;
+  const int blk = block_of_colour(g, h, 1 - a.colour);
+  cpx<float> o[6];
+  const bool any = eo_cross<LP, DD>(a, dg, ro, y.phi, p, blk, s, o);
+  if (act && any) eo_add_half(y.rho + ((size_t)(p * g.nbl + blk) * 6 + 3 * ro.role) * g.vbh + s, g.vbh, o);
 }
 
 // the single-GPU kernel keeps its parameter list; the DD twin takes the
 // slab's geometry with the received faces
-template <class P>
-__global__ void __launch_bounds__(128, SAP_BND_MINB) k_sap_bnd(SapArgs a) {
-  sap_bnd_body<P, 0>(a, DDGeom{0, 0, nullptr, nullptr});
+template <class LP, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_sap_bnd(SapArgs a) {
+  sap_bnd_body<LP, 0>(a, DDGeom{0, 0, nullptr, nullptr});
 }
-template <class P>
-__global__ void __launch_bounds__(128, SAP_BND_MINB) k_sap_bnd_dd(SapArgs a, DDGeom dg) {
-  sap_bnd_body<P, 1>(a, dg);
+template <class LP>
+__global__ void __launch_bounds__(128, 5) k_sap_bnd_dd(SapArgs a, DDGeom dg) {
+  sap_bnd_body<LP, 1>(a, dg);
 }
 
 // DD: the x0-faces of the block solutions phi (FP32 half spinors, as
 // k_dd_pack in dd.cu, with the links as the boundary hops read them)
-template <class P>
+template <class LP>
 __global__ void k_sap_dd_pack(SapArgs a, DDGeom dg, void *dn, void *up) {
   const Geom &g = a.g;
   const int F = face_sites(g);
@@ -614,31 +687,28 @@ __global__ void k_sap_dd_pack(SapArgs a, DDGeom dg, void *dn, void *up) {
   face_site(g, side, f, chunk, s, n, y);
   const spinor<float> v = Store<float>::load_spinor(a.phi[0], chunk, s, g.vbh);
   vec3<float> h0, h1;
-  if (side == 0) {
-    dd_proj_fwd<float>(v, h0, h1);
-    Half<float>::store(dn, F, f, h0, h1);
-  } else {
-    const su3<float> uu = P::blink(a.ub, chunk, 0, s, g.vbh, dg.x0off + g.L[0] - 1 == dg.N0 - 1);
-    dd_proj_bwd<float>(uu, v, h0, h1);
-    Half<float>::store(up, F, f, h0, h1);
-  }
+  eo_face_send<LP>(side, v, a.ub, g.vbh, chunk, s, dg.x0off + g.L[0] - 1 == dg.N0 - 1, h0, h1);
+  Half<float>::store(side == 0 ? dn : up, F, f, h0, h1);
 }
 
-template <class P>
+template <class LP>
 static void sap_bnd_launch(Ctx &c, SapArgs a, cudaStream_t st) {
   const size_t nb_sites = (size_t)(c.g.nbl / 2) * c.g.vb;
-  const unsigned nbnd = (unsigned)((nb_sites + 127) / 128);
+  const unsigned nbnd = (unsigned)((nb_sites + 63) / 64);   // 64 lane pairs per CTA
   DDGeom dg = c.ddg;
   if (!dd_on(c)) {
-    k_sap_bnd<P><<<nbnd * a.nsys, 128, 0, st>>>(a);
+    // one wave of the form with more registers, or the form with more CTAs
+    const unsigned n = nbnd * a.nsys;
+    if (n <= 5 * 148) k_sap_bnd<LP, 5><<<n, 128, 0, st>>>(a);
+    else k_sap_bnd<LP, 8><<<n, 128, 0, st>>>(a);
     return;
   }
   const int F = c.g.L[1] * c.g.L[2] * c.g.L[3];
-  k_sap_dd_pack<P><<<(unsigned)((2 * F + 127) / 128), 128, 0, st>>>(a, dg, c.dd.buf[0], c.dd.buf[1]);
+  k_sap_dd_pack<LP><<<(unsigned)((2 * F + 127) / 128), 128, 0, st>>>(a, dg, c.dd.buf[0], c.dd.buf[1]);
   if (dd_exchange(c, (size_t)F * 48, st)) return;
   dg.hup = c.dd.buf[2];
   dg.hdn = c.dd.buf[3];
-  k_sap_bnd_dd<P><<<nbnd, 128, 0, st>>>(a, dg);
+  k_sap_bnd_dd<LP><<<nbnd, 128, 0, st>>>(a, dg);
 }
 
 // dynamic shared memory a block kernel may use (of 227 KB per CTA)
@@ -652,6 +722,31 @@ static int pick_threads(int vbh, int &ns) {
   }
   ns = 0;
   return 0;
+}
+
+// Launch variants of the even-odd block kernel: sites per lane pair, the
+// launch bound and the register budget it implies.  The autotuner below
+// times every variant that fits the block on the resident fields and keeps
+// the fastest per block size and storage mode.
+struct EoVariant {
+  int ns, maxt;
+  void (*k[3])(SapArgs);   // per storage mode
+};
+#define EO_KERNELS(NS, MAXT, MINB)                                                                      \
+  {k_sap_blocks_eo<NS, EoFull, SapF32, MAXT, MINB>, k_sap_blocks_eo<NS, EoHalf, SapF16, MAXT, MINB>,     \
+   k_sap_blocks_eo<NS, EoTwoRow, SapF32, MAXT, MINB>}
+static const EoVariant kEo[] = {
+    {1, 256, EO_KERNELS(1, 256, 2)}, {1, 512, EO_KERNELS(1, 512, 1)}, {2, 672, EO_KERNELS(2, 672, 1)},
+    {3, 448, EO_KERNELS(3, 448, 1)}, {3, 512, EO_KERNELS(3, 512, 1)},
+};
+static const int kNEo = sizeof(kEo) / sizeof(kEo[0]);
+
+static size_t eo_smem(int vbh) { return (size_t)(((vbh + 7) & ~7) + 8) * 2 * EO_SREC * sizeof(float4); }
+// threads of a variant, 0 if it does not fit the block size
+static int eo_threads(const EoVariant &v, int vbh) {
+  if (eo_smem(vbh) > (size_t)SAP_SMEM_MAX) return 0;
+  const int t = 32 * ((vbh + 16 * v.ns - 1) / (16 * v.ns));
+  return t > v.maxt ? 0 : t;
 }
 
 // FP16 copies of the FP32 links and Pauli matrices, same plane indexing
@@ -687,7 +782,7 @@ static int sap_half_fields(Ctx &c, cudaStream_t st) {
 // link satisfies row3 = conj(row1 x row2) to FP32 accuracy, with the sign
 // flipped on the time links at x0 = N0-1 (the antiperiodic boundary phase
 // of bc type 3); bad[0] counts links that do not.
-__global__ void k_links12(Geom g, DDGeom dg, size_t nlink, const float2 *__restrict__ u32, float2 *u12, int *bad) {
+__global__ void k_links12(Geom g, DDGeom dg, size_t nlink, const float2 *__restrict__ u32, float4 *u12, int *bad) {
   const int vbh = g.vbh;
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= nlink) return;
@@ -701,9 +796,9 @@ __global__ void k_links12(Geom g, DDGeom dg, size_t nlink, const float2 *__restr
   float2 e[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) e[k] = p[(size_t)k * vbh];
-  float2 *q = u12 + cm * 6 * vbh + s;
+  float4 *q = u12 + cm * 3 * vbh + s;
 #pragma unroll
-  for (int k = 0; k < 6; k++) q[(size_t)k * vbh] = e[k];
+  for (int j = 0; j < 3; j++) q[(size_t)j * vbh] = make_float4(e[2 * j].x, e[2 * j].y, e[2 * j + 1].x, e[2 * j + 1].y);
   float dp = 0.0f, dm = 0.0f;
 #pragma unroll
   for (int j = 0; j < 3; j++) {
@@ -724,7 +819,7 @@ static int sap_link12_fields(Ctx &c, cudaStream_t st) {
   int *bad = nullptr;
   if (cudaMallocAsync(&bad, sizeof(int), st) != cudaSuccess) return fail("out of device memory");
   cudaMemsetAsync(bad, 0, sizeof(int), st);
-  k_links12<<<(unsigned)((nlink + 255) / 256), 256, 0, st>>>(c.g, c.ddg, nlink, c.u32, (float2 *)c.u12, bad);
+  k_links12<<<(unsigned)((nlink + 255) / 256), 256, 0, st>>>(c.g, c.ddg, nlink, c.u32, (float4 *)c.u12, bad);
   int h = 0;
   cudaMemcpyAsync(&h, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
   cudaFreeAsync(bad, st);
@@ -751,29 +846,6 @@ static int sap_mode(Ctx &c, int isolv, cudaStream_t st) {
   if (sap_link12_fields(c, st)) return -1;
   return c.u12_ok ? 2 : 0;
 }
-
-// Launch variants of the even-odd block kernel: sites per thread, the
-// launch bound and the register budget it implies.  The autotuner below
-// times every variant that fits the block on the resident fields and keeps
-// the fastest per block size and storage mode.
-struct EoVariant {
-  int ns, maxt;
-  void (*k[3])(SapArgs);   // per storage mode
-};
-static const EoVariant kEo[] = {
-    {1, 256, {k_sap_blocks_eo<1, SapF32, 256, 2>, k_sap_blocks_eo<1, SapF16, 256, 2>, k_sap_blocks_eo<1, SapF32R, 256, 2>}},
-    {1, 672, {k_sap_blocks_eo<1, SapF32, 672, 1>, k_sap_blocks_eo<1, SapF16, 672, 1>, k_sap_blocks_eo<1, SapF32R, 672, 1>}},
-    {2, 384, {k_sap_blocks_eo<2, SapF32, 384, 1>, k_sap_blocks_eo<2, SapF16, 384, 1>, k_sap_blocks_eo<2, SapF32R, 384, 1>}},
-    {3, 256, {k_sap_blocks_eo<3, SapF32, 256, 1>, k_sap_blocks_eo<3, SapF16, 256, 1>, k_sap_blocks_eo<3, SapF32R, 256, 1>}},
-};
-static const int kNEo = sizeof(kEo) / sizeof(kEo[0]);
-
-static int eo_threads(const EoVariant &v, int vbh) {
-  int t = ((vbh + v.ns - 1) / v.ns + 31) / 32 * 32;
-  return t > v.maxt ? 0 : t;
-}
-
-static size_t eo_smem(int vbh) { return (size_t)vbh * 72 * sizeof(float); }
 
 static void launch_blocks(Ctx &c, const SapArgs &a, int isolv, int mode, cudaStream_t st) {
   const int nbh = c.g.nbl / 2;
@@ -816,10 +888,13 @@ static SapArgs sap_args(Ctx &c, float mu, int nmr, int mode, void *psi, void *rh
 // MR steps, on a random residual) and keep the fastest.
 static int sap_autotune(Ctx &c, int mode, cudaStream_t st) {
   if (c.sap_tuned_vbh[mode] == c.g.vbh) return 0;
-  for (int i = 0; i < kNEo; i++)
+  bool fits = false;
+  for (int i = 0; i < kNEo; i++) {
     for (int m = 0; m < 3; m++)
       cudaFuncSetAttribute(kEo[i].k[m], cudaFuncAttributeMaxDynamicSharedMemorySize, SAP_SMEM_MAX);
-  if (eo_smem(c.g.vbh) > (size_t)SAP_SMEM_MAX) return fail("sap: block too large for shared memory");
+    fits |= eo_threads(kEo[i], c.g.vbh) != 0;
+  }
+  if (!fits) return fail("sap: block too large for shared memory");
   const size_t nb = spinor_bytes(c, 32);
   void *psi = nullptr, *rho = nullptr, *phi = nullptr;
   if (cudaMallocAsync(&psi, nb, st) != cudaSuccess || cudaMallocAsync(&rho, nb, st) != cudaSuccess ||
@@ -879,9 +954,9 @@ int sap_set_variant(Ctx &c, int v) {
     c.sap_tuned_vbh[mode] = 0;
     return 0;
   }
-  if (v >= kNEo || !eo_threads(kEo[v], c.g.vbh)) return fail("sap: this launch variant does not fit the block size");
-  for (int m = 0; m < 3; m++)
-    cudaFuncSetAttribute(kEo[v].k[m], cudaFuncAttributeMaxDynamicSharedMemorySize, SAP_SMEM_MAX);
+  if (v >= kNEo || !eo_threads(kEo[v], c.g.vbh))
+    return fail("sap: this launch variant does not fit the block size");
+  cudaFuncSetAttribute(kEo[v].k[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, SAP_SMEM_MAX);
   c.sap_variant[mode] = v;
   c.sap_tuned_vbh[mode] = c.g.vbh;
   c.sap_tuned_ms[mode] = 0.0f;
@@ -921,15 +996,19 @@ static int sap_ready(Ctx &c, int isolv, cudaStream_t st) {
   return mode;
 }
 
-// the launches of one cycle: block solves and boundary updates, colour 0
-// then colour 1 (sap.c:720)
-static void sap_cycle_launch(Ctx &c, SapArgs a, int isolv, int mode, cudaStream_t st) {
-  for (int ic = 0; ic < 2; ic++) {
-    a.colour = ic;
+// the launches of ncy cycles: per cycle the block solves and boundary
+// updates of colour 0, then of colour 1 (sap.c:720).  (A block kernel that
+// gathered the other colour's boundary hops itself before it solved its
+// blocks was tried: 78 against 80 us per cycle on 16^4, but 806 against 788 us
+// on 32^4 and 7 % slower with 6^4 blocks, for want of warps to hide the
+// gather's latency.)
+static void sap_cycles_launch(Ctx &c, SapArgs a, int isolv, int mode, int ncy, cudaStream_t st) {
+  for (int n = 0; n < 2 * ncy; n++) {
+    a.colour = n & 1;
     launch_blocks(c, a, isolv, mode, st);
-    if (mode == 1) sap_bnd_launch<SapF16>(c, a, st);
-    else if (mode == 2) sap_bnd_launch<SapF32R>(c, a, st);
-    else sap_bnd_launch<SapF32>(c, a, st);
+    if (mode == 1) sap_bnd_launch<EoHalf>(c, a, st);
+    else if (mode == 2) sap_bnd_launch<EoTwoRow>(c, a, st);
+    else sap_bnd_launch<EoFull>(c, a, st);
   }
 }
 
@@ -962,7 +1041,7 @@ int sap_cycles(Ctx &c, float mu, int isolv, int nmr, int ncy, void *psi, void *r
   const int mode = sap_ready(c, isolv, st);
   if (mode < 0) return -1;
   const SapArgs a = sap_args(c, mu, nmr, mode, psi, rho, phi_blk);
-  for (int n = 0; n < ncy; n++) sap_cycle_launch(c, a, isolv, mode, st);
+  sap_cycles_launch(c, a, isolv, mode, ncy, st);
   return cudaGetLastError() == cudaSuccess ? 0 : fail("sap: launch failed");
 }
 
@@ -988,7 +1067,7 @@ int sap_cycles_multi(Ctx &c, int n, float mu, int isolv, int nmr, int ncy, void 
       a.phi[r] = (float4 *)phi_blk[r0 + r];
       a.mus[r] = mu;
     }
-    for (int k = 0; k < ncy; k++) sap_cycle_launch(c, a, isolv, mode, st);
+    sap_cycles_launch(c, a, isolv, mode, ncy, st);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : fail("sap: launch failed");
 }
@@ -1043,7 +1122,7 @@ int sap_mop(Ctx &c, float mu, int isolv, int nmr, int ncy, const void *rh, void 
   if (rh != srho) la_copy(c, 32, rh, 32, srho, PAR_ALL, st);
   const int rc = graph_run(c, &key, sizeof(key), st, [&]() {
     la_zero(c, 32, spsi, PAR_ALL, st);
-    for (int n = 0; n < ncy; n++) sap_cycle_launch(c, key.a, isolv, mode, st);
+    sap_cycles_launch(c, key.a, isolv, mode, ncy, st);
     return cudaGetLastError() == cudaSuccess ? 0 : fail("sap: launch failed");
   });
   if (rc) return -1;
@@ -1125,7 +1204,7 @@ int sap_mop_multi(Ctx &c, int ns, const float *mu, int isolv, int nmr, int ncy, 
     }
     const int rc = graph_run(c, &key, sizeof(key), st, [&]() {
       cudaMemsetAsync(c.sap_mfld[0], 0, (size_t)m * fb, st);
-      for (int k = 0; k < ncy; k++) sap_cycle_launch(c, key.a, isolv, mode, st);
+      sap_cycles_launch(c, key.a, isolv, mode, ncy, st);
       return cudaGetLastError() == cudaSuccess ? 0 : fail("sap: launch failed");
     });
     if (rc) return -1;
@@ -1149,7 +1228,7 @@ int sap_mop_multi(Ctx &c, int ns, const float *mu, int isolv, int nmr, int ncy, 
 int sap_cycle(Ctx &c, float mu, int isolv, int nmr, void *psi, void *rho, void *phi_blk, cudaStream_t st) {
   const int mode = sap_ready(c, isolv, st);
   if (mode < 0) return -1;
-  sap_cycle_launch(c, sap_args(c, mu, nmr, mode, psi, rho, phi_blk), isolv, mode, st);
+  sap_cycles_launch(c, sap_args(c, mu, nmr, mode, psi, rho, phi_blk), isolv, mode, 1, st);
   return cudaGetLastError() == cudaSuccess ? 0 : fail("sap: launch failed");
 }
 

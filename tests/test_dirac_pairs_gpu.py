@@ -1,0 +1,52 @@
+"""The FP32 operators with two lanes per site on blocks whose sites do not
+fill a warp's 16 pairs, with 12-real and 18-real links: every operator, the
+residual-update form, and the host pipeline's block lists, against the CPU
+restatement (oracle/qcd_oracle.c, modules/dirac/Dw.c:973)."""
+import numpy as np
+import pytest
+
+import openqcd_b200 as qb
+import oracle as O
+from helpers import OPS, site_rel_err
+
+pytestmark = pytest.mark.gpu
+
+MU = 0.07
+TOL = 2e-6      # FP32 rounding of one operator, the bar of the other parity tests
+
+SHAPES = [((4, 4, 4, 4), (2, 2, 2, 2)), ((8, 4, 4, 12), (4, 2, 2, 6)), ((8, 12, 8, 8), (4, 6, 4, 4)),
+          ((12, 12, 12, 12), (6, 6, 6, 6))]
+
+
+@pytest.mark.parametrize("L,bs", SHAPES, ids=["x".join(map(str, b)) for _, b in SHAPES])
+@pytest.mark.parametrize("eoflg", [0, 1])
+def test_fp32_operators(L, bs, eoflg):
+    ipt = qb.even_first_ipt(L)
+    V = ipt.size
+    qb.geometry(L, bs, ipt)
+    qb.set_parms(1.5, 0.0, eoflg)
+    qb.random_ud(0.4, 99)
+    assert qb.sw_term() == 0
+    U = O.links_ref2lex(qb.download_ud(V), ipt, L)
+    sw = [O.pauli_ref2lex(qb.download_swd(V, k), ipt) for k in (0, 1)]
+    g = np.random.default_rng(3)
+    s, r0 = (g.standard_normal(24 * V).astype(np.float32) for _ in range(2))
+    ref = {op: O.spinor_lex2ref(O.dirac(L, k, MU, eoflg, U, sw[0], sw[1], O.spinor_ref2lex(s, ipt),
+                                        O.spinor_ref2lex(r0, ipt)), ipt) for k, op in enumerate(OPS)}
+    try:
+        for l12 in (1, 0):
+            qb.set_sap_link12(l12)
+            assert not l12 or qb.links12_active()
+            for op in OPS:
+                assert site_rel_err(qb.dirac_ref(op, 32, MU, s, r0), ref[op], V) <= TOL, (op, l12)
+            S, B, R = qb.DevField(32).from_ref(s), qb.DevField(32).from_ref(r0), qb.DevField(32)
+            qb.dev_dirac_multi(MU, [S], [R], [B])
+            assert site_rel_err(R.to_ref(V), r0 - ref["Dw"], V) <= TOL
+            hs, hr = qb.HostArray(24 * V, np.float32), qb.HostArray(24 * V, np.float32)
+            hs.a[:] = s
+            qb.lib().Dw(MU, hs.ptr, hr.ptr)
+            assert np.array_equal(np.array(hr.a), qb.dirac_ref("Dw", 32, MU, s))
+            hs.free()
+            hr.free()
+    finally:
+        qb.set_sap_link12(1)
