@@ -252,12 +252,8 @@ void flat_cscale(Ctx &c, double2 *y, size_t n, double a) {
 }
 
 int flat_scratch(Ctx &c, double **scratch, double **out) {
-  if (!c.red) {
-    if (cudaMalloc(&c.red, (size_t)FB * 4 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&c.red_out, 8 * sizeof(double)) != cudaSuccess ||
-        cudaMallocHost(&c.h_red, 8 * sizeof(double)) != cudaSuccess)
-      return fail("out of memory (reduction buffers)");
-  }
+  static_assert(FB <= LA_RB, "the shared reduction buffer holds LA_RB blocks");
+  if (la_buffers(c)) return -1;
   *scratch = c.red;
   *out = c.red_out;
   return 0;

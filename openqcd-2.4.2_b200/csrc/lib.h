@@ -180,9 +180,11 @@ struct Ctx {
   void *stage = nullptr;        // staging buffer for reference-layout transfers
   size_t stage_bytes = 0;
   double *red = nullptr;        // reduction partials
-  double *red_out = nullptr;    // reduction results (device)
-  double *h_red = nullptr;      // pinned host mirror of red_out
-  int red_blocks = 0;
+  double *red_out = nullptr;    // reduction results (device) of blas.cu
+  unsigned *red_cnt = nullptr;  // blocks of the running reduction that are done
+  double *h_red = nullptr;      // reduction results (page-locked, written by the device)
+  double2 *gcr_rec = nullptr, *h_gcr_rec = nullptr;   // products of a GCR step, device and page-locked
+  int gcr_n = 0;
   cudaStream_t stream = nullptr;
   // error flag of bounded waits in the operator kernels: page-locked host
   // memory mapped into the device (h_kerr host view, d_kerr device view)
@@ -287,9 +289,14 @@ size_t graphs_cached();
 // Reductions accumulate in double per thread and in double-double across
 // blocks, deterministically.
 enum { PAR_ALL = 2, PAR_EVEN = 0, PAR_ODD = 1 };
+constexpr int LA_RB = 1184;   // blocks of a reduction at most: 8 per SM on 148 SMs
+int la_buffers(Ctx &c);       // the reduction buffers, made once
 int la_norm2(Ctx &c, int prec, const void *x, int par, double *res_dd);                 // |x|^2 -> (hi,lo)
 int la_dot(Ctx &c, int prec, const void *x, const void *y, int par, double *res);       // (x,y) -> re,im (dd each)
 int la_unorm(Ctx &c, int prec, const void *x, int par, double *res);                    // max site norm
+struct cplxf { float re, im; };
+// one gcr_step (fgcr.c:157) on FP32 fields with its products kept on the device
+int la_gcr_step(Ctx &c, int k, void *const *chi, void *rho, cplxf *a, float *b, cplxf *cc, double *rn);
 int la_xr_norm2(Ctx &c, void *x, void *r, const void *p, const void *ap, double a, int par,
                 double *res_dd);                                 // FP64: x += a p, r -= a ap, |r|^2
 int la_mulg5_norm2(Ctx &c, void *x, int par, double *res_dd);    // FP64: x = g5 x, |x|^2
@@ -323,7 +330,6 @@ void la_lincomb32(const Ctx &c, void *y, int n, const float *cre, const float *c
 // solver.cu: the GCR recursion over an abstract set of FP32/FP64 field
 // operations, so the same code serves device-layout fields (sap_gcr) and
 // caller arrays (the generic fgcr drop-in).
-struct cplxf { float re, im; };
 struct KrylovOps {
   std::function<double(const void *, int)> res32;                 // get_res (fgcr.c:128)
   std::function<cplxf(const void *, const void *)> dot32;         // spinor_prod
@@ -336,6 +342,10 @@ struct KrylovOps {
   // y = sum of c[l] x[l], l = 0..n-1 in this order (optional: without it
   // the recursion zeroes y and applies one axpy32 per term)
   std::function<void(void *, int, const cplxf *, void *const *)> lincomb32;
+  // gcr_step after the preconditioner, with the 2-norm of the residual
+  // (optional): chi[0..k], rho -> a[l] = (chi_l, chi_k), b, c, |rho|; false
+  // if it failed
+  std::function<bool(int, void *const *, void *, cplxf *, float *, cplxf *, double *)> step32;
 };
 double fgcr_core(const KrylovOps &o, int nkv, int nmx, int istop, double res, const void *eta, void *psi,
                  int *status, const std::function<void(const void *, void *)> &Dop,

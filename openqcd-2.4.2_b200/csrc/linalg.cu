@@ -8,16 +8,19 @@
 // everything here works on flat arrays: FP64 fields as double2 (one complex
 // component), FP32 fields as float4 (two complex components).
 //
-// Reductions are two deterministic passes: a fixed grid of RB blocks sums in
-// double (per thread, then a fixed tree in the block), then one block adds
-// the RB partials in double-double (Knuth's TwoSum), so results are
-// bit-identical from run to run.
+// Reductions are two deterministic passes in one launch: a grid of at most
+// RB blocks (fixed by the field's size) sums in double (per thread, then a
+// fixed tree in the block), then the last block to finish adds the partials
+// in the order of the blocks in double-double (Knuth's TwoSum) and writes the
+// result to page-locked host memory, so results are bit-identical from run
+// to run and a reduction costs the host one launch and one wait.
+#include <cmath>
 #include <cstring>
 #include "lib.h"
 
 namespace qcd {
 
-static const int RB = 1184;   // 8 blocks per SM on 148 SMs
+static const int RB = LA_RB;
 static const int RT = 256;
 
 struct Range { size_t beg, n; };
@@ -56,35 +59,78 @@ __device__ __forceinline__ void block_store(double v[NC], double *out) {
   }
 }
 
-// final pass: out[2k], out[2k+1] = double-double sum of part[NC*b + k]
-template <int NC>
-__global__ void k_finish(const double *__restrict__ part, int nb, double *out) {
-  __shared__ double hi[NC][32], lo[NC][32];
-  int t = threadIdx.x;   // 32 threads
+// (h, l) += (x, xl) in double-double (Knuth's TwoSum)
+__device__ __forceinline__ void dd_acc(double &h, double &l, double x, double xl) {
+  const double s = h + x, bb = s - h;
+  l += (h - (s - bb)) + (x - bb) + xl;
+  h = s;
+}
+
+// The second pass in the same launch: every block stores its NC partial sums
+// and the block that arrives last at the counter adds them all, in the order
+// of the blocks' indices whichever block that is, in double-double.  True in
+// thread 0 of that block only, with the sums in (hi, lo) pairs; the counter
+// is zero again for the next launch of the stream.  (As kernels of their own
+// the second pass and the copy of its result to the host cost two more
+// launches, about 10 us per reduction.)
+struct Fin {
+  double *part;
+  unsigned *cnt;
+};
+template <int NC> __device__ __forceinline__ bool block_last(const Fin &f) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(f.cnt, 1u) == gridDim.x - 1;
+    if (last) *f.cnt = 0u;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+template <int NC> __device__ __forceinline__ bool block_finish(double v[NC], const Fin &f, double (&hi)[NC], double (&lo)[NC]) {
+  __shared__ double sh[RT / 32][2 * NC];
+  block_store<NC>(v, f.part);
+  if (!block_last<NC>(f)) return false;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < NC; k++) hi[k] = lo[k] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += RT)
+#pragma unroll
+    for (int k = 0; k < NC; k++) dd_acc(hi[k], lo[k], __ldcg(f.part + (size_t)NC * b + k), 0.0);
+#pragma unroll
   for (int k = 0; k < NC; k++) {
-    double h = 0.0, l = 0.0;
-    for (int b = t; b < nb; b += 32) {
-      double x = part[(size_t)NC * b + k];
-      double s = h + x, bb = s - h;
-      l += (h - (s - bb)) + (x - bb);
-      h = s;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double h2 = __shfl_down_sync(0xffffffffu, hi[k], o), l2 = __shfl_down_sync(0xffffffffu, lo[k], o);
+      dd_acc(hi[k], lo[k], h2, l2);
     }
-    hi[k][t] = h;
-    lo[k][t] = l;
-  }
-  __syncwarp();
-  if (t < NC) {
-    double h = 0.0, l = 0.0;
-    for (int j = 0; j < 32; j++) {
-      double x = hi[t][j];
-      double s = h + x, bb = s - h;
-      l += (h - (s - bb)) + (x - bb) + lo[t][j];
-      h = s;
+    if (lane == 0) {
+      sh[w][2 * k] = hi[k];
+      sh[w][2 * k + 1] = lo[k];
     }
-    double s = h + l;
-    out[2 * t] = s;
-    out[2 * t + 1] = l - (s - h);
   }
+  __syncthreads();
+  if (threadIdx.x) return false;
+#pragma unroll
+  for (int k = 0; k < NC; k++) {
+    for (int j = 1; j < RT / 32; j++) dd_acc(hi[k], lo[k], sh[j][2 * k], sh[j][2 * k + 1]);
+    const double s = hi[k] + lo[k];
+    lo[k] -= s - hi[k];
+    hi[k] = s;
+  }
+  return true;
+}
+// the sums to out[2k], out[2k+1] (page-locked host memory)
+template <int NC> __device__ __forceinline__ void finish_to(double v[NC], const Fin &f, double *out) {
+  double hi[NC], lo[NC];
+  if (block_finish<NC>(v, f, hi, lo))
+#pragma unroll
+    for (int k = 0; k < NC; k++) {
+      out[2 * k] = hi[k];
+      out[2 * k + 1] = lo[k];
+    }
 }
 
 // FP32 fields: the products of one float4 (two complex components) are
@@ -92,9 +138,9 @@ __global__ void k_finish(const double *__restrict__ part, int nb, double *out) {
 // arithmetic made these reductions FP64-throughput bound on B200, at about
 // half their bandwidth-bound speed)
 template <typename R>
-__global__ void k_norm2(const void *__restrict__ x, Range r, double *part) {
+__global__ void k_norm2(const void *__restrict__ x, Range r, Fin f, double *out) {
   double v[1] = {0.0};
-  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < r.n; i += (size_t)RB * RT) {
+  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < r.n; i += (size_t)gridDim.x * RT) {
     if (sizeof(R) == 8) {
       double2 a = __ldg((const double2 *)x + r.beg + i);
       v[0] += a.x * a.x + a.y * a.y;
@@ -103,13 +149,13 @@ __global__ void k_norm2(const void *__restrict__ x, Range r, double *part) {
       v[0] += (double)(a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w);
     }
   }
-  block_store<1>(v, part);
+  finish_to<1>(v, f, out);
 }
 
 template <typename R>
-__global__ void k_dot(const void *__restrict__ x, const void *__restrict__ y, Range r, double *part) {
+__global__ void k_dot(const void *__restrict__ x, const void *__restrict__ y, Range r, Fin f, double *out) {
   double v[2] = {0.0, 0.0};
-  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < r.n; i += (size_t)RB * RT) {
+  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < r.n; i += (size_t)gridDim.x * RT) {
     if (sizeof(R) == 8) {
       double2 a = __ldg((const double2 *)x + r.beg + i), b = __ldg((const double2 *)y + r.beg + i);
       v[0] += a.x * b.x + a.y * b.y;
@@ -120,15 +166,15 @@ __global__ void k_dot(const void *__restrict__ x, const void *__restrict__ y, Ra
       v[1] += (double)(a.x * b.y - a.y * b.x + a.z * b.w - a.w * b.z);
     }
   }
-  block_store<2>(v, part);
+  finish_to<2>(v, f, out);
 }
 
 // uniform norm: max over sites of the spinor norm (sflds/unorm.c)
 template <typename R>
-__global__ void k_unorm(Geom g, const void *__restrict__ x, int c0, int nch, double *part) {
+__global__ void k_unorm(Geom g, const void *__restrict__ x, int c0, int nch, Fin f, double *out) {
   double m = 0.0;
   size_t nsite = (size_t)nch * g.vbh;
-  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < nsite; i += (size_t)RB * RT) {
+  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < nsite; i += (size_t)gridDim.x * RT) {
     int chunk = c0 + (int)(i / g.vbh), s = (int)(i % g.vbh);
     spinor<R> v = Store<R>::load_spinor(x, chunk, s, g.vbh);
     double n2 = 0.0;
@@ -146,52 +192,58 @@ __global__ void k_unorm(Geom g, const void *__restrict__ x, int c0, int nch, dou
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int w = 0; w < RT / 32; w++) t = fmax(t, sh[w]);
-    part[blockIdx.x] = t;
+    f.part[blockIdx.x] = t;
+  }
+  if (!block_last<1>(f) || threadIdx.x >= 32) return;
+  m = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) m = fmax(m, __ldcg(f.part + b));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+  if (threadIdx.x == 0) {
+    out[0] = sqrt(m);
+    out[1] = 0.0;
   }
 }
 
-__global__ void k_max_finish(const double *__restrict__ part, int nb, double *out) {
-  double m = 0.0;
-  for (int b = threadIdx.x; b < nb; b += 32) m = fmax(m, part[b]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  if (threadIdx.x == 0) { out[0] = sqrt(m); out[1] = 0.0; }
-}
-
-static int ensure_red(Ctx &c) {
+int la_buffers(Ctx &c) {
   if (c.red) return 0;
   if (cudaMalloc(&c.red, (size_t)RB * 4 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c.red_out, 8 * sizeof(double)) != cudaSuccess ||
+      cudaMalloc(&c.red_cnt, sizeof(unsigned)) != cudaSuccess ||
       cudaMallocHost(&c.h_red, 8 * sizeof(double)) != cudaSuccess)
     return fail("out of memory (reduction buffers)");
-  c.red_blocks = RB;
+  cudaMemsetAsync(c.red_cnt, 0, sizeof(unsigned), c.stream);
   return 0;
 }
+static Fin fin(const Ctx &c) { return Fin{c.red, c.red_cnt}; }
+// blocks of a reduction over n elements: at most RB, none without work
+static unsigned rgrid(size_t n) {
+  const size_t b = (n + RT - 1) / RT;
+  return (unsigned)(b < 1 ? 1 : (b < (size_t)RB ? b : (size_t)RB));
+}
 
-// the nc (hi, lo) results of this rank, then (domain decomposition) their
-// sum or maximum over the ranks, the same on every rank
+// the nc (hi, lo) results of this rank, which the kernel wrote to h_red,
+// then (domain decomposition) their sum or maximum over the ranks, the same
+// on every rank
 static int finish(Ctx &c, int nc, double *res, bool is_max = false) {
-  cudaMemcpyAsync(c.h_red, c.red_out, 2 * nc * sizeof(double), cudaMemcpyDeviceToHost, c.stream);
   if (cudaStreamSynchronize(c.stream) != cudaSuccess) return fail("reduction: CUDA error");
   for (int k = 0; k < 2 * nc; k++) res[k] = c.h_red[k];
   return dd_on(c) ? dd_global(c, res, nc, is_max) : 0;
 }
 
 int la_norm2(Ctx &c, int prec, const void *x, int par, double *res) {
-  if (ensure_red(c)) return -1;
+  if (la_buffers(c)) return -1;
   Range r = range(c, prec, par);
-  if (prec == 64) k_norm2<double><<<RB, RT, 0, c.stream>>>(x, r, c.red);
-  else k_norm2<float><<<RB, RT, 0, c.stream>>>(x, r, c.red);
-  k_finish<1><<<1, 32, 0, c.stream>>>(c.red, RB, c.red_out);
+  if (prec == 64) k_norm2<double><<<rgrid(r.n), RT, 0, c.stream>>>(x, r, fin(c), c.h_red);
+  else k_norm2<float><<<rgrid(r.n), RT, 0, c.stream>>>(x, r, fin(c), c.h_red);
   return finish(c, 1, res);
 }
 
 int la_dot(Ctx &c, int prec, const void *x, const void *y, int par, double *res) {
-  if (ensure_red(c)) return -1;
+  if (la_buffers(c)) return -1;
   Range r = range(c, prec, par);
-  if (prec == 64) k_dot<double><<<RB, RT, 0, c.stream>>>(x, y, r, c.red);
-  else k_dot<float><<<RB, RT, 0, c.stream>>>(x, y, r, c.red);
-  k_finish<2><<<1, 32, 0, c.stream>>>(c.red, RB, c.red_out);
+  if (prec == 64) k_dot<double><<<rgrid(r.n), RT, 0, c.stream>>>(x, y, r, fin(c), c.h_red);
+  else k_dot<float><<<rgrid(r.n), RT, 0, c.stream>>>(x, y, r, fin(c), c.h_red);
   return finish(c, 2, res);
 }
 
@@ -199,10 +251,10 @@ int la_dot(Ctx &c, int prec, const void *x, const void *y, int par, double *res)
 // multi-shift solver (modules/linsolv/mscg.c:242-275, cg_step2 with the norm
 // of cg_step3) in one pass
 __global__ void k_xr_norm2(Range rg, double2 *__restrict__ x, double2 *__restrict__ r,
-                           const double2 *__restrict__ p, const double2 *__restrict__ ap, double a,
-                           double *part) {
+                           const double2 *__restrict__ p, const double2 *__restrict__ ap, double a, Fin f,
+                           double *out) {
   double v[1] = {0.0};
-  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < rg.n; i += (size_t)RB * RT) {
+  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < rg.n; i += (size_t)gridDim.x * RT) {
     const size_t j = rg.beg + i;
     const double2 pp = __ldg(p + j), aa = __ldg(ap + j);
     double2 xx = x[j], rr = r[j];
@@ -214,24 +266,23 @@ __global__ void k_xr_norm2(Range rg, double2 *__restrict__ x, double2 *__restric
     r[j] = rr;
     v[0] += rr.x * rr.x + rr.y * rr.y;
   }
-  block_store<1>(v, part);
+  finish_to<1>(v, f, out);
 }
 
 int la_xr_norm2(Ctx &c, void *x, void *r, const void *p, const void *ap, double a, int par, double *res) {
-  if (ensure_red(c)) return -1;
+  if (la_buffers(c)) return -1;
   Range rg = range(c, 64, par);
-  k_xr_norm2<<<RB, RT, 0, c.stream>>>(rg, (double2 *)x, (double2 *)r, (const double2 *)p, (const double2 *)ap, a,
-                                      c.red);
-  k_finish<1><<<1, 32, 0, c.stream>>>(c.red, RB, c.red_out);
+  k_xr_norm2<<<rgrid(rg.n), RT, 0, c.stream>>>(rg, (double2 *)x, (double2 *)r, (const double2 *)p, (const double2 *)ap, a,
+                                               fin(c), c.h_red);
   return finish(c, 1, res);
 }
 
 // x -> gamma5 x on a parity range of an FP64 field (spin components 2, 3 of
 // every site change sign: double2 planes 6..11 of a chunk), then |x|^2
-__global__ void k_mulg5_norm2(Range rg, double2 *__restrict__ x, int vbh, double *part) {
+__global__ void k_mulg5_norm2(Range rg, double2 *__restrict__ x, int vbh, Fin f, double *out) {
   double v[1] = {0.0};
   const size_t per = (size_t)12 * vbh;
-  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < rg.n; i += (size_t)RB * RT) {
+  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < rg.n; i += (size_t)gridDim.x * RT) {
     const size_t j = rg.beg + i;
     double2 xx = x[j];
     if ((j % per) / vbh >= 6) {
@@ -241,25 +292,119 @@ __global__ void k_mulg5_norm2(Range rg, double2 *__restrict__ x, int vbh, double
     }
     v[0] += xx.x * xx.x + xx.y * xx.y;
   }
-  block_store<1>(v, part);
+  finish_to<1>(v, f, out);
 }
 
 int la_mulg5_norm2(Ctx &c, void *x, int par, double *res) {
-  if (ensure_red(c)) return -1;
+  if (la_buffers(c)) return -1;
   Range rg = range(c, 64, par);
-  k_mulg5_norm2<<<RB, RT, 0, c.stream>>>(rg, (double2 *)x, c.g.vbh, c.red);
-  k_finish<1><<<1, 32, 0, c.stream>>>(c.red, RB, c.red_out);
+  k_mulg5_norm2<<<rgrid(rg.n), RT, 0, c.stream>>>(rg, (double2 *)x, c.g.vbh, fin(c), c.h_red);
   return finish(c, 1, res);
 }
 
 int la_unorm(Ctx &c, int prec, const void *x, int par, double *res) {
-  if (ensure_red(c)) return -1;
+  if (la_buffers(c)) return -1;
   int c0 = par == PAR_ODD ? c.g.nbl : 0;
   int nch = par == PAR_ALL ? 2 * c.g.nbl : c.g.nbl;
-  if (prec == 64) k_unorm<double><<<RB, RT, 0, c.stream>>>(c.g, x, c0, nch, c.red);
-  else k_unorm<float><<<RB, RT, 0, c.stream>>>(c.g, x, c0, nch, c.red);
-  k_max_finish<<<1, 32, 0, c.stream>>>(c.red, RB, c.red_out);
+  const unsigned nb = rgrid((size_t)nch * c.g.vbh);
+  if (prec == 64) k_unorm<double><<<nb, RT, 0, c.stream>>>(c.g, x, c0, nch, fin(c), c.h_red);
+  else k_unorm<float><<<nb, RT, 0, c.stream>>>(c.g, x, c0, nch, fin(c), c.h_red);
   return finish(c, 1, res, true);
+}
+
+// ---------------------------------------------- one step of the flexible GCR
+// gcr_step of modules/linsolv/fgcr.c:157 (modified Gram-Schmidt of chi_k
+// against chi_0..chi_{k-1}, normalisation, update of the residual rho) with
+// its coefficients kept on the device: pass l subtracts the product of pass
+// l-1 and forms the next one, so the step is k + 3 launches and one wait of
+// the host, where launches, a wait and an update per product took k + 3 waits
+// of about 25 us: sap_gcr on 8^4 2.86 -> 2.35 ms, on 32x16^3 13.7 -> 11.3 ms.  The arithmetic is that of
+// la_dot, la_norm2, la_axpy and la_scale with the host's roundings between.
+// rec[l] (l < k) = (chi_l, chi_k), rec[k] = |chi_k|^2, rec[k+1] = (chi_k,
+// rho), rec[k+2] = |rho|^2, on the device and in page-locked memory.
+enum { GS_DOT, GS_NORM, GS_SCALE };
+// y -= z xp (z = *zp rounded to FP32) or, with GS_SCALE, y /= |y| (|y|^2 =
+// *zp); then (xn, y), |y|^2 (GS_NORM) or (y, xn) (GS_SCALE)
+template <int MODE>
+__global__ void __launch_bounds__(RT) k_gcr_pass(size_t n, float4 *y, const float4 *__restrict__ xp,
+                                                 const double2 *zp, const float4 *__restrict__ xn, Fin f, double2 *rec,
+                                                 double2 *hrec) {
+  constexpr int NC = MODE == GS_NORM ? 1 : 2;
+  float zr = 0.0f, zi = 0.0f;
+  bool upd = xp != nullptr;
+  if (MODE == GS_SCALE) {
+    const float nn = (float)sqrt((double)(float)zp->x);
+    upd = nn != 0.0f;
+    zr = upd ? 1.0f / nn : 1.0f;
+  } else if (upd) {
+    zr = -(float)zp->x;
+    zi = -(float)zp->y;
+  }
+  double v[NC];
+#pragma unroll
+  for (int k = 0; k < NC; k++) v[k] = 0.0;
+  for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < n; i += (size_t)gridDim.x * RT) {
+    float4 b = y[i];
+    if (MODE == GS_SCALE) {
+      b = make_float4(zr * b.x, zr * b.y, zr * b.z, zr * b.w);
+    } else if (upd) {
+      const float4 a = __ldg(xp + i);
+      b.x += zr * a.x - zi * a.y;
+      b.y += zr * a.y + zi * a.x;
+      b.z += zr * a.z - zi * a.w;
+      b.w += zr * a.w + zi * a.z;
+    }
+    if (upd) y[i] = b;
+    if (MODE == GS_NORM) {
+      v[0] += (double)(b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w);
+    } else {
+      const float4 x = __ldg(xn + i);
+      v[0] += (double)(x.x * b.x + x.y * b.y + x.z * b.z + x.w * b.w);
+      const double im = (double)(x.x * b.y - x.y * b.x + x.z * b.w - x.w * b.z);
+      v[NC - 1] += MODE == GS_SCALE ? -im : im;   // (xn, y) or (y, xn)
+    }
+  }
+  double hi[NC], lo[NC];
+  if (block_finish<NC>(v, f, hi, lo)) {
+    const double2 r = make_double2(hi[0] + lo[0], NC == 2 ? hi[NC - 1] + lo[NC - 1] : 0.0);
+    *rec = r;
+    *hrec = r;
+  }
+}
+
+// chi[0..k], rho: FP32 fields.  On return chi[k] is normalised and rho
+// reduced; a[l], b, cc and rn are those of gcr_step.
+int la_gcr_step(Ctx &c, int k, void *const *chi, void *rho, cplxf *a, float *b, cplxf *cc, double *rn) {
+  if (la_buffers(c)) return -1;
+  if (c.gcr_n < k + 3) {
+    cudaFree(c.gcr_rec);
+    cudaFreeHost(c.h_gcr_rec);
+    c.gcr_rec = c.h_gcr_rec = nullptr;
+    c.gcr_n = 0;
+    const int m = k + 3 < 64 ? 64 : k + 3 + 64;
+    if (cudaMalloc(&c.gcr_rec, m * sizeof(double2)) != cudaSuccess ||
+        cudaMallocHost(&c.h_gcr_rec, m * sizeof(double2)) != cudaSuccess)
+      return fail("out of memory (GCR record)");
+    c.gcr_n = m;
+  }
+  const size_t n = range(c, 32, PAR_ALL).n;
+  const unsigned nb = rgrid(n);
+  const Fin f = fin(c);
+  double2 *r = c.gcr_rec, *h = c.h_gcr_rec;
+  float4 *y = (float4 *)chi[k], *rh = (float4 *)rho;
+  for (int l = 0; l < k; l++)
+    k_gcr_pass<GS_DOT><<<nb, RT, 0, c.stream>>>(n, y, l ? (const float4 *)chi[l - 1] : nullptr, l ? r + l - 1 : nullptr,
+                                                (const float4 *)chi[l], f, r + l, h + l);
+  k_gcr_pass<GS_NORM><<<nb, RT, 0, c.stream>>>(n, y, k ? (const float4 *)chi[k - 1] : nullptr, k ? r + k - 1 : nullptr,
+                                               nullptr, f, r + k, h + k);
+  k_gcr_pass<GS_SCALE><<<nb, RT, 0, c.stream>>>(n, y, nullptr, r + k, rh, f, r + k + 1, h + k + 1);
+  k_gcr_pass<GS_NORM><<<nb, RT, 0, c.stream>>>(n, rh, y, r + k + 1, nullptr, f, r + k + 2, h + k + 2);
+  if (cudaStreamSynchronize(c.stream) != cudaSuccess) return fail("gcr step: CUDA error");
+  for (int l = 0; l < k; l++) a[l] = cplxf{(float)h[l].x, (float)h[l].y};
+  *b = (float)std::sqrt((double)(float)h[k].x);
+  *cc = cplxf{(float)h[k + 1].x, (float)h[k + 1].y};
+  *rn = std::sqrt((double)(float)h[k + 2].x);
+  return 0;
 }
 
 // ------------------------------------------------------------- elementwise

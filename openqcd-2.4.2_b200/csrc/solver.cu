@@ -35,7 +35,7 @@ double fgcr_core(const KrylovOps &o, int nkv, int nmx, int istop, double res, co
     fail("fgcr: parameters are out of range");
     return -1.0;
   }
-  std::vector<cplxf> a((size_t)nkv * nkv), cc(nkv);
+  std::vector<cplxf> a((size_t)nkv * nkv), ak(nkv), cc(nkv);
   std::vector<float> b(nkv);
   const double PRECISION_LIMIT = (double)(100.0f * FLT_EPSILON);
 
@@ -51,15 +51,20 @@ double fgcr_core(const KrylovOps &o, int nkv, int nmx, int istop, double res, co
     for (k = 0;; k++) {
       // gcr_step (fgcr.c:157)
       Mop(k, rho, phi[k], chi[k]);
-      for (int l = 0; l < k; l++) {
-        cplxf z = o.dot32(chi[l], chi[k]);
-        a[(size_t)nkv * l + k] = z;
-        o.axpy32(chi[k], -z.re, -z.im, chi[l]);
+      if (o.step32 && istop == 0) {
+        if (!o.step32(k, chi.data(), rho, ak.data(), &b[k], &cc[k], &rn)) return -1.0;
+        for (int l = 0; l < k; l++) a[(size_t)nkv * l + k] = ak[l];
+      } else {
+        for (int l = 0; l < k; l++) {
+          cplxf z = o.dot32(chi[l], chi[k]);
+          a[(size_t)nkv * l + k] = z;
+          o.axpy32(chi[k], -z.re, -z.im, chi[l]);
+        }
+        b[k] = o.normalize32(chi[k]);
+        cc[k] = o.dot32(chi[k], rho);
+        o.axpy32(rho, -cc[k].re, -cc[k].im, chi[k]);
+        rn = o.res32(rho, istop);
       }
-      b[k] = o.normalize32(chi[k]);
-      cc[k] = o.dot32(chi[k], rho);
-      o.axpy32(rho, -cc[k].re, -cc[k].im, chi[k]);
-      rn = o.res32(rho, istop);
       status[0] += 1;
       if (rn <= tol || rn < PRECISION_LIMIT * rn_old || k == nkv - 1 || status[0] >= nmx) break;
     }
@@ -134,6 +139,11 @@ KrylovOps dev_krylov_ops(Ctx &c) {
     }
     la_lincomb32(c, y, n, re.data(), im.data(), x, st);
   };
+  // with domain decomposition every product is summed over the ranks by the host
+  if (!dd_on(c))
+    o.step32 = [&c](int k, void *const *chi, void *rho, cplxf *a, float *b, cplxf *cc, double *rn) {
+      return la_gcr_step(c, k, chi, rho, a, b, cc, rn) == 0;
+    };
   o.zero64 = [&c, st](void *x) { la_zero(c, 64, x, PAR_ALL, st); };
   o.copy64to32 = [&c, st](const void *x, void *y) { la_copy(c, 64, x, 32, y, PAR_ALL, st); };
   o.add32to64 = [&c, st](const void *s, void *d) { la_add_s2sd(c, s, d, PAR_ALL, st); };
