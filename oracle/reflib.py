@@ -43,7 +43,7 @@ def ensure_built(L, T=None, ref="/root/reference", portable=False):
     selects the reference's plain-C code paths (no AVX inline assembly)."""
     T = T or GEOMETRIES[tuple(L)]
     p = lib_path(L, T, portable)
-    if not os.path.exists(p) and os.path.isdir(ref):
+    if not os.path.exists(p) and os.path.isfile(os.path.join(ref, "include", "global.h")):
         import importlib.util
         spec = importlib.util.spec_from_file_location("build_ref", os.path.join(HERE, "build_ref.py"))
         m = importlib.util.module_from_spec(spec)
