@@ -609,7 +609,7 @@ def sustained_dw(qb, n, chunk=20):
 def scan_block_orders(qb):
     """Dw_dble on 32^3x64 under each block traversal order: first two
     launches per order (the launches a 10-launch ncu capture of
-    dirac_staged sees), then 3 x 20 timed launches per order."""
+    Dw_dble kernel sees), then 3 x 20 timed launches per order."""
     L = LATTICE
     qb.geometry(L, BS, qb.even_first_ipt(L))
     qb.set_parms(CSW, M0, 0)
@@ -1006,7 +1006,7 @@ def run_b200(args, d):
             "data": DATA if L == LATTICE else "synthetic (device-generated links exp(0.3 X), Gaussian source)",
             "config": bench_config(d.world) if L == LATTICE else {"workload": "Dw_dble profiling case",
                                                                   "lattice": list(L)},
-            "roofline": {"bound": "hbm", "kernel": "dirac_staged_kernel<OP_SW|OP_HOP, all sites> (Dw_dble, SW staged)",
+            "roofline": {"bound": "hbm", "kernel": "dirac_pair_kernel<OP_SW|OP_HOP, all sites, FP64> (Dw_dble, two lanes per site)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                          "bytes_per_launch": bytes_step},

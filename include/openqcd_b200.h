@@ -256,11 +256,9 @@ int b200_set_sap_link12(int on);
 /* 1 when the FP32 operators read 12-real links for the current gauge field
  * (on, and every link passed the check), 0 when they read 18 reals. */
 int b200_links12_active(void);
-/* mode != 0 (default): the FP64 operators with an SW term (all but
- * Dwoe_dble and Dweo_dble) stage each tile's SW matrices in shared memory
- * with bulk asynchronous copies; 0 reads them directly.  Same arithmetic,
- * identical results.  Returns the previous mode (no reference
- * counterpart). */
+/* Kept for its callers: the FP64 operators have one form, which reads the SW
+ * matrices directly, so both modes (0 and 1, the default) give identical
+ * results.  Returns the previous mode (no reference counterpart). */
 int b200_set_dw_staged(int mode);
 /* Traversal order of the blocks in the full-lattice operator kernels (no
  * reference counterpart; results do not depend on it, only how long a

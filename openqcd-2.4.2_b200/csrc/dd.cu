@@ -48,14 +48,9 @@ __global__ void k_dd_pack(Geom g, DDGeom dg, const void *__restrict__ t, const v
   face_site(g, side, f, chunk, s, n, y);
   const spinor<R> v = Store<R>::load_spinor(t, chunk, s, g.vbh);
   vec3<R> a, b;
-  if constexpr (sizeof(R) == 4) {
-    using LP = typename std::conditional<L12 != 0, EoTwoRow, EoFull>::type;
-    eo_face_send<LP>(side, v, u, g.vbh, chunk, s, dg.x0off + g.L[0] - 1 == dg.N0 - 1, a, b);
-  } else if (side == 0) {
-    dd_proj_fwd<R>(v, a, b);
-  } else {
-    dd_proj_bwd<R>(Store<R>::load_link(u, chunk, 0, s, g.vbh), v, a, b);
-  }
+  using LP32 = typename std::conditional<L12 != 0, EoTwoRow, EoFull>::type;
+  using LP = typename std::conditional<sizeof(R) == 8, EoDouble, LP32>::type;
+  eo_face_send<LP>(side, v, u, g.vbh, chunk, s, dg.x0off + g.L[0] - 1 == dg.N0 - 1, a, b);
   Half<R>::store(side == 0 ? dn : up, F, f, a, b);
 }
 

@@ -189,9 +189,7 @@ struct Ctx {
   // error flag of bounded waits in the operator kernels: page-locked host
   // memory mapped into the device (h_kerr host view, d_kerr device view)
   int *h_kerr = nullptr, *d_kerr = nullptr;
-  // FP64 operators with an SW term: SW matrices staged in shared memory by
-  // bulk copies (1) or read directly (0)
-  int dw_staged = 1;
+  int dw_staged = 1;            // b200_set_dw_staged's mode (without effect)
   // repeated launch sequences (the SAP preconditioner) run as CUDA graphs,
   // on three library-owned FP32 fields (solution, residual, block scratch)
   int use_graphs = 1;

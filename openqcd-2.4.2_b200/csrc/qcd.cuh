@@ -328,33 +328,6 @@ template <> struct Store<float> {
   }
 };
 
-// FP32 link stored as its first two rows (12 reals, three float4 planes of
-// two complex entries each, ((chunk*4 + mu)*3 + j)*vbh + s); the third row is rebuilt as the complex
-// conjugate of the cross product of the first two, exact for SU(3), and
-// negated for a link that carries the antiperiodic time-boundary sign
-// (neg).  The library checks every link for this relation, with the sign
-// its position implies, before it reads 12-real links.
-__device__ __forceinline__ su3<float> load_link12(const void *base, int chunk, int mu, int s, int vbh, bool neg) {
-  const float4 *p = (const float4 *)base + ((size_t)chunk * 4 + mu) * 3 * vbh + s;
-  su3<float> r;
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const float4 v = __ldg(p + (size_t)j * vbh);
-    r.e[2 * j] = mk<float>(v.x, v.y);
-    r.e[2 * j + 1] = mk<float>(v.z, v.w);
-  }
-  const float sg = neg ? -1.0f : 1.0f;
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const int a = (j + 1) % 3, b = (j + 2) % 3;
-    const cpx<float> x1 = r.e[a], y2 = r.e[3 + b], x2 = r.e[b], y1 = r.e[3 + a];
-    const float re = x1.re * y2.re - x1.im * y2.im - (x2.re * y1.re - x2.im * y1.im);
-    const float im = x1.re * y2.im + x1.im * y2.re - (x2.re * y1.im + x2.im * y1.re);
-    r.e[6 + j] = mk<float>(sg * re, -sg * im);
-  }
-  return r;
-}
-
 // ---------------------------------------------------------------- Pauli 6x6
 // The Hermitian 6x6 matrix is packed as in the reference
 // (modules/sw_term/pauli_dble.c:1336-1442 and set_aa :1644-1675): u[0..5] the
@@ -495,35 +468,6 @@ template <> struct Half<float> {
     p[2 * (size_t)F] = make_float4(h1.c[1].re, h1.c[1].im, h1.c[2].re, h1.c[2].im);
   }
 };
-
-// The x0 hops across a rank boundary, split where the two ranks meet.  The
-// forward hop U(x,0)(1 - g0) s(x+0) needs the neighbour's projection
-// h = (s1 + s3, s2 + s4) (the same sums hop_fwd forms); the backward hop
-// U(x-0,0)^dag (1 + g0) s(x-0) needs c = U^dag (s1 - s3, s2 - s4), which the
-// rank holding the link forms.  Same operations in the same order as
-// hop_fwd / hop_bwd with mu = 0, so the results are bit-identical.
-template <typename R>
-__device__ __forceinline__ void dd_proj_fwd(const spinor<R> &s, vec3<R> &h0, vec3<R> &h1) {
-  h0 = vadd(s.c[0], s.c[2]);
-  h1 = vadd(s.c[1], s.c[3]);
-}
-template <typename R>
-__device__ __forceinline__ void dd_proj_bwd(const su3<R> &u, const spinor<R> &s, vec3<R> &c0, vec3<R> &c1) {
-  c0 = udagmul(u, vsub(s.c[0], s.c[2]));
-  c1 = udagmul(u, vsub(s.c[1], s.c[3]));
-}
-template <typename R>
-__device__ __forceinline__ void dd_hop_fwd(const su3<R> &u, const vec3<R> &h0, const vec3<R> &h1, spinor<R> &acc) {
-  vec3<R> c = umul(u, h0);
-  vacc(acc.c[0], c); vacc(acc.c[2], c);
-  c = umul(u, h1);
-  vacc(acc.c[1], c); vacc(acc.c[3], c);
-}
-template <typename R>
-__device__ __forceinline__ void dd_hop_bwd(const vec3<R> &c0, const vec3<R> &c1, spinor<R> &acc) {
-  vacc(acc.c[0], c0); vdec(acc.c[2], c0);
-  vacc(acc.c[1], c1); vdec(acc.c[3], c1);
-}
 
 template <typename R> __device__ __forceinline__ void sscale(spinor<R> &s, R c) {
 #pragma unroll

@@ -218,11 +218,14 @@ __device__ __forceinline__ void block_allreduce3(double (&v)[3], double *red) {
 constexpr int EO_SREC = 9;   // float4 of a spinor record
 
 template <int FI, int DAG>
-__device__ __forceinline__ void hop_pair(const float4 *rec, int lo_slot, const float (&u)[18], float gy, Pair3 &up,
-                                         Pair3 &lo) {
+__device__ __forceinline__ void hop_pair(const float4 *rec, int lo_slot, const float (&u)[18], float gy,
+                                         Pair3<float> &up, Pair3<float> &lo) {
   float2 hr[3], hi[3];
 #pragma unroll
-  for (int k = 0; k < 3; k++) hop_project<FI, DAG>(rec[3 * k], rec[3 * k + lo_slot], gy, hr[k], hi[k]);
+  for (int k = 0; k < 3; k++) {
+    const float4 a = rec[3 * k], b = rec[3 * k + lo_slot];
+    hop_project<FI, DAG>(mk2(a.x, a.y), mk2(a.z, a.w), mk2(b.x, b.y), mk2(b.z, b.w), gy, hr[k], hi[k]);
+  }
   hop_link<FI, DAG>(hr, hi, u, gy, up, lo);
 }
 
@@ -237,9 +240,9 @@ __device__ __forceinline__ void eo_hop(const SapArgs &a, const EoRole &ro, int p
   const int l = y[0] * g.lstr[0] + y[1] * g.lstr[1] + y[2] * g.lstr[2] + y[3];
   const int ya = ro.role ? y[2] : y[0], yb = ro.role ? y[1] : y[3];
   const int chunk = p * g.nbl + blk, ochunk = (1 - p) * g.nbl + blk;
-  Pair3 up, lo;
-#pragma unroll
-  for (int k = 0; k < 3; k++) up.re[k] = up.im[k] = lo.re[k] = lo.im[k] = make_float2(0.0f, 0.0f);
+  Pair3<float> up, lo;
+  pair_zero(up);
+  pair_zero(lo);
   // a neighbour outside the block is one of the eight zero records at index
   // vbh8 (the one in the banks of the record it replaces), with any link: no
   // branches, so that the loads of a hop overlap the arithmetic of the one
@@ -333,9 +336,9 @@ __device__ __forceinline__ bool eo_cross(const SapArgs &a, const DDGeom &dg, con
   const int ya = ro.role ? x.y[2] : x.y[0], yb = ro.role ? x.y[1] : x.y[3];
   // global time coordinate: the time links at x0 = N0-1 carry the boundary sign
   const int x0 = (DD ? dg.x0off : 0) + x.n[0] * g.bs[0] + x.y[0], xlast = (DD ? dg.N0 : g.L[0]) - 1;
-  Pair3 up, lo;
-#pragma unroll
-  for (int k = 0; k < 3; k++) up.re[k] = up.im[k] = lo.re[k] = lo.im[k] = make_float2(0.0f, 0.0f);
+  Pair3<float> up, lo;
+  pair_zero(up);
+  pair_zero(lo);
   // chunk and site of the neighbour in the block across the face: block
   // coordinate n of nb, step bstr, in-block stride str
   auto across = [&](int n, int nb, int bstr, int bs, int str, int dir, int &c2, int &s2) {

@@ -360,8 +360,8 @@ def graphs_cached():
 
 
 def set_dw_staged(mode):
-    """FP64 operators: 1 SW matrices staged in shared memory (default), 0
-    read directly; returns the previous mode"""
+    """without effect since the FP64 operators have one form; returns the
+    previous mode"""
     return lib().b200_set_dw_staged(int(mode))
 
 
