@@ -32,28 +32,20 @@ __device__ __forceinline__ const double2 *lvec(const double2 *base, int nvec, si
   return base + ((size_t)r * nvec + j) * nv;
 }
 
-__global__ void __launch_bounds__(256) k_bmdot(const double2 *__restrict__ base, int nvec, size_t nv,
-                                               const int *__restrict__ act, int jq0, int k, int jy, int n,
-                                               double2 *part) {
-  __shared__ double2 red[8][BK];
-  const int r = act[blockIdx.y];
-  const double2 *y = lvec(base, nvec, nv, r, jy);
-  double ar[BK], ai[BK];
-#pragma unroll
-  for (int j = 0; j < BK; j++) ar[j] = ai[j] = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double2 yy = y[i];
-#pragma unroll
-    for (int j = 0; j < BK; j++)
-      if (j < k) {
-        const double2 q = lvec(base, nvec, nv, r, jq0 + j)[i];
-        ar[j] += q.x * yy.x + q.y * yy.y;
-        ai[j] += q.x * yy.y - q.y * yy.x;
-      }
-  }
+// Sums over the entries of a little vector in one launch: the block stores
+// its k partial sums and the block of the row that arrives last at the row's
+// counter adds all blocks' in the order of their indices, whichever block
+// that is, into out[0..k).  As a second kernel with one thread per sum this
+// addition was the largest item of the deflated solve on small lattices (19
+// us a sum, 30 % of the device time with 32 blocks and 20 modes).
+template <int KM>
+__device__ __forceinline__ void brow_sum(double (&ar)[KM], double (&ai)[KM], int k, double2 *part, unsigned *cnt,
+                                         double2 *out) {
+  __shared__ double2 red[8][KM];
+  __shared__ bool last;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 #pragma unroll
-  for (int j = 0; j < BK; j++)
+  for (int j = 0; j < KM; j++)
     if (j < k) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -63,40 +55,79 @@ __global__ void __launch_bounds__(256) k_bmdot(const double2 *__restrict__ base,
       if (lane == 0) red[wp][j] = make_double2(ar[j], ai[j]);
     }
   __syncthreads();
+  const bool alone = gridDim.x == 1;
   if ((int)threadIdx.x < k) {
     double re = 0.0, im = 0.0;
     for (int w = 0; w < 8; w++) {
       re += red[w][threadIdx.x].x;
       im += red[w][threadIdx.x].y;
     }
-    part[((size_t)blockIdx.y * BGRID + blockIdx.x) * BK + threadIdx.x] = make_double2(re, im);
+    (alone ? out : part + (size_t)blockIdx.x * BK)[threadIdx.x] = make_double2(re, im);
+    __threadfence();
+  }
+  if (alone) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(cnt, 1u) == gridDim.x - 1;
+    if (last) *cnt = 0u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int j = wp; j < k; j += 8) {
+    double re = 0.0, im = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) {
+      const double2 v = __ldcg(part + (size_t)b * BK + j);
+      re += v.x;
+      im += v.y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      re += __shfl_down_sync(0xffffffffu, re, o);
+      im += __shfl_down_sync(0xffffffffu, im, o);
+    }
+    if (lane == 0) out[j] = make_double2(re, im);
   }
 }
 
-// dots[r*64 + off + j] = sum over the CTAs of row y = slot (fixed order)
-__global__ void k_bmdot_fin(const double2 *__restrict__ part, int k, const int *__restrict__ act, double2 *dots,
-                            int off) {
-  const int y = blockIdx.x, r = act[y], j = threadIdx.x;
-  if (j >= k) return;
-  double re = 0.0, im = 0.0;
-  for (int b = 0; b < BGRID; b++) {
-    const double2 a = part[((size_t)y * BGRID + b) * BK + j];
-    re += a.x;
-    im += a.y;
+// dots[r*64 + off + j] = (vector jq0 + j, vector jy), j < k <= KM
+template <int KM>
+__global__ void __launch_bounds__(256) k_bmdot(const double2 *__restrict__ base, int nvec, size_t nv,
+                                               const int *__restrict__ act, int jq0, int k, int jy, int n,
+                                               double2 *part, unsigned *cnt, double2 *dots, int off) {
+  const int r = act[blockIdx.y];
+  const double2 *y = lvec(base, nvec, nv, r, jy);
+  double ar[KM], ai[KM];
+#pragma unroll
+  for (int j = 0; j < KM; j++) ar[j] = ai[j] = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double2 yy = y[i];
+#pragma unroll
+    for (int j = 0; j < KM; j++)
+      if (j < k) {
+        const double2 q = lvec(base, nvec, nv, r, jq0 + j)[i];
+        ar[j] += q.x * yy.x + q.y * yy.y;
+        ai[j] += q.x * yy.y - q.y * yy.x;
+      }
   }
-  dots[r * 64 + off + j] = make_double2(re, im);
+  brow_sum<KM>(ar, ai, k, part + (size_t)blockIdx.y * BGRID * BK, cnt + blockIdx.y, dots + r * 64 + off);
 }
 
-// q_k -= sum_j dots_j q_j ; p_k -= sum_j dots_j p_j
-__global__ void k_bgs_sub(double2 *base, int nvec, size_t nv, const int *__restrict__ act, int k,
-                          const double2 *__restrict__ dots, int jq0, int jp0, int n) {
+// q_k -= sum_j dots_j q_j ; p_k -= sum_j dots_j p_j ; with NORM |q_k|^2 into
+// dots[32]
+template <int NORM>
+__global__ void __launch_bounds__(256) k_bgs_sub(double2 *base, int nvec, size_t nv, const int *__restrict__ act,
+                                                 int k, double2 *dots, int jq0, int jp0, int n, double2 *part,
+                                                 unsigned *cnt) {
   __shared__ double2 c[BK];
   const int r = act[blockIdx.y];
   if ((int)threadIdx.x < k) c[threadIdx.x] = dots[r * 64 + threadIdx.x];
   __syncthreads();
   double2 *qk = (double2 *)lvec(base, nvec, nv, r, jq0 + k), *pk = (double2 *)lvec(base, nvec, nv, r, jp0 + k);
+  double ar[1] = {0.0}, ai[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double2 q = qk[i], p = pk[i];
+#pragma unroll 4
     for (int j = 0; j < k; j++) {
       const double2 a = lvec(base, nvec, nv, r, jq0 + j)[i], b = lvec(base, nvec, nv, r, jp0 + j)[i], z = c[j];
       q.x -= z.x * a.x - z.y * a.y; q.y -= z.x * a.y + z.y * a.x;
@@ -104,31 +135,46 @@ __global__ void k_bgs_sub(double2 *base, int nvec, size_t nv, const int *__restr
     }
     qk[i] = q;
     pk[i] = p;
+    ar[0] += q.x * q.x + q.y * q.y;
   }
+  if (NORM) brow_sum<1>(ar, ai, 1, part + (size_t)blockIdx.y * BGRID * BK, cnt + blockIdx.y, dots + r * 64 + 32);
 }
 
-// q, p /= |q| with |q|^2 = dots[off] (unchanged when zero)
-__global__ void k_bnorm(double2 *base, int nvec, size_t nv, const int *__restrict__ act,
-                        const double2 *__restrict__ dots, int off, int jq, int jp, int n) {
+// q, p /= |q| with |q|^2 = dots[32] (unchanged when zero), then (q, rv) into
+// dots[33]
+__global__ void __launch_bounds__(256) k_bnorm_dot(double2 *base, int nvec, size_t nv, const int *__restrict__ act,
+                                                   double2 *dots, int jq, int jp, int jr, int n, double2 *part,
+                                                   unsigned *cnt) {
   const int r = act[blockIdx.y];
-  const double s2 = dots[r * 64 + off].x;
-  if (!(s2 > 0.0)) return;
-  const double f = 1.0 / sqrt(s2);
+  const double s2 = dots[r * 64 + 32].x;
+  const bool ok = s2 > 0.0;
+  const double f = ok ? 1.0 / sqrt(s2) : 1.0;
   double2 *q = (double2 *)lvec(base, nvec, nv, r, jq), *p = (double2 *)lvec(base, nvec, nv, r, jp);
+  const double2 *rv = lvec(base, nvec, nv, r, jr);
+  double ar[1] = {0.0}, ai[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double2 a = q[i], b = p[i];
-    q[i] = make_double2(a.x * f, a.y * f);
-    p[i] = make_double2(b.x * f, b.y * f);
+    double2 a = q[i];
+    const double2 b = p[i], y = rv[i];
+    if (ok) {
+      a = make_double2(a.x * f, a.y * f);
+      q[i] = a;
+      p[i] = make_double2(b.x * f, b.y * f);
+    }
+    ar[0] += a.x * y.x + a.y * y.y;
+    ai[0] += a.x * y.y - a.y * y.x;
   }
+  brow_sum<1>(ar, ai, 1, part + (size_t)blockIdx.y * BGRID * BK, cnt + blockIdx.y, dots + r * 64 + 33);
 }
 
-// x += z p ; rv -= z q with z = dots[off]
-__global__ void k_bxr(double2 *base, int nvec, size_t nv, const int *__restrict__ act,
-                      const double2 *__restrict__ dots, int off, int jx, int jr, int jp, int jq, int n) {
+// x += z p ; rv -= z q with z = dots[33], then |rv|^2 into dots[34]
+__global__ void __launch_bounds__(256) k_bxr(double2 *base, int nvec, size_t nv, const int *__restrict__ act,
+                                             double2 *dots, int jx, int jr, int jp, int jq, int n, double2 *part,
+                                             unsigned *cnt) {
   const int r = act[blockIdx.y];
-  const double2 z = dots[r * 64 + off];
+  const double2 z = dots[r * 64 + 33];
   double2 *x = (double2 *)lvec(base, nvec, nv, r, jx), *rv = (double2 *)lvec(base, nvec, nv, r, jr);
   const double2 *p = lvec(base, nvec, nv, r, jp), *q = lvec(base, nvec, nv, r, jq);
+  double ar[1] = {0.0}, ai[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double2 pp = p[i], qq = q[i];
     double2 xx = x[i], rr = rv[i];
@@ -136,7 +182,9 @@ __global__ void k_bxr(double2 *base, int nvec, size_t nv, const int *__restrict_
     rr.x -= z.x * qq.x - z.y * qq.y; rr.y -= z.x * qq.y + z.y * qq.x;
     x[i] = xx;
     rv[i] = rr;
+    ar[0] += rr.x * rr.x + rr.y * rr.y;
   }
+  brow_sum<1>(ar, ai, 1, part + (size_t)blockIdx.y * BGRID * BK, cnt + blockIdx.y, dots + r * 64 + 34);
 }
 
 // dst = src (sgn = 0) or dst = src - dst (sgn = 1), first n entries
@@ -162,6 +210,7 @@ struct LtlBatch {
   int nvec = 0, nsys = 0;
   size_t nv = 0;
   double2 *part = nullptr, *dots = nullptr, *h_dots = nullptr;
+  unsigned *cnt = nullptr;   // blocks of each row's running sum that are done
   int *act = nullptr, *h_act = nullptr;
 };
 static LtlBatch g_lb;
@@ -173,6 +222,7 @@ static int ltl_batch_alloc(Ctx &c, int nr) {
   cudaFree(g_lb.base);
   cudaFree(g_lb.part);
   cudaFree(g_lb.dots);
+  cudaFree(g_lb.cnt);
   cudaFree(g_lb.act);
   if (g_lb.h_dots) cudaFreeHost(g_lb.h_dots);
   if (g_lb.h_act) cudaFreeHost(g_lb.h_act);
@@ -184,9 +234,11 @@ static int ltl_batch_alloc(Ctx &c, int nr) {
       cudaMalloc(&g_lb.part, (size_t)nr * BGRID * BK * sizeof(double2)) != cudaSuccess ||
       cudaMalloc(&g_lb.dots, (size_t)nr * 64 * sizeof(double2)) != cudaSuccess ||
       cudaMalloc(&g_lb.act, nr * sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&g_lb.cnt, nr * sizeof(unsigned)) != cudaSuccess ||
       cudaMallocHost(&g_lb.h_dots, (size_t)nr * 64 * sizeof(double2)) != cudaSuccess ||
       cudaMallocHost(&g_lb.h_act, nr * sizeof(int)) != cudaSuccess)
     return fail("out of device memory (batched little solver)");
+  cudaMemsetAsync(g_lb.cnt, 0, nr * sizeof(unsigned), c.stream);
   return 0;
 }
 
@@ -194,6 +246,7 @@ void ltl_batch_release() {
   cudaFree(g_lb.base);
   cudaFree(g_lb.part);
   cudaFree(g_lb.dots);
+  cudaFree(g_lb.cnt);
   cudaFree(g_lb.act);
   if (g_lb.h_dots) cudaFreeHost(g_lb.h_dots);
   if (g_lb.h_act) cudaFreeHost(g_lb.h_act);
@@ -226,15 +279,15 @@ int ltl_gcr_b(Ctx &c, double mu, int nr, const double2 *const *eta, double2 *con
     for (int r = 0; r < nr; r++) v[r] = B.base + ((size_t)r * nvec + j) * nv;
     return v;
   };
-  const unsigned gv = (unsigned)std::min<size_t>((nvh + 255) / 256, 148);
+  const unsigned gv = (unsigned)std::min<size_t>((nvh + 255) / 256, BGRID);
   std::vector<int> act;
   auto set_act = [&](const std::vector<int> &a) {
     for (size_t i = 0; i < a.size(); i++) B.h_act[i] = a[i];
     cudaMemcpyAsync(B.act, B.h_act, a.size() * sizeof(int), cudaMemcpyHostToDevice, st);
   };
   auto mdot = [&](int na, int jq0, int k, int jy, int off) {
-    k_bmdot<<<dim3(BGRID, na), 256, 0, st>>>(B.base, nvec, nv, B.act, jq0, k, jy, n, B.part);
-    k_bmdot_fin<<<na, 32, 0, st>>>(B.part, k, B.act, B.dots, off);
+    const auto f = k <= 1 ? k_bmdot<1> : k <= 4 ? k_bmdot<4> : k <= 8 ? k_bmdot<8> : k <= 16 ? k_bmdot<16> : k_bmdot<BK>;
+    f<<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, jq0, k, jy, n, B.part, B.cnt, B.dots, off);
   };
   auto read_dots = [&]() {
     cudaMemcpyAsync(B.h_dots, B.dots, (size_t)nr * 64 * sizeof(double2), cudaMemcpyDeviceToHost, st);
@@ -290,16 +343,16 @@ int ltl_gcr_b(Ctx &c, double mu, int nr, const double2 *const *eta, double2 *con
                                        Ya = pick(Y, act);
           dfl_Awhat_b(c, na, (const double2 *const *)Pk.data(), Qk.data(), Ya.data(), st);
         }
-        if (k > 0)
-          for (int pass = 0; pass < 2; pass++) {
-            mdot(na, JQ, k, JQ + k, 0);
-            k_bgs_sub<<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, k, B.dots, JQ, JP, n);
-          }
-        mdot(na, JQ + k, 1, JQ + k, 32);
-        k_bnorm<<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, B.dots, 32, JQ + k, JP + k, n);
-        mdot(na, JQ + k, 1, JR, 33);
-        k_bxr<<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, B.dots, 33, JX, JR, JP + k, JQ + k, n);
-        mdot(na, JR, 1, JR, 34);
+        if (k > 0) {
+          mdot(na, JQ, k, JQ + k, 0);
+          k_bgs_sub<0><<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, k, B.dots, JQ, JP, n, B.part, B.cnt);
+          mdot(na, JQ, k, JQ + k, 0);
+          k_bgs_sub<1><<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, k, B.dots, JQ, JP, n, B.part, B.cnt);
+        } else {
+          mdot(na, JQ, 1, JQ, 32);
+        }
+        k_bnorm_dot<<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, B.dots, JQ + k, JP + k, JR, n, B.part, B.cnt);
+        k_bxr<<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, B.dots, JX, JR, JP + k, JQ + k, n, B.part, B.cnt);
         return cudaGetLastError() == cudaSuccess ? 0 : fail("ltl_gcr: launch failed");
       });
       if (rc) return -1;
