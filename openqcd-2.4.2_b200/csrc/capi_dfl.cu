@@ -57,6 +57,7 @@ static int stage_bytes_ok(Ctx &c, size_t n) {
 
 // reference-layout FP32 field (host or device) -> device-layout field
 static int ref32_in(Ctx &c, const void *q, void *dev) {
+  if (ref_direct(c, q)) return spinor_from_ref(c, 32, q, dev, c.stream);
   size_t nb = spinor_bytes(c, 32);
   if (stage_bytes_ok(c, nb)) return -1;
   cudaMemcpyAsync(c.stage, q, nb, cudaMemcpyDefault, c.stream);
@@ -64,10 +65,14 @@ static int ref32_in(Ctx &c, const void *q, void *dev) {
 }
 
 static int ref32_out(Ctx &c, const void *dev, void *q) {
-  size_t nb = spinor_bytes(c, 32);
-  if (stage_bytes_ok(c, nb)) return -1;
-  if (spinor_to_ref(c, 32, dev, c.stage, c.stream)) return -1;
-  cudaMemcpyAsync(q, c.stage, nb, cudaMemcpyDefault, c.stream);
+  if (ref_direct(c, q)) {
+    if (spinor_to_ref(c, 32, dev, q, c.stream)) return -1;
+  } else {
+    size_t nb = spinor_bytes(c, 32);
+    if (stage_bytes_ok(c, nb)) return -1;
+    if (spinor_to_ref(c, 32, dev, c.stage, c.stream)) return -1;
+    cudaMemcpyAsync(q, c.stage, nb, cudaMemcpyDefault, c.stream);
+  }
   return cudaStreamSynchronize(c.stream) == cudaSuccess ? 0 : fail("CUDA error");
 }
 

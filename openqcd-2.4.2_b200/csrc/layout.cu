@@ -231,53 +231,84 @@ int geometry_init(Ctx &c, const int L[4], const int bs[4], const int *ipt) {
 }
 
 // ------------------------------------------------------------------ spinors
-template <typename R>
-__global__ void k_spinor_from_ref(Geom g, const int *__restrict__ d2q, const R *__restrict__ q, void *dev, int d0,
-                                  int nd) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nd) return;
-  const int d = d0 + i;
-  int chunk = d / g.vbh, s = d - chunk * g.vbh;
-  const R *src = q + (size_t)__ldg(d2q + d) * 24;
-  spinor<R> v;
+// A warp moves the records of 32 sites (24 reals each in the reference's
+// order) through shared memory, so that the array of structures is accessed
+// in whole records by neighbouring lanes and the planes by sites; a record
+// takes one 16-byte element more than it has, which keeps the site-wise
+// accesses free of bank conflicts.  With one site per lane on both sides the
+// records were read and written 16 bytes at a time at strides of 96 or 192
+// bytes (33 and 81 us for an FP32 field of 48x24^3, 64 MB each way).  The
+// restriction and prolongation of four such fields with 28 modes, conversions
+// included: 1618 -> 1175 us, with the copy of device-resident arrays to the
+// staging buffer left out as well (ref_direct).
+template <typename R> struct RefRec;
+template <> struct RefRec<float> {
+  using E = float4;
+  static constexpr int N = 6;    // elements of a record
+};
+template <> struct RefRec<double> {
+  using E = double2;
+  static constexpr int N = 12;
+};
+constexpr int REF_T = 128;
+// site i of the launch (i < n): its record iq in the reference's array and its
+// place d on the device; lanes beyond n take part in the copies of their warp
+template <typename R, bool IN>
+__device__ __forceinline__ void ref_records(const Geom &g, int i, int n, int iq, int d, R *q, void *dev) {
+  using E = typename RefRec<R>::E;
+  constexpr int N = RefRec<R>::N;
+  __shared__ E sm[REF_T / 32][32 * (N + 1)];
+  E *t = sm[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31, nw = min(32, n - (i - lane));   // sites of this warp
+  const int chunk = d / g.vbh, s = d - chunk * g.vbh;
+  E *p = (E *)dev + (size_t)chunk * N * g.vbh + s, *rec = reinterpret_cast<E *>(q);
+  if (!IN && i < n)
 #pragma unroll
-  for (int k = 0; k < 12; k++) v.c[k / 3].c[k % 3] = mk<R>(src[2 * k], src[2 * k + 1]);
-  Store<R>::store_spinor(dev, chunk, s, g.vbh, v);
+    for (int k = 0; k < N; k++) t[lane * (N + 1) + k] = p[(size_t)k * g.vbh];
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const int f = k * 32 + lane, site = f / N, e = f - site * N;
+    const size_t o = (size_t)__shfl_sync(0xffffffffu, iq, site) * N + e;
+    if (site < nw) {
+      if (IN) t[site * (N + 1) + e] = __ldg(rec + o);
+      else rec[o] = t[site * (N + 1) + e];
+    }
+  }
+  __syncwarp();
+  if (IN && i < n)
+#pragma unroll
+    for (int k = 0; k < N; k++) p[(size_t)k * g.vbh] = t[lane * (N + 1) + k];
 }
 
 template <typename R>
-__global__ void k_spinor_to_ref(Geom g, const int *__restrict__ d2q, const void *dev, R *q, int d0, int nd) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nd) return;
-  const int d = d0 + i;
-  int chunk = d / g.vbh, s = d - chunk * g.vbh;
-  R *dst = q + (size_t)__ldg(d2q + d) * 24;
-  spinor<R> v = Store<R>::load_spinor_rw(dev, chunk, s, g.vbh);
-#pragma unroll
-  for (int k = 0; k < 12; k++) { dst[2 * k] = v.c[k / 3].c[k % 3].re; dst[2 * k + 1] = v.c[k / 3].c[k % 3].im; }
+__global__ void __launch_bounds__(REF_T) k_spinor_from_ref(Geom g, const int *__restrict__ d2q, const R *q, void *dev,
+                                                           int d0, int nd) {
+  const int i = blockIdx.x * REF_T + threadIdx.x, d = d0 + min(i, nd - 1);
+  ref_records<R, true>(g, i, nd, __ldg(d2q + d), d, const_cast<R *>(q), dev);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(REF_T) k_spinor_to_ref(Geom g, const int *__restrict__ d2q, const void *dev, R *q,
+                                                         int d0, int nd) {
+  const int i = blockIdx.x * REF_T + threadIdx.x, d = d0 + min(i, nd - 1);
+  ref_records<R, false>(g, i, nd, __ldg(d2q + d), d, q, const_cast<void *>(dev));
 }
 
 // the sites of a piece, both parity halves in one launch: thread i takes
-// storage index q0[0] + i or q0[1] + (i - n0), reads it (contiguous) and
-// stores it at its device site
+// storage index q0[0] + i or q0[1] + (i - n0), and stores it at its device
+// site
 template <typename R>
-__global__ void k_spinor_from_ref_piece(Geom g, const int *__restrict__ q2d, const R *__restrict__ q, void *dev,
-                                        int qa, int na, int qb, int nb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= na + nb) return;
-  const int iq = i < na ? qa + i : qb + (i - na);
-  const int d = __ldg(q2d + iq);
-  const int chunk = d / g.vbh, s = d - chunk * g.vbh;
-  const R *src = q + (size_t)iq * 24;
-  spinor<R> v;
-#pragma unroll
-  for (int k = 0; k < 12; k++) v.c[k / 3].c[k % 3] = mk<R>(src[2 * k], src[2 * k + 1]);
-  Store<R>::store_spinor(dev, chunk, s, g.vbh, v);
+__global__ void __launch_bounds__(REF_T) k_spinor_from_ref_piece(Geom g, const int *__restrict__ q2d, const R *q,
+                                                                 void *dev, int qa, int na, int qb, int nb) {
+  const int i = blockIdx.x * REF_T + threadIdx.x, j = min(i, na + nb - 1);
+  const int iq = j < na ? qa + j : qb + (j - na);
+  ref_records<R, true>(g, i, na + nb, iq, __ldg(q2d + iq), const_cast<R *>(q), dev);
 }
 
 int spinor_from_ref_piece(const Ctx &c, int prec, const void *q, void *dev, const Piece &pc, cudaStream_t st) {
   if (!c.d_q2dev) return fail("no reference site order: pass ipt[] to the geometry call");
-  const int t = 128, na = pc.q1[0] - pc.q0[0], nb = pc.q1[1] - pc.q0[1];
+  const int t = REF_T, na = pc.q1[0] - pc.q0[0], nb = pc.q1[1] - pc.q0[1];
   const unsigned grid = (unsigned)((na + nb + t - 1) / t);
   if (prec == 64)
     k_spinor_from_ref_piece<double><<<grid, t, 0, st>>>(c.g, c.d_q2dev, (const double *)q, dev, pc.q0[0], na,
@@ -290,7 +321,7 @@ int spinor_from_ref_piece(const Ctx &c, int prec, const void *q, void *dev, cons
 
 int spinor_from_ref_range(const Ctx &c, int prec, const void *q, void *dev, int d0, int n, cudaStream_t st) {
   if (!c.have_ipt) return fail("no reference site order: pass ipt[] to the geometry call");
-  const int t = 128;
+  const int t = REF_T;
   if (n <= 0) return 0;
   if (prec == 64)
     k_spinor_from_ref<double><<<(n + t - 1) / t, t, 0, st>>>(c.g, c.d_dev2q, (const double *)q, dev, d0, n);
@@ -301,11 +332,22 @@ int spinor_from_ref_range(const Ctx &c, int prec, const void *q, void *dev, int 
 
 int spinor_to_ref_range(const Ctx &c, int prec, const void *dev, void *q, int d0, int n, cudaStream_t st) {
   if (!c.have_ipt) return fail("no reference site order: pass ipt[] to the geometry call");
-  const int t = 128;
+  const int t = REF_T;
   if (n <= 0) return 0;
   if (prec == 64) k_spinor_to_ref<double><<<(n + t - 1) / t, t, 0, st>>>(c.g, c.d_dev2q, dev, (double *)q, d0, n);
   else k_spinor_to_ref<float><<<(n + t - 1) / t, t, 0, st>>>(c.g, c.d_dev2q, dev, (float *)q, d0, n);
   return cudaGetLastError() == cudaSuccess ? 0 : fail("spinor_to_ref: launch failed");
+}
+
+// whether the conversions can work on the caller's array itself: memory of
+// the library's device, aligned for 16-byte accesses
+bool ref_direct(const Ctx &c, const void *q) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == c.dev && (uintptr_t)q % 16 == 0;
 }
 
 int spinor_from_ref(const Ctx &c, int prec, const void *q, void *dev, cudaStream_t st) {
