@@ -731,6 +731,17 @@ static int pick_threads(int vbh, int &ns) {
 // launch bound and the register budget it implies.  The autotuner below
 // times every variant that fits the block on the resident fields and keeps
 // the fastest per block size and storage mode.
+// Which one wins, in us per cycle of four MR steps:
+//   ns maxt (registers)   8^4, 4^4 blocks  32^4, 4^4  4x4x6x4   48x24^3, 6^4  8x4x6x8
+//   1   512 (128)               72            769        -              -             -
+//   1   256 (255)               66            958        -              -             -
+//   3   512 (128)              130            987        -             666           364
+//   1   768 (80)                80            797       132            -             -
+//   2   320 (96, two CTAs/SM)  111            941       379            -             -
+// Few blocks leave one CTA to an SM: what counts is a lane's chain, and
+// registers shorten it; many blocks want warps.  A block shared by a cluster
+// of 2, 4 or 8 CTAs, each writing its sites into the others' shared memory,
+// took 86 to 95 us where one CTA takes 66.
 struct EoVariant {
   int ns, maxt;
   void (*k[3])(SapArgs);   // per storage mode
@@ -739,8 +750,8 @@ struct EoVariant {
   {k_sap_blocks_eo<NS, EoFull, SapF32, MAXT, MINB>, k_sap_blocks_eo<NS, EoHalf, SapF16, MAXT, MINB>,     \
    k_sap_blocks_eo<NS, EoTwoRow, SapF32, MAXT, MINB>}
 static const EoVariant kEo[] = {
-    {1, 256, EO_KERNELS(1, 256, 2)}, {1, 512, EO_KERNELS(1, 512, 1)}, {2, 672, EO_KERNELS(2, 672, 1)},
-    {3, 448, EO_KERNELS(3, 448, 1)}, {3, 512, EO_KERNELS(3, 512, 1)},
+    {1, 512, EO_KERNELS(1, 512, 1)}, {1, 256, EO_KERNELS(1, 256, 1)}, {3, 512, EO_KERNELS(3, 512, 1)},
+    {1, 768, EO_KERNELS(1, 768, 1)}, {2, 320, EO_KERNELS(2, 320, 2)},
 };
 static const int kNEo = sizeof(kEo) / sizeof(kEo[0]);
 
