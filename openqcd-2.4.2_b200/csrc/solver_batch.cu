@@ -334,7 +334,8 @@ int ltl_gcr_b(Ctx &c, double mu, int nr, const double2 *const *eta, double2 *con
       std::vector<uint64_t> key = {0x17a9ull, (uint64_t)na, (uint64_t)k, (uint64_t)(uintptr_t)B.base, nv,
                                    (uint64_t)nvec, (uint64_t)(uintptr_t)d.Mhop, (uint64_t)(uintptr_t)d.Mhop32,
                                    (uint64_t)(uintptr_t)B.act, (uint64_t)(uintptr_t)B.dots,
-                                   (uint64_t)(uintptr_t)B.part, (uint64_t)(uintptr_t)d.nbr, (uint64_t)d.Ns};
+                                   (uint64_t)(uintptr_t)B.part, (uint64_t)(uintptr_t)B.cnt, (uint64_t)(uintptr_t)d.nbr,
+                                   (uint64_t)d.Ns};
       for (int r : act) key.push_back((uint64_t)r);
       const int rc = graph_run(c, key.data(), key.size() * sizeof(uint64_t), st, [&]() {
         k_bcopy<<<dim3(gv, na), 256, 0, st>>>(B.base, nvec, nv, B.act, JR, JP + k, n, 0);
@@ -945,7 +946,8 @@ int gcr_batch(Ctx &c, int nr, int dfl, int nkv, int nmx, int istop, double res, 
     if (fused) {
       // captured as one CUDA graph per step shape (the systems' k and
       // fields), replayed by later steps and solves of the same shape
-      std::vector<uint64_t> key = {0x0e7a0ull, (uint64_t)na, (uint64_t)(size_t)c.g.vol};
+      std::vector<uint64_t> key = {0x0e7a0ull, (uint64_t)na, (uint64_t)(size_t)c.g.vol,
+                                   (uint64_t)(uintptr_t)g_ob.dsum, (uint64_t)(uintptr_t)g_ob.part};
       for (int i = 0; i < na; i++) {
         const SysState &y = S[A[i]];
         key.push_back((uint64_t)y.k);
