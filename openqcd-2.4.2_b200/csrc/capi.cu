@@ -333,6 +333,7 @@ int b200_geometry(const int L[4], const int bs[4], const int *ipt) {
   qcd::dfl_release(c);
   qcd::net_fields_release(c);
   qcd::graphs_release();
+  qcd::gcr_batch_release();   // its fields have the old lattice's size
   c.ready = false;
   if (geometry_init(c, L, bs, ipt) || qcd::dd_buffers(c)) return -1;
   c.ready = true;
