@@ -130,7 +130,7 @@ int export_cnfg(Ctx &c, const char *out) {
   const int *L = c.g.L;
   const size_t nd = (size_t)c.g.vol * 36;
   std::vector<double2> hu(nd);
-  if (cudaMemcpy(hu.data(), c.ud, nd * sizeof(double2), cudaMemcpyDeviceToHost) != cudaSuccess)
+  if (copy_now(c, hu.data(), c.ud, nd * sizeof(double2)))
     return fail("export_cnfg: CUDA error");
   double ps = 0.0;
   if (plaq_sum(c, &ps)) return -1;
@@ -227,7 +227,7 @@ int import_cnfg(Ctx &c, const char *in, int mask) {
   fclose(f);
   if (!ok) return fail("import_cnfg: incorrect read count");
   if (!c.ud && cudaMalloc(&c.ud, nd * sizeof(double2)) != cudaSuccess) return fail("out of device memory (links)");
-  if (cudaMemcpy(c.ud, hu.data(), nd * sizeof(double2), cudaMemcpyHostToDevice) != cudaSuccess)
+  if (copy_now(c, c.ud, hu.data(), nd * sizeof(double2)))
     return fail("import_cnfg: CUDA error");
   c.have_ud = true;
   c.have_sw = false;   // the SW term belongs to the old field: recompute it
@@ -271,7 +271,7 @@ int export_sfld(Ctx &c, const char *out, int eo, const void *sd) {
   const int *L = c.g.L;
   const size_t V = (size_t)c.g.vol;
   std::vector<double> h(V * 24);
-  if (cudaMemcpy(h.data(), sd, V * 24 * sizeof(double), cudaMemcpyDefault) != cudaSuccess)
+  if (copy_now(c, h.data(), sd, V * 24 * sizeof(double)))
     return fail("export_sfld: cannot read the field");
   double norm = norm_sq(h.data(), eo ? V / 2 : V);
   FILE *f = fopen(out, "wb");
@@ -315,7 +315,7 @@ int import_sfld(Ctx &c, const char *in, int eo, void *sd) {
     return fail("import_sfld: lattice sizes or eo flag do not match");
   }
   std::vector<double> h(V * 24);
-  if (cudaMemcpy(h.data(), sd, V * 24 * sizeof(double), cudaMemcpyDefault) != cudaSuccess) {
+  if (copy_now(c, h.data(), sd, V * 24 * sizeof(double))) {
     fclose(f);
     return fail("import_sfld: cannot read the field");
   }
@@ -339,7 +339,7 @@ int import_sfld(Ctx &c, const char *in, int eo, void *sd) {
   const double norm1 = norm_sq(h.data(), eo ? V / 2 : V);
   // the check of sarchive.c:612-615
   if (std::fabs(norm1 - norm0) > 64.0 * (norm0 + norm1) * DBL_EPSILON) return fail("import_sfld: incorrect square norm");
-  if (cudaMemcpy(sd, h.data(), V * 24 * sizeof(double), cudaMemcpyDefault) != cudaSuccess)
+  if (copy_now(c, sd, h.data(), V * 24 * sizeof(double)))
     return fail("import_sfld: cannot write the field");
   return 0;
 }

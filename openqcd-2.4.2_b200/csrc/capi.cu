@@ -51,6 +51,14 @@ static int ensure_tmp(Ctx &c) {
   return 0;
 }
 
+// a field of zeros, ready for what follows on the library's stream
+static void *alloc_spinor(Ctx &c, int prec) {
+  void *p = nullptr;
+  if (cudaMalloc(&p, spinor_bytes(c, prec)) != cudaSuccess) { fail("out of device memory"); return nullptr; }
+  cudaMemsetAsync(p, 0, spinor_bytes(c, prec), c.stream);
+  return p;
+}
+
 static int check_ready(const Ctx &c) { return need(c.ready, "geometry not set (call b200_geometry first)"); }
 static int check_fields(const Ctx &c) {
   if (check_ready(c)) return -1;
@@ -732,7 +740,7 @@ void sap(float mu, int isolv, int nmr, spinor *psi, spinor *rho) {
   if (sap_prepare(c, c.stream)) return;
   size_t nb = spinor_bytes(c, 32);
   if (ensure_stage(c, 2 * nb)) return;
-  void *fp = b200_dev_alloc_spinor(32), *fr = b200_dev_alloc_spinor(32), *fb = b200_dev_alloc_spinor(32);
+  void *fp = alloc_spinor(c, 32), *fr = alloc_spinor(c, 32), *fb = alloc_spinor(c, 32);
   if (!fp || !fr || !fb) return;
   char *s0 = (char *)c.stage, *s1 = s0 + nb;
   cudaStream_t st = c.stream;
@@ -755,7 +763,7 @@ double sap_gcr(int nkv, int nmx, int istop, double res, double mu, spinor_dble *
   if (check_fields(c)) return -1.0;
   size_t nb = spinor_bytes(c, 64);
   if (ensure_stage(c, nb)) return -1.0;
-  void *fe = b200_dev_alloc_spinor(64), *fp = b200_dev_alloc_spinor(64);
+  void *fe = alloc_spinor(c, 64), *fp = alloc_spinor(c, 64);
   if (!fe || !fp) return -1.0;
   cudaStream_t st = c.stream;
   cudaMemcpyAsync(c.stage, eta, nb, cudaMemcpyDefault, st);
@@ -772,9 +780,8 @@ double sap_gcr(int nkv, int nmx, int istop, double res, double mu, spinor_dble *
 void *b200_dev_alloc_spinor(int prec) {
   Ctx &c = ctx();
   if (check_ready(c)) return nullptr;
-  void *p = nullptr;
-  if (cudaMalloc(&p, spinor_bytes(c, prec)) != cudaSuccess) { fail("out of device memory"); return nullptr; }
-  cudaMemset(p, 0, spinor_bytes(c, prec));
+  void *p = alloc_spinor(c, prec);
+  if (p) cudaStreamSynchronize(c.stream);   // the caller may go on with it on a stream of its own
   return p;
 }
 void b200_dev_free(void *p) { cudaFree(p); }

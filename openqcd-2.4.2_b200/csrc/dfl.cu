@@ -55,7 +55,7 @@ static int dfl_alloc(Ctx &c) {
   d.nv = Ns * nb;
   // block tables
   std::vector<int> bco(nb), v2l(nb), l2v(nb), nbr(8 * nb);
-  cudaMemcpy(bco.data(), c.d_bcoord, nb * sizeof(int), cudaMemcpyDeviceToHost);
+  copy_now(c, bco.data(), c.d_bcoord, nb * sizeof(int));
   for (int n = 0; n < nb; n++) {
     v2l[n] = lex_of_vd(c.g, bco, n);
     l2v[v2l[n]] = n;
@@ -71,10 +71,10 @@ static int dfl_alloc(Ctx &c) {
       nbr[8 * n + ifc] = l2v[lb];
     }
   }
-  auto up = [](int *&p, const std::vector<int> &v) {
+  auto up = [&c](int *&p, const std::vector<int> &v) {
     cudaFree(p);
     cudaMalloc(&p, v.size() * sizeof(int));
-    cudaMemcpy(p, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice);
+    copy_now(c, p, v.data(), v.size() * sizeof(int));
   };
   up(d.vd2lex, v2l);
   up(d.nbr, nbr);
@@ -104,12 +104,12 @@ static int dfl_alloc(Ctx &c) {
   while ((int)d.basis.size() < Ns) {
     void *p = nullptr;
     if (cudaMalloc(&p, spinor_bytes(c, 32)) != cudaSuccess) return fail("out of device memory (deflation basis)");
-    cudaMemset(p, 0, spinor_bytes(c, 32));
+    cudaMemsetAsync(p, 0, spinor_bytes(c, 32), c.stream);
     d.basis.push_back(p);
   }
   cudaFree(d.d_basis);
   cudaMalloc(&d.d_basis, Ns * sizeof(void *));
-  cudaMemcpy(d.d_basis, d.basis.data(), Ns * sizeof(void *), cudaMemcpyHostToDevice);
+  copy_now(c, d.d_basis, d.basis.data(), Ns * sizeof(void *));
   cudaFree(d.rpart);
   if (cudaMalloc(&d.rpart, (size_t)nb * 2 * Ns * sizeof(double2)) != cudaSuccess)
     return fail("out of device memory (deflation)");
@@ -888,7 +888,7 @@ int dfl_subspace_dev(Ctx &c, const std::vector<void *> &modes, cudaStream_t st, 
     // dfl_subspace.c:171-240, to rounding): modes -> basis
     float4 **dm = nullptr;
     if (cudaMalloc(&dm, d.Ns * sizeof(void *)) != cudaSuccess) return fail("out of device memory");
-    cudaMemcpy(dm, modes.data(), d.Ns * sizeof(void *), cudaMemcpyHostToDevice);
+    copy_now(c, dm, modes.data(), d.Ns * sizeof(void *));
     const int rc = dfl_cholqr(c, (const float4 *const *)dm, (float4 *const *)d.d_basis, false, st);
     cudaFree(dm);
     if (rc < 0) return -1;
@@ -1046,7 +1046,7 @@ static int ltl_ensure(Ctx &c) {
       tab[nkv + k] = d.lv[6 + nkv + k];
     }
     tab[2 * nkv] = d.lv[1];
-    cudaMemcpy(d.lvtab, tab.data(), tab.size() * sizeof(double2 *), cudaMemcpyHostToDevice);
+    copy_now(c, d.lvtab, tab.data(), tab.size() * sizeof(double2 *));
     d.lvtab_nkv = nkv;
   }
   return 0;
@@ -1286,7 +1286,7 @@ int dfl_modes_dev(Ctx &c, uint64_t seed, int *ifail, int *status) {
   // device table of the mode fields (for the Cholesky QR kernels)
   float4 **dmodes = nullptr;
   if (cudaMalloc(&dmodes, d.Ns * sizeof(void *)) != cudaSuccess) return fail("out of device memory");
-  cudaMemcpy(dmodes, d.modes.data(), d.Ns * sizeof(void *), cudaMemcpyHostToDevice);
+  copy_now(c, dmodes, d.modes.data(), d.Ns * sizeof(void *));
   struct FreeTab {
     float4 **p;
     ~FreeTab() { cudaFree(p); }

@@ -571,7 +571,7 @@ int dfl_batch_alloc(Ctx &c) {
   if (cudaMalloc(&d.bpart, (size_t)d.nb * 2 * ns * BT * d.Ns * sizeof(double2)) != cudaSuccess ||
       cudaMalloc(&d.kerr, sizeof(int)) != cudaSuccess)
     return fail("out of device memory (batched deflation)");
-  cudaMemset(d.kerr, 0, sizeof(int));
+  cudaMemsetAsync(d.kerr, 0, sizeof(int), c.stream);
   return 0;
 }
 
@@ -580,9 +580,9 @@ int dfl_batch_check(Ctx &c) {
   DflState &d = c.dfl;
   if (!d.kerr) return 0;
   int h = 0;
-  cudaMemcpy(&h, d.kerr, sizeof(int), cudaMemcpyDeviceToHost);
+  copy_now(c, &h, d.kerr, sizeof(int));
   if (h) {
-    cudaMemset(d.kerr, 0, sizeof(int));
+    cudaMemsetAsync(d.kerr, 0, sizeof(int), c.stream);
     return fail("deflation: a bulk copy did not complete in time");
   }
   return 0;

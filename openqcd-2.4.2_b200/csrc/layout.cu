@@ -69,7 +69,7 @@ int set_block_order(Ctx &c, int kind) {
   for (int b = 0; b < g.nbl; b++) sch[b] = key[b].second;
   if (!c.sched && cudaMalloc(&c.sched, g.nbl * sizeof(int)) != cudaSuccess)
     return fail("block order: device allocation failed");
-  cudaMemcpy(c.sched, sch.data(), g.nbl * sizeof(int), cudaMemcpyHostToDevice);
+  copy_now(c, c.sched, sch.data(), g.nbl * sizeof(int));
   c.block_order = kind;
   return 0;
 }
@@ -165,8 +165,8 @@ int geometry_init(Ctx &c, const int L[4], const int bs[4], const int *ipt) {
   if (cudaMalloc(&c.d_bcoord, g.nbl * sizeof(int)) != cudaSuccess ||
       cudaMalloc(&c.d_lcoord, g.vb * sizeof(int)) != cudaSuccess)
     return fail("geometry: device allocation failed");
-  cudaMemcpy(c.d_bcoord, bco.data(), g.nbl * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(c.d_lcoord, lco.data(), g.vb * sizeof(int), cudaMemcpyHostToDevice);
+  copy_now(c, c.d_bcoord, bco.data(), g.nbl * sizeof(int));
+  copy_now(c, c.d_lcoord, lco.data(), g.vb * sizeof(int));
   if (set_block_order(c, c.block_order)) return -1;
   g.bcoord = c.d_bcoord;
   g.lcoord = c.d_lcoord;
@@ -206,14 +206,14 @@ int geometry_init(Ctx &c, const int L[4], const int bs[4], const int *ipt) {
     if (cudaMalloc(&c.d_dev2q, g.vol * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&c.d_link2q, 4 * (size_t)g.vol * sizeof(int)) != cudaSuccess)
       return fail("geometry: device allocation failed");
-    cudaMemcpy(c.d_dev2q, d2q.data(), g.vol * sizeof(int), cudaMemcpyHostToDevice);
+    copy_now(c, c.d_dev2q, d2q.data(), g.vol * sizeof(int));
     {
       std::vector<int> q2d(g.vol);
       for (int d = 0; d < g.vol; d++) q2d[d2q[d]] = d;
       if (cudaMalloc(&c.d_q2dev, g.vol * sizeof(int)) != cudaSuccess) return fail("geometry: device allocation failed");
-      cudaMemcpy(c.d_q2dev, q2d.data(), g.vol * sizeof(int), cudaMemcpyHostToDevice);
+      copy_now(c, c.d_q2dev, q2d.data(), g.vol * sizeof(int));
     }
-    cudaMemcpy(c.d_link2q, l2q.data(), 4 * (size_t)g.vol * sizeof(int), cudaMemcpyHostToDevice);
+    copy_now(c, c.d_link2q, l2q.data(), 4 * (size_t)g.vol * sizeof(int));
     c.h_dev2q = d2q;
     c.h_ipt.assign(ipt, ipt + g.vol);
     c.have_ipt = true;
@@ -225,7 +225,7 @@ int geometry_init(Ctx &c, const int L[4], const int bs[4], const int *ipt) {
     std::vector<int> id(g.nbl);
     for (int b = 0; b < g.nbl; b++) id[b] = b;
     if (cudaMalloc(&c.d_ident, g.nbl * sizeof(int)) != cudaSuccess) return fail("geometry: device allocation failed");
-    cudaMemcpy(c.d_ident, id.data(), g.nbl * sizeof(int), cudaMemcpyHostToDevice);
+    copy_now(c, c.d_ident, id.data(), g.nbl * sizeof(int));
   }
   return cudaGetLastError() == cudaSuccess ? 0 : fail("geometry: CUDA error");
 }

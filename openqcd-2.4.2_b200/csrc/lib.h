@@ -219,6 +219,18 @@ int fail(const std::string &msg);   // records msg, returns -1 (or aborts in fat
 
 size_t spinor_bytes(const Ctx &c, int prec);   // prec 64 or 32
 
+// A copy on the library's stream, complete on return: 0, or -1 if it failed.
+// The stream is a non-blocking one, which does not wait for the legacy default
+// stream where cudaMemcpy and cudaMemset work: a fill there may still run
+// after the kernels that follow it here, and a copy from pageable memory may
+// return before the device has the data.
+inline int copy_now(const Ctx &c, void *dst, const void *src, size_t bytes) {
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, c.stream) == cudaSuccess &&
+                 cudaStreamSynchronize(c.stream) == cudaSuccess
+             ? 0
+             : -1;
+}
+
 // dd.cu: domain decomposition along x0
 int dd_buffers(Ctx &c);
 int dd_exchange(Ctx &c, size_t bytes, cudaStream_t st);

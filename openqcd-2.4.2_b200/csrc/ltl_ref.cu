@@ -286,11 +286,11 @@ static int ensure_base(Ctx &c) {
 }
 
 template <typename T>
-static int grow(std::vector<T *> &v, size_t n, size_t len) {
+static int grow(const Ctx &c, std::vector<T *> &v, size_t n, size_t len) {
   while (v.size() < n) {
     T *p = nullptr;
     if (cudaMalloc(&p, len * sizeof(T)) != cudaSuccess) return fail("out of device memory (little vectors)");
-    cudaMemset(p, 0, len * sizeof(T));
+    cudaMemsetAsync(p, 0, len * sizeof(T), c.stream);
     v.push_back(p);
   }
   return 0;
@@ -393,7 +393,7 @@ int ltl_lmodes_from_fields(Ctx &c, const std::vector<void *> &modes, cudaStream_
   DflState &d = c.dfl;
   if (ensure_base(c)) return -1;
   LtlRef &r = *lr(c);
-  if (grow(r.lmode, d.Ns, d.nv) || dfl_batch_alloc(c)) return -1;
+  if (grow(c, r.lmode, d.Ns, d.nv) || dfl_batch_alloc(c)) return -1;
   for (int l0 = 0; l0 < d.Ns; l0 += 4) {
     const int na = std::min(4, d.Ns - l0);
     const void *f[4];
@@ -416,7 +416,7 @@ int ltl_lmode_set(Ctx &c, int l, const void *v32) {
   if (ensure_base(c)) return -1;
   LtlRef &r = *lr(c);
   if (l < 0 || l >= d.Ns) return fail("little mode index out of range");
-  if (grow(r.lmode, d.Ns, d.nv) || grow(r.wvs, 1, d.nv)) return -1;
+  if (grow(c, r.lmode, d.Ns, d.nv) || grow(c, r.wvs, 1, d.nv)) return -1;
   cudaMemcpyAsync(r.wvs[0], v32, (size_t)d.nv * sizeof(float2), cudaMemcpyDefault, c.stream);
   k_v32to64<<<vgrid(d.nv), 256, 0, c.stream>>>(r.wvs[0], r.lmode[l], d.nv);
   if (cudaStreamSynchronize(c.stream) != cudaSuccess) return fail("CUDA error");
@@ -502,7 +502,7 @@ int ltl_set_modes(Ctx &c) {
   LtlRef &r = *lr(c);
   if (!r.lmode_valid) return fail("ltl_gcr: no little modes (the subspace was not built from modes)");
   const int Ns = d.Ns, nvh = r.nvh;
-  if (grow(r.vds, Ns, d.nv) || grow(r.vs, Ns, d.nv)) return -1;
+  if (grow(c, r.vds, Ns, d.nv) || grow(c, r.vs, Ns, d.nv)) return -1;
   // vs2vds: the even halves, orthonormalised in the reference's order
   for (int l = 0; l < Ns; l++) vcopy64(c, r.vds[l], r.lmode[l], nvh);
   double rr = vnorm2<double2>(c, r.vds[0], nvh);
@@ -837,7 +837,7 @@ double ltl_gcr_ref(Ctx &c, double mu, const double2 *eta, double2 *psi, int *ifa
     }
   }
   if (mhop32(c)) return -1.0;
-  if (grow(r.wvd, 2 * d.nkv + 3, nv) || grow(r.wvs, 2 * d.nmx_gcr + 3, nv)) return -1.0;
+  if (grow(c, r.wvd, 2 * d.nkv + 3, nv) || grow(c, r.wvs, 2 * d.nmx_gcr + 3, nv)) return -1.0;
   double2 *w0 = r.wvd[0], *w1 = r.wvd[1];
   // wvd1 = eta; odd: Aoo^-1 eta_o; even: eta_e - Aeo (.); w0_e = Aee^-1 (.)
   vcopy64(c, w1, eta, nv);

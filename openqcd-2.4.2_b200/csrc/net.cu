@@ -244,9 +244,9 @@ static int net_upload(Ctx &c) {
           wa[(db * ci + i) * co + o] = make_float2(re, -im);
         }
     }
-    cudaMemcpy(n.dev_w[l], w.data(), w.size() * sizeof(float2), cudaMemcpyHostToDevice);
-    cudaMemcpy(n.dev_wadj[l], wa.data(), wa.size() * sizeof(float2), cudaMemcpyHostToDevice);
-    cudaMemcpy(n.dev_w16[l], w16.data(), w16.size() * sizeof(float2), cudaMemcpyHostToDevice);
+    copy_now(c, n.dev_w[l], w.data(), w.size() * sizeof(float2));
+    copy_now(c, n.dev_wadj[l], wa.data(), wa.size() * sizeof(float2));
+    copy_now(c, n.dev_w16[l], w16.data(), w16.size() * sizeof(float2));
   }
   n.ready = true;
   return cudaGetLastError() == cudaSuccess ? 0 : fail("network: upload failed");
@@ -379,7 +379,7 @@ static void grad_zero(Ctx &c, cudaStream_t st) {
 static void grad_read(Ctx &c, std::vector<double> *g) {
   for (int l = 0; l < NLAY; l++) {
     g[l].resize(2 * wsize(l));
-    cudaMemcpy(g[l].data(), c.net.dev_grad[l], wsize(l) * sizeof(double2), cudaMemcpyDeviceToHost);
+    copy_now(c, g[l].data(), c.net.dev_grad[l], wsize(l) * sizeof(double2));
   }
 }
 
