@@ -166,7 +166,7 @@ def test_dirac_multi(setup, n):
         assert site_rel_err(Q[i].to_ref(setup.vol), diff, setup.vol) <= 2e-6
 
 
-def test_rhs_tile_autotuner(setup):
+def test_rhs_tile_autotuner(dfl):
     """After a deflated batched solve the RHS-tile autotuner has timed the
     restriction and prolongation with 1, 2 and 4 fields per pass on the CUDA
     cores and 4 on the tensor cores, and kept the fastest."""
