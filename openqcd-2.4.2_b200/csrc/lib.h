@@ -231,6 +231,18 @@ inline int copy_now(const Ctx &c, void *dst, const void *src, size_t bytes) {
              : -1;
 }
 
+// Buffers that are there together or not at all: if one of them cannot be had,
+// those made so far are freed and every pointer is null again, so that a guard
+// on any of the pointers stands for all of them.  0, or -1.
+struct Buffer {
+  void **p;
+  size_t bytes;
+  bool host;   // page-locked host memory
+};
+template <typename T> Buffer dev_buf(T *&p, size_t n) { return {(void **)&p, n * sizeof(T), false}; }
+template <typename T> Buffer host_buf(T *&p, size_t n) { return {(void **)&p, n * sizeof(T), true}; }
+int alloc_all(std::initializer_list<Buffer> want);
+
 // dd.cu: domain decomposition along x0
 int dd_buffers(Ctx &c);
 int dd_exchange(Ctx &c, size_t bytes, cudaStream_t st);

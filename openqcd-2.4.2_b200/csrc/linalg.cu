@@ -205,12 +205,27 @@ __global__ void k_unorm(Geom g, const void *__restrict__ x, int c0, int nch, Fin
   }
 }
 
+int alloc_all(std::initializer_list<Buffer> want) {
+  bool ok = true;
+  for (const Buffer &b : want) {
+    *b.p = nullptr;
+    if (!ok) continue;
+    ok = (b.host ? cudaMallocHost(b.p, b.bytes) : cudaMalloc(b.p, b.bytes)) == cudaSuccess;
+    if (!ok) *b.p = nullptr;
+  }
+  if (ok) return 0;
+  for (const Buffer &b : want) {
+    if (b.host) cudaFreeHost(*b.p);
+    else cudaFree(*b.p);
+    *b.p = nullptr;
+  }
+  cudaGetLastError();   // reported by the caller, not by the next launch
+  return -1;
+}
+
 int la_buffers(Ctx &c) {
   if (c.red) return 0;
-  if (cudaMalloc(&c.red, (size_t)RB * 4 * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c.red_out, 8 * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c.red_cnt, sizeof(unsigned)) != cudaSuccess ||
-      cudaMallocHost(&c.h_red, 8 * sizeof(double)) != cudaSuccess)
+  if (alloc_all({dev_buf(c.red, (size_t)RB * 4), dev_buf(c.red_out, 8), dev_buf(c.red_cnt, 1), host_buf(c.h_red, 8)}))
     return fail("out of memory (reduction buffers)");
   cudaMemsetAsync(c.red_cnt, 0, sizeof(unsigned), c.stream);
   return 0;
