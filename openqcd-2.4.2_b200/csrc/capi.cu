@@ -25,6 +25,7 @@ void set_error(const std::string &m) { g_err = m; }
 
 int fail(const std::string &msg) {
   g_err = msg;
+  cudaGetLastError();   // reported here, not by the launch check of the next call
   if (g_fatal) {
     fprintf(stderr, "\nError in openqcd_b200: %s\nProgram aborted\n", msg.c_str());
     fflush(stderr);

@@ -53,6 +53,12 @@ static int dfl_alloc(Ctx &c) {
   const int Ns = d.Ns, nb = c.g.nbl;
   d.nb = nb;
   d.nv = Ns * nb;
+  d.ready = d.have_basis = false;   // until everything is there
+  auto grab = [](auto *&p, size_t bytes) {
+    cudaFree(p);
+    p = nullptr;
+    return cudaMalloc(&p, bytes) == cudaSuccess;
+  };
   // block tables
   std::vector<int> bco(nb), v2l(nb), l2v(nb), nbr(8 * nb);
   copy_now(c, bco.data(), c.d_bcoord, nb * sizeof(int));
@@ -71,13 +77,10 @@ static int dfl_alloc(Ctx &c) {
       nbr[8 * n + ifc] = l2v[lb];
     }
   }
-  auto up = [&c](int *&p, const std::vector<int> &v) {
-    cudaFree(p);
-    cudaMalloc(&p, v.size() * sizeof(int));
-    copy_now(c, p, v.data(), v.size() * sizeof(int));
+  auto up = [&](int *&p, const std::vector<int> &v) {
+    return grab(p, v.size() * sizeof(int)) && !copy_now(c, p, v.data(), v.size() * sizeof(int));
   };
-  up(d.vd2lex, v2l);
-  up(d.nbr, nbr);
+  bool ok = up(d.vd2lex, v2l) && up(d.nbr, nbr);
   // sites (p << 16 | s) of a block on each of its 8 faces, block-local
   {
     const int *bs = c.g.bs;
@@ -96,8 +99,7 @@ static int dfl_alloc(Ctx &c) {
               if (y[mu] == ((ifc & 1) ? bs[mu] - 1 : 0)) fs[ifc * fmax + nf[ifc]++] = (p << 16) | (l >> 1);
             }
           }
-    up(d.faces, fs);
-    up(d.nfc, nf);
+    ok = ok && up(d.faces, fs) && up(d.nfc, nf);
     d.fmax = fmax;
   }
   // basis and matrices
@@ -107,27 +109,17 @@ static int dfl_alloc(Ctx &c) {
     cudaMemsetAsync(p, 0, spinor_bytes(c, 32), c.stream);
     d.basis.push_back(p);
   }
-  cudaFree(d.d_basis);
-  cudaMalloc(&d.d_basis, Ns * sizeof(void *));
-  copy_now(c, d.d_basis, d.basis.data(), Ns * sizeof(void *));
-  cudaFree(d.rpart);
-  if (cudaMalloc(&d.rpart, (size_t)nb * 2 * Ns * sizeof(double2)) != cudaSuccess)
+  if (!ok || !grab(d.d_basis, Ns * sizeof(void *)) || copy_now(c, d.d_basis, d.basis.data(), Ns * sizeof(void *)) ||
+      !grab(d.rpart, (size_t)nb * 2 * Ns * sizeof(double2)))
     return fail("out of device memory (deflation)");
   size_t m = (size_t)nb * Ns * Ns * sizeof(double2);
-  double2 **mats[] = {&d.Ablk, &d.Ainv, &d.Ahop, &d.Mhop};
-  size_t sz[] = {m, m, 8 * m, 8 * m};
-  for (int i = 0; i < 4; i++) {
-    cudaFree(*mats[i]);
-    if (cudaMalloc(mats[i], sz[i]) != cudaSuccess) return fail("out of device memory (little operator)");
-  }
-  cudaFree(d.Mhop32);
-  if (cudaMalloc(&d.Mhop32, 4 * m) != cudaSuccess) return fail("out of device memory (little operator)");
+  if (!grab(d.Ablk, m) || !grab(d.Ainv, m) || !grab(d.Ahop, 8 * m) || !grab(d.Mhop, 8 * m) || !grab(d.Mhop32, 4 * m))
+    return fail("out of device memory (little operator)");
   // the further masses' arrays have the old sizes
   for (auto &x : d.xsets)
     for (void *p : x) cudaFree(p);
   d.xsets.clear();
   d.aw_valid = d.awhat_valid = false;
-  d.have_basis = false;
   d.ready = true;
   return cudaGetLastError() == cudaSuccess ? 0 : fail("deflation: CUDA error in set-up");
 }
@@ -899,11 +891,14 @@ int dfl_subspace_dev(Ctx &c, const std::vector<void *> &modes, cudaStream_t st, 
   }
   float4 **dm = nullptr;
   int *dfail = nullptr;
-  cudaMallocAsync(&dm, d.Ns * sizeof(void *), st);
-  cudaMallocAsync(&dfail, sizeof(int), st);
+  if (!c.tmp64 && cudaMalloc(&c.tmp64, spinor_bytes(c, 64)) != cudaSuccess) return fail("out of device memory");
+  if (cudaMallocAsync(&dm, d.Ns * sizeof(void *), st) != cudaSuccess) return fail("out of device memory");
+  if (cudaMallocAsync(&dfail, sizeof(int), st) != cudaSuccess) {
+    cudaFreeAsync(dm, st);
+    return fail("out of device memory");
+  }
   cudaMemcpyAsync(dm, modes.data(), d.Ns * sizeof(void *), cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(dfail, 0, sizeof(int), st);
-  if (!c.tmp64 && cudaMalloc(&c.tmp64, spinor_bytes(c, 64)) != cudaSuccess) return fail("out of device memory");
   k_dfl_gs<<<d.nb, 256, 0, st>>>(c.g, d.vd2lex, (float4 *const *)d.d_basis, (const float4 *const *)dm, d.Ns,
                                  (double2 *)c.tmp64, dfail);
   int hf = 0;
@@ -954,7 +949,7 @@ int dfl_set_Awhat(Ctx &c, double mu, cudaStream_t st, bool diag_only) {
   if (dfl_set_Aw(c, mu, st, diag_only)) return -1;
   if (d.awhat_valid && !diag_only) return d.awhat_fail;
   int *dfail = nullptr;
-  cudaMallocAsync(&dfail, sizeof(int), st);
+  if (cudaMallocAsync(&dfail, sizeof(int), st) != cudaSuccess) return fail("out of device memory (little operator)");
   cudaMemsetAsync(dfail, 0, sizeof(int), st);
   size_t shm = (size_t)2 * d.Ns * d.Ns * sizeof(double2);
   cudaFuncSetAttribute(k_cinv, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -1032,10 +1027,8 @@ static int ltl_ensure(Ctx &c) {
     grown = true;
   }
   if (!d.lvtab) {
-    if (cudaMalloc(&d.lvtab, (2 * LMAXK + 8) * sizeof(double2 *)) != cudaSuccess ||
-        cudaMalloc(&d.ldots, 64 * sizeof(double2)) != cudaSuccess ||
-        cudaMalloc(&d.lpart, (size_t)LGRID * LMAXK * sizeof(double2)) != cudaSuccess ||
-        cudaMallocHost(&d.h_ldots, 4 * sizeof(double2)) != cudaSuccess)
+    if (alloc_all({dev_buf(d.lvtab, 2 * LMAXK + 8), dev_buf(d.ldots, 64), dev_buf(d.lpart, (size_t)LGRID * LMAXK),
+                   host_buf(d.h_ldots, 4)}))
       return fail("out of device memory (little solver)");
     grown = true;
   }
@@ -1077,7 +1070,9 @@ double dfl_ltl_gcr(Ctx &c, double mu, const double2 *eta, double2 *psi, int *ifa
   status[0] = 0;
   const size_t nv = (size_t)d.nv, nvh = nv / 2;
   const int nbh = d.nb / 2, n = (int)nvh;
-  if (dfl_set_Awhat(c, mu, st)) {
+  const int aw = dfl_set_Awhat(c, mu, st);
+  if (aw < 0) return -1.0;
+  if (aw) {
     ifail[0] = -2;
     cudaMemsetAsync(psi, 0, nv * sizeof(double2), st);
     return sqrt(lv_dot_re(c, eta, eta, nv, nullptr));
@@ -1214,6 +1209,7 @@ double dfl_sap_gcr_dev(Ctx &c, int nkv, int nmx, int istop, double res, double m
   if (sap_prepare(c, c.stream) || ensure_lvd(c)) return -1.0;
   cudaStream_t st = c.stream;
   double rho;
+  int aw = 0;
   {
     double r[2];
     if (istop) { la_unorm(c, 64, eta, PAR_ALL, r); rho = r[0]; }
@@ -1221,7 +1217,8 @@ double dfl_sap_gcr_dev(Ctx &c, int nkv, int nmx, int istop, double res, double m
   }
   if (c.isolv == 1 && (c.sw_inv_fail & 2)) {
     ifail[0] = -3;
-  } else if ((dfl_mark(c, 5), dfl_set_Awhat(c, mu, st))) {
+  } else if ((dfl_mark(c, 5), aw = dfl_set_Awhat(c, mu, st))) {
+    if (aw < 0) return -1.0;
     ifail[0] = -2;
   } else if ((dfl_mark(c, 2), rho != 0.0)) {
     if (reserve32(c, c.ws32, 2 * nkv + 3)) return -1.0;
@@ -1330,7 +1327,8 @@ int dfl_modes_dev(Ctx &c, uint64_t seed, int *ifail, int *status) {
     if (dfl_subspace_dev(c, d.modes, st)) return -1;
     dfl_mark(c, 1);
     for (; n < d.gen_ninv && ifail[0] == 0; n++) {
-      if (dfl_set_Awhat(c, d.gen_mu, st)) {
+      if (const int aw = dfl_set_Awhat(c, d.gen_mu, st)) {
+        if (aw < 0) return -1;
         ifail[0] = -2;
         break;
       }

@@ -568,8 +568,7 @@ int dfl_batch_alloc(Ctx &c) {
   DflState &d = c.dfl;
   if (d.bpart) return 0;
   const int ns = chunk_split(c.g.vbh);
-  if (cudaMalloc(&d.bpart, (size_t)d.nb * 2 * ns * BT * d.Ns * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&d.kerr, sizeof(int)) != cudaSuccess)
+  if (alloc_all({dev_buf(d.bpart, (size_t)d.nb * 2 * ns * BT * d.Ns), dev_buf(d.kerr, 1)}))
     return fail("out of device memory (batched deflation)");
   cudaMemsetAsync(d.kerr, 0, sizeof(int), c.stream);
   return 0;

@@ -219,7 +219,6 @@ int alloc_all(std::initializer_list<Buffer> want) {
     else cudaFree(*b.p);
     *b.p = nullptr;
   }
-  cudaGetLastError();   // reported by the caller, not by the next launch
   return -1;
 }
 

@@ -275,11 +275,8 @@ static int ensure_base(Ctx &c) {
   }
   LtlRef &q = *lr(c);
   if (!q.part) {
-    if (cudaMalloc(&q.part, (size_t)DG * 32 * sizeof(double2)) != cudaSuccess ||
-        cudaMalloc(&q.dots, VT * sizeof(double2)) != cudaSuccess ||
-        cudaMallocHost(&q.h_dots, VT * sizeof(double2)) != cudaSuccess ||
-        cudaMalloc(&q.t64, (size_t)q.nv * sizeof(double2)) != cudaSuccess ||
-        cudaMalloc(&q.t32, (size_t)q.nv * sizeof(float2)) != cudaSuccess)
+    if (alloc_all({dev_buf(q.part, (size_t)DG * 32), dev_buf(q.dots, VT), host_buf(q.h_dots, VT), dev_buf(q.t64, q.nv),
+                   dev_buf(q.t32, q.nv)}))
       return fail("out of device memory (little solver)");
   }
   return 0;

@@ -213,15 +213,11 @@ __global__ void k_wgrad_sum(const float2 *__restrict__ part, int nw, int ncta, d
 // ----------------------------------------------------------- host side
 static int net_alloc(Ctx &c) {
   NetState &n = c.net;
-  if (n.dev_w[0]) return 0;
-  for (int l = 0; l < NLAY; l++) {
-    if (cudaMalloc(&n.dev_w[l], wsize(l) * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&n.dev_wadj[l], wsize(l) * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&n.dev_w16[l], wsize(l) * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&n.dev_grad[l], wsize(l) * sizeof(double2)) != cudaSuccess)
+  for (int l = 0; l < NLAY; l++)
+    if (!n.dev_w[l] && alloc_all({dev_buf(n.dev_w[l], wsize(l)), dev_buf(n.dev_wadj[l], wsize(l)),
+                                  dev_buf(n.dev_w16[l], wsize(l)), dev_buf(n.dev_grad[l], wsize(l))}))
       return fail("out of device memory (network)");
-  }
-  if (cudaMalloc(&n.part, (size_t)WG_GRID * 9 * 64 * sizeof(float2)) != cudaSuccess)
+  if (!n.part && cudaMalloc(&n.part, (size_t)WG_GRID * 9 * 64 * sizeof(float2)) != cudaSuccess)
     return fail("out of device memory (network)");
   return 0;
 }

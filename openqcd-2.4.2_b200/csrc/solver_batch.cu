@@ -219,25 +219,14 @@ static int ltl_batch_alloc(Ctx &c, int nr) {
   DflState &d = c.dfl;
   const int nvec = 2 * d.nkv + 6;
   if (g_lb.base && g_lb.nsys >= nr && g_lb.nvec == nvec && g_lb.nv == (size_t)d.nv) return 0;
-  cudaFree(g_lb.base);
-  cudaFree(g_lb.part);
-  cudaFree(g_lb.dots);
-  cudaFree(g_lb.cnt);
-  cudaFree(g_lb.act);
-  if (g_lb.h_dots) cudaFreeHost(g_lb.h_dots);
-  if (g_lb.h_act) cudaFreeHost(g_lb.h_act);
-  g_lb = LtlBatch();
+  ltl_batch_release();
+  if (alloc_all({dev_buf(g_lb.base, (size_t)nr * nvec * d.nv), dev_buf(g_lb.part, (size_t)nr * BGRID * BK),
+                 dev_buf(g_lb.dots, (size_t)nr * 64), dev_buf(g_lb.act, nr), dev_buf(g_lb.cnt, nr),
+                 host_buf(g_lb.h_dots, (size_t)nr * 64), host_buf(g_lb.h_act, nr)}))
+    return fail("out of device memory (batched little solver)");
   g_lb.nvec = nvec;
   g_lb.nsys = nr;
   g_lb.nv = (size_t)d.nv;
-  if (cudaMalloc(&g_lb.base, (size_t)nr * nvec * d.nv * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&g_lb.part, (size_t)nr * BGRID * BK * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&g_lb.dots, (size_t)nr * 64 * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&g_lb.act, nr * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&g_lb.cnt, nr * sizeof(unsigned)) != cudaSuccess ||
-      cudaMallocHost(&g_lb.h_dots, (size_t)nr * 64 * sizeof(double2)) != cudaSuccess ||
-      cudaMallocHost(&g_lb.h_act, nr * sizeof(int)) != cudaSuccess)
-    return fail("out of device memory (batched little solver)");
   cudaMemsetAsync(g_lb.cnt, 0, nr * sizeof(unsigned), c.stream);
   return 0;
 }
@@ -259,7 +248,9 @@ int ltl_gcr_b(Ctx &c, double mu, int nr, const double2 *const *eta, double2 *con
               cudaStream_t st) {
   DflState &d = c.dfl;
   for (int r = 0; r < nr; r++) ifail[r] = status[r] = 0;
-  if (dfl_set_Awhat(c, mu, st)) {
+  const int aw = dfl_set_Awhat(c, mu, st);
+  if (aw < 0) return -1;
+  if (aw) {
     for (int r = 0; r < nr; r++) {
       ifail[r] = -2;
       cudaMemsetAsync(psi[r], 0, (size_t)d.nv * sizeof(double2), st);

@@ -19,7 +19,7 @@ std::map<char *, size_t> g_mem;        // live allocations, device and page-lock
 std::map<char *, size_t> g_dev;        // the device ones
 std::map<const void *, std::string> g_name;
 std::vector<Watch> g_watch;
-int g_allocs, g_fail_at, g_legacy, g_null, g_launches;
+int g_allocs, g_fail_at, g_legacy, g_null, g_launches, g_bad_frees;
 cudaError_t g_last;
 
 cudaError_t err(cudaError_t e) {
@@ -37,7 +37,7 @@ cudaError_t alloc(void **p, size_t n, bool dev) {
 }
 cudaError_t release(void *p) {
   if (!p) return cudaSuccess;
-  if (!g_mem.erase((char *)p)) return err(cudaErrorInvalidValue);
+  if (!g_mem.erase((char *)p)) return g_bad_frees++, err(cudaErrorInvalidValue);
   g_dev.erase((char *)p);
   free(p);
   return cudaSuccess;
@@ -51,7 +51,7 @@ size_t room(const void *p) {
   return off < it->second ? it->second - off : (size_t)-1;
 }
 cudaError_t copy(void *d, const void *s, size_t n) {
-  if (n > room(d) || n > room(s)) return err(cudaErrorInvalidValue);
+  if (!d || !s || n > room(d) || n > room(s)) return err(cudaErrorInvalidValue);
   memmove(d, s, n);
   return cudaSuccess;
 }
@@ -72,6 +72,7 @@ int fake_legacy() { return g_legacy; }
 int fake_launches() { return g_launches; }
 void fake_watch(const char *kernel, int arg, int n) { g_watch.push_back({kernel, arg, n}); }
 int fake_null_args() { return g_null; }
+int fake_bad_frees() { return g_bad_frees; }
 
 // -------------------------------------------------------------- the runtime
 cudaError_t cudaMalloc(void **p, size_t n) { return alloc(p, n, true); }
@@ -90,7 +91,7 @@ cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { retur
 cudaError_t cudaMemset(void *d, int v, size_t n) { return g_legacy++, memset(d, v, n), cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t st) {
   g_legacy += st == nullptr;
-  if (n > room(d)) return err(cudaErrorInvalidValue);
+  if (!d || n > room(d)) return err(cudaErrorInvalidValue);
   return memset(d, v, n), cudaSuccess;
 }
 cudaError_t cudaMemcpy2DAsync(void *d, size_t dp, const void *s, size_t sp, size_t w, size_t h, cudaMemcpyKind,

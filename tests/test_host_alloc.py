@@ -39,3 +39,91 @@ def test_reduction_buffers(qb, n):
     x.norm2()
     assert f.b200_last_error() == b"" and f.fake_launches() == launches + 1
     assert f.fake_null_args() == 0 and f.fake_live() == live + 4
+
+
+def _deflated(qb):
+    nv = qb.set_dfl_parms(BS, NS)
+    qb.set_dfl_pro_parms(2, 2, 1e-2, 2, 1e-2)
+    for l in range(NS):
+        qb.dfl_set_basis(l, np.ones(24 * V, np.float32))
+    return nv
+
+
+def _every_failure(prepare, call, watched):
+    """call(qb, state) with its n-th allocation failing, for every n, and again
+    without a failure, in a library of its own each time"""
+    n, seen = 1, 0
+    while True:
+        qb = hostlib.load()
+        qb.geometry(L, BS, qb.even_first_ipt(L))
+        qb.set_parms(1.5, 0.0, 0)
+        qb.random_ud(0.3, 1)
+        qb.sw_term()
+        qb.set_sap_parms(BS, 1, 4, 2)
+        state = prepare(qb)
+        f = qb.lib()
+        for w in watched:
+            f.fake_watch(*w)
+        f.fake_fail_at(n)
+        f.b200_clear_error()
+        try:
+            call(qb, state)
+            error = f.b200_last_error().decode()
+        except qb.B200Error as e:
+            error = str(e)
+        if "memory" in error or "allocation" in error:
+            seen += 1
+        elif f.fake_allocs() < n:
+            assert not error or "unsafe" in error
+            return n - 1, seen      # the call makes no more than that
+        f.fake_fail_at(0)
+        f.b200_clear_error()
+        try:
+            call(qb, state)
+        except qb.B200Error as e:       # without its kernels' results a call may find its data degenerate
+            assert "unsafe" in str(e)
+        assert f.fake_null_args() == 0 and f.fake_bad_frees() == 0, n
+        n += 1
+
+
+def test_deflation_parameters():
+    def call(qb, _):
+        try:
+            assert qb.set_dfl_parms(BS, NS) > 0
+        except qb.B200Error:
+            with pytest.raises(qb.B200Error, match="not set"):     # nothing works on what is left of it
+                qb.dfl_s2vd(np.ones(24 * V, np.float32), 1)
+            raise qb.B200Error("out of memory")
+    total, seen = _every_failure(lambda qb: None, call, [])
+    assert seen == total >= 13
+
+
+@pytest.mark.parametrize("what", ["dfl_modes", "dfl_sap_gcr", "ltl_gcr", "ltl_gcr_ref", "batch", "network"])
+def test_solver_workspaces(what):
+    def prepare(qb):
+        nv = _deflated(qb)
+        qb.set_dfl_gen_parms(0.125, 0.0, 4, 4, 2)
+        E, P = ([qb.DevField(64) for _ in range(2)] for _ in range(2))
+        qb.dev_gcr_batch(2, 2, 0, 1e-10, [0.0] * 2, E, P)      # what a batch without deflation needs is there
+        if what == "ltl_gcr_ref":
+            qb.dfl_subspace([np.ones(24 * V, np.float32)] * NS)
+            qb.set_ltl_solver(1)
+        return nv, E, P, [qb.DevField(32) for _ in range(2)]
+
+    def call(qb, s):
+        nv, E, P, R = s
+        if what == "dfl_modes":
+            qb.dfl_modes(1)
+        elif what == "dfl_sap_gcr":
+            qb.dev_dfl_sap_gcr(2, 2, 0, 1e-10, 0.0, E[0], P[0])
+        elif what == "batch":
+            qb.dev_gcr_batch(2, 2, 0, 1e-10, [0.0] * 2, E, P, dfl=True)
+        elif what == "network":
+            qb.net_init(1, 0.25)
+            qb.net_grad(*R)
+        else:
+            qb.ltl_gcr(0.0, np.ones(2 * nv))
+    # the tables, partial sums, counters and results of the little solvers' sums
+    watched = [(b"k_bmdot", k, 1) for k in (0, 3, 8, 9, 10)] + [(b"k_bcopy", 0, 1), (b"k_mdot", 0, 1), (b"k_cinv", 3, 1)]
+    total, seen = _every_failure(prepare, call, watched)
+    assert total >= 4 and seen >= total - 1      # the SAP input field has a stand-in
