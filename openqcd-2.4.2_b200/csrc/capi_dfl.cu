@@ -57,21 +57,21 @@ static int stage_bytes_ok(Ctx &c, size_t n) {
 
 // reference-layout FP32 field (host or device) -> device-layout field
 static int ref32_in(Ctx &c, const void *q, void *dev) {
-  if (ref_direct(c, q)) return spinor_from_ref(c, 32, q, dev, c.stream);
-  size_t nb = spinor_bytes(c, 32);
+  const size_t nb = spinor_bytes(c, 32);
+  if (ref_direct(c, q, nb)) return spinor_from_ref(c, 32, q, dev, c.stream);
   if (stage_bytes_ok(c, nb)) return -1;
-  cudaMemcpyAsync(c.stage, q, nb, cudaMemcpyDefault, c.stream);
+  if (cudaMemcpyAsync(c.stage, q, nb, cudaMemcpyDefault, c.stream) != cudaSuccess) return fail("cannot read the field");
   return spinor_from_ref(c, 32, c.stage, dev, c.stream);
 }
 
 static int ref32_out(Ctx &c, const void *dev, void *q) {
-  if (ref_direct(c, q)) {
+  const size_t nb = spinor_bytes(c, 32);
+  if (ref_direct(c, q, nb)) {
     if (spinor_to_ref(c, 32, dev, q, c.stream)) return -1;
   } else {
-    size_t nb = spinor_bytes(c, 32);
     if (stage_bytes_ok(c, nb)) return -1;
     if (spinor_to_ref(c, 32, dev, c.stage, c.stream)) return -1;
-    cudaMemcpyAsync(q, c.stage, nb, cudaMemcpyDefault, c.stream);
+    if (cudaMemcpyAsync(q, c.stage, nb, cudaMemcpyDefault, c.stream) != cudaSuccess) return fail("cannot write the field");
   }
   return cudaStreamSynchronize(c.stream) == cudaSuccess ? 0 : fail("CUDA error");
 }

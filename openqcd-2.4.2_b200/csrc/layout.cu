@@ -339,15 +339,34 @@ int spinor_to_ref_range(const Ctx &c, int prec, const void *dev, void *q, int d0
   return cudaGetLastError() == cudaSuccess ? 0 : fail("spinor_to_ref: launch failed");
 }
 
+// bytes from p to the end of its device allocation, 0 if that cannot be told
+static size_t room_from(const void *p) {
+  using Fn = int (*)(unsigned long long *, size_t *, unsigned long long);   // cuMemGetAddressRange
+  static const Fn fn = [] {
+    void *f = nullptr;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, nullptr) != cudaSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return (Fn)f;
+  }();
+  unsigned long long base = 0;
+  size_t n = 0;
+  if (!fn || fn(&base, &n, (unsigned long long)(uintptr_t)p)) return 0;
+  return (size_t)(base + n - (unsigned long long)(uintptr_t)p);
+}
+
 // whether the conversions can work on the caller's array itself: memory of
-// the library's device, aligned for 16-byte accesses
-bool ref_direct(const Ctx &c, const void *q) {
+// the library's device, aligned for 16-byte accesses, and all of it within its
+// allocation (a copy to or from a shorter array is refused by the runtime; a
+// kernel would read or write what lies behind it)
+bool ref_direct(const Ctx &c, const void *q, size_t bytes) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return a.type == cudaMemoryTypeDevice && a.device == c.dev && (uintptr_t)q % 16 == 0;
+  return a.type == cudaMemoryTypeDevice && a.device == c.dev && (uintptr_t)q % 16 == 0 && room_from(q) >= bytes;
 }
 
 int spinor_from_ref(const Ctx &c, int prec, const void *q, void *dev, cudaStream_t st) {

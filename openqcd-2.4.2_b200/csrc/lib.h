@@ -280,7 +280,7 @@ int spinor_from_ref_piece(const Ctx &c, int prec, const void *q, void *dev, cons
 void pipeline_plan(const int L[4], const int bs[4], const int *ipt, std::vector<Piece> &piece,
                    std::vector<Slab> &slab);
 int spinor_to_ref(const Ctx &c, int prec, const void *dev, void *q, cudaStream_t st);
-bool ref_direct(const Ctx &c, const void *q);   // the conversions can work on this array itself
+bool ref_direct(const Ctx &c, const void *q, size_t bytes);   // the conversions can work on this array itself
 int links_from_ref(Ctx &c, const void *qud, cudaStream_t st);                           // qud on device
 int links_to_ref(const Ctx &c, void *qud, cudaStream_t st);
 int pauli_from_ref(Ctx &c, const void *qsw, cudaStream_t st);                           // qsw on device

@@ -108,6 +108,17 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
   a->type = dev ? cudaMemoryTypeDevice : room(p) != (size_t)-1 ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
   return cudaSuccess;
 }
+static int address_range(unsigned long long *base, size_t *n, unsigned long long p) {
+  auto it = g_dev.upper_bound((char *)p);
+  if (it == g_dev.begin() || (char *)p >= std::prev(it)->first + std::prev(it)->second) return 1;
+  *base = (unsigned long long)std::prev(it)->first;
+  *n = std::prev(it)->second;
+  return 0;
+}
+cudaError_t cudaGetDriverEntryPoint(const char *name, void **f, unsigned long long, cudaDriverEntryPointQueryResult *) {
+  *f = strcmp(name, "cuMemGetAddressRange") ? nullptr : (void *)address_range;
+  return *f ? cudaSuccess : err(cudaErrorInvalidValue);
+}
 cudaError_t cudaGetLastError() {
   const cudaError_t e = g_last;
   g_last = cudaSuccess;
