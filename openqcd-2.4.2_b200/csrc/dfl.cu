@@ -1288,9 +1288,20 @@ int dfl_modes_dev(Ctx &c, uint64_t seed, int *ifail, int *status) {
     float4 **p;
     ~FreeTab() { cudaFree(p); }
   } free_tab{dmodes};
-  // generation mass and eo flag
-  const double m0_save = c.m0;
-  const int eo_save = c.eoflg;
+  // generation mass and eo flag, and the caller's ones again on every way out
+  struct Parms {
+    Ctx &c;
+    cudaStream_t st;
+    const double m0;
+    const int eo;
+    int restore() {
+      c.eoflg = eo;
+      const int rc = c.m0 == m0 ? 0 : sw_shift_mass(c, m0 - c.m0, st);
+      c.m0 = m0;
+      return rc;
+    }
+    ~Parms() { restore(); }
+  } parms{c, st, c.m0, c.eoflg};
   const double m0g = 1.0 / (2.0 * d.gen_kappa) - 4.0;
   if (m0g != c.m0) {
     if (sw_shift_mass(c, m0g - c.m0, st)) return -1;
@@ -1394,12 +1405,7 @@ int dfl_modes_dev(Ctx &c, uint64_t seed, int *ifail, int *status) {
   } else {
     if (dfl_subspace_dev(c, d.modes, st)) return -1;
   }
-  // restore the mass and the eo flag
-  c.eoflg = eo_save;
-  if (c.m0 != m0_save) {
-    if (sw_shift_mass(c, m0_save - c.m0, st)) return -1;
-    c.m0 = m0_save;
-  }
+  if (parms.restore()) return -1;
   d.aw_valid = d.awhat_valid = false;
   // the modes are regenerated from random fields by every call
   for (void *p : d.modes) cudaFree(p);

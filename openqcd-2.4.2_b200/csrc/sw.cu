@@ -582,7 +582,11 @@ int sw_shift_mass(Ctx &c, double dm, cudaStream_t st) {
   }
   int t = 128;
   k_sw_shift<<<(c.g.vol + t - 1) / t, t, 0, st>>>(c.g, c.swd, dm);
-  return sw_refresh_derived(c, st);
+  if (sw_refresh_derived(c, st)) {
+    c.have_sw = false;   // neither the old term nor the new one
+    return -1;
+  }
+  return 0;
 }
 
 // ------------------------------------------------------------ FP32 links

@@ -18,6 +18,7 @@ struct Watch {
 std::map<char *, size_t> g_mem;        // live allocations, device and page-locked
 std::map<char *, size_t> g_dev;        // the device ones
 std::map<const void *, std::string> g_name;
+std::map<std::string, int> g_count;    // launches by kernel
 std::vector<Watch> g_watch;
 int g_allocs, g_fail_at, g_legacy, g_null, g_launches, g_bad_frees;
 cudaError_t g_last;
@@ -71,6 +72,12 @@ int fake_live() { return (int)g_mem.size(); }
 int fake_legacy() { return g_legacy; }
 int fake_launches() { return g_launches; }
 void fake_watch(const char *kernel, int arg, int n) { g_watch.push_back({kernel, arg, n}); }
+int fake_launched(const char *kernel) {
+  int n = 0;
+  for (const auto &k : g_count)
+    if (k.first.find(kernel) != std::string::npos) n += k.second;
+  return n;
+}
 int fake_null_args() { return g_null; }
 int fake_bad_frees() { return g_bad_frees; }
 
@@ -170,6 +177,7 @@ cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **args, size_t,
   g_legacy += st == nullptr;
   if (!g.x || !g.y || !g.z || !b.x || b.x * b.y * b.z > 1024) return err(cudaErrorInvalidConfiguration);
   const std::string &name = g_name[f];
+  g_count[name]++;
   for (const Watch &w : g_watch)
     if (name.find(w.kernel) != std::string::npos)
       for (int i = 0; i < w.n; i++) g_null += ((void **)args[w.arg])[i] == nullptr;

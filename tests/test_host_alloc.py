@@ -127,3 +127,27 @@ def test_solver_workspaces(what):
     watched = [(b"k_bmdot", k, 1) for k in (0, 3, 8, 9, 10)] + [(b"k_bcopy", 0, 1), (b"k_mdot", 0, 1), (b"k_cinv", 3, 1)]
     total, seen = _every_failure(prepare, call, watched)
     assert total >= 4 and seen >= total - 1      # the SAP input field has a stand-in
+
+
+def test_subspace_generation_restores_the_mass():
+    """the generation mass and the eo flag do not outlive a call that failed"""
+    def prepare(qb):
+        _deflated(qb)
+        qb.set_dfl_gen_parms(0.11, 0.02, 4, 4, 2)
+        qb.dirac_ref("Dw", 64, 0.0, np.ones(24 * V))
+        return qb.lib().fake_launched
+
+    def call(qb, launched):
+        before = launched(b"k_sw_shift")
+        try:
+            qb.dfl_modes(1)
+        finally:
+            shifts = launched(b"k_sw_shift") - before
+            try:
+                qb.dirac_ref("Dw", 64, 0.0, np.ones(24 * V))
+                assert shifts % 2 == 0              # there and back
+            except qb.B200Error as e:
+                assert "SW field" in str(e)         # or the SW term is gone, and said to be
+                qb.sw_term()
+    total, seen = _every_failure(prepare, call, [])
+    assert seen == total >= 20
