@@ -333,7 +333,8 @@ int b200_geometry(const int L[4], const int bs[4], const int *ipt) {
   c.ud = nullptr; c.u32 = nullptr; c.swd = c.swd_inv = nullptr; c.sw32 = c.sw32_inv = nullptr;
   c.tmp64 = c.tmp32 = c.stage = nullptr; c.stage_bytes = 0;
   c.u16 = c.sw16 = c.sw16_inv = nullptr; c.h16_valid = false;
-  c.sap_tuned_vbh[0] = c.sap_tuned_vbh[1] = c.sap_tuned_vbh[2] = 0;
+  for (auto &m : c.sap_tuned)
+    for (auto &t : m) t.vbh = 0;
   c.u12 = nullptr; c.u12_valid = c.u12_ok = false;
   c.sap_fld[0] = c.sap_fld[1] = c.sap_fld[2] = nullptr;
   c.sap_mfld[0] = c.sap_mfld[1] = c.sap_mfld[2] = nullptr;
@@ -610,10 +611,10 @@ int b200_sap_tuning(int prec, int *variant, int *threads, float *ms) {
   Ctx &c = ctx();
   if (check_ready(c)) return -1;
   const int slot = prec == 16 ? 1 : (prec == 12 ? 2 : 0);
-  if (c.sap_tuned_vbh[slot] != c.g.vbh) return fail("sap_tuning: the SAP kernel is not tuned for this geometry yet");
-  *variant = c.sap_variant[slot];
-  *threads = qcd::sap_variant_threads(c, slot);
-  *ms = c.sap_tuned_ms[slot];
+  const Ctx::SapTuned *t = qcd::sap_tuned_one(c, slot, threads);
+  if (!t) return fail("sap_tuning: the SAP kernel is not tuned for this geometry yet");
+  *variant = t->variant;
+  *ms = t->ms;
   return 0;
 }
 

@@ -162,10 +162,13 @@ struct Ctx {
   int sap_prec = 32;
   void *u16 = nullptr, *sw16 = nullptr, *sw16_inv = nullptr;
   bool h16_valid = false;
-  // SAP block-kernel launch variant chosen by the autotuner, per storage
-  // precision (0: FP32, 1: FP16), for the block size it was tuned on
-  int sap_variant[3] = {0, 0, 0}, sap_tuned_vbh[3] = {0, 0, 0};
-  float sap_tuned_ms[3] = {0.0f, 0.0f, 0.0f};
+  // SAP block-kernel launch variant chosen by the autotuner, per storage mode
+  // (0: FP32, 1: FP16, 2: FP32 with 12-real links) and size of launch (0: one
+  // CTA per SM at most, 1: more), for the block size it was tuned on
+  struct SapTuned {
+    int variant = 0, vbh = 0;
+    float ms = 0.0f;
+  } sap_tuned[3][2];
   // 12-real FP32 links for the SAP block solver (first two rows; the third
   // is rebuilt), used when every link passes the SU(3) check
   int sap_link12 = 1;
@@ -471,8 +474,8 @@ double dfl_sap_gcr_dev(Ctx &c, int nkv, int nmx, int istop, double res, double m
 int dfl_modes_dev(Ctx &c, uint64_t seed, int *ifail, int *status);
 
 // sap.cu
-int sap_prepare(Ctx &c, cudaStream_t st);
-int sap_variant_threads(const Ctx &c, int slot);
+int sap_prepare(Ctx &c, cudaStream_t st, int nsys = 1);
+const Ctx::SapTuned *sap_tuned_one(const Ctx &c, int slot, int *threads);   // launches of one system
 int sap_set_variant(Ctx &c, int v);
 int sap_storage_mode(Ctx &c);
 int sap_cycle(Ctx &c, float mu, int isolv, int nmr, void *psi, void *rho, void *phi_blk, cudaStream_t st);

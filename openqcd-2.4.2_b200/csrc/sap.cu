@@ -730,7 +730,7 @@ static int pick_threads(int vbh, int &ns) {
 // Launch variants of the even-odd block kernel: sites per lane pair, the
 // launch bound and the register budget it implies.  The autotuner below
 // times every variant that fits the block on the resident fields and keeps
-// the fastest per block size and storage mode.
+// the fastest per block size, storage mode and size of launch.
 // Which one wins, in us per cycle of four MR steps:
 //   ns maxt (registers)   8^4, 4^4 blocks  32^4, 4^4  4x4x6x4   48x24^3, 6^4  8x4x6x8
 //   1   512 (128)               72            769        -              -             -
@@ -861,12 +861,22 @@ static int sap_mode(Ctx &c, int isolv, cudaStream_t st) {
   return c.u12_ok ? 2 : 0;
 }
 
+// The choice for launches of nsys systems.  One CTA per SM at most, or more:
+// with several systems the first can become the second, and the variant that
+// wins one (one CTA of 255 registers per SM) loses the other: six GCR steps of
+// four systems on 16^4 with 4^4 blocks 9.24 ms with the one-system choice,
+// 8.11 ms with its own; on 24^2x16x8 with 4x6x8x4 blocks 11.77 and 10.61 ms.
+static Ctx::SapTuned &sap_tuned(Ctx &c, int mode, int nsys) { return c.sap_tuned[mode][c.g.nbl / 2 * nsys > 148]; }
+
+static void launch_eo(const Ctx &c, const SapArgs &a, int variant, int mode, cudaStream_t st) {
+  const EoVariant &v = kEo[variant];
+  v.k[mode]<<<c.g.nbl / 2 * a.nsys, eo_threads(v, c.g.vbh), eo_smem(c.g.vbh), st>>>(a);
+}
+
 static void launch_blocks(Ctx &c, const SapArgs &a, int isolv, int mode, cudaStream_t st) {
   const int nbh = c.g.nbl / 2;
   if (isolv) {
-    const EoVariant &v = kEo[c.sap_variant[mode]];
-    const int t = eo_threads(v, c.g.vbh);
-    v.k[mode]<<<nbh * a.nsys, t, eo_smem(c.g.vbh), st>>>(a);
+    launch_eo(c, a, sap_tuned(c, mode, a.nsys).variant, mode, st);
   } else {
     int ns;
     int t = pick_threads(c.g.vbh, ns);
@@ -899,9 +909,12 @@ static SapArgs sap_args(Ctx &c, float mu, int nmr, int mode, void *psi, void *rh
 }
 
 // Time every fitting variant of the even-odd block kernel (both colours, 4
-// MR steps, on a random residual) and keep the fastest.
-static int sap_autotune(Ctx &c, int mode, cudaStream_t st) {
-  if (c.sap_tuned_vbh[mode] == c.g.vbh) return 0;
+// MR steps, on random residuals) and keep the fastest: on one system if that
+// makes a launch of the size in question, or on nsys of them, or as many as
+// there is room for.
+static int sap_autotune(Ctx &c, int mode, int nsys, cudaStream_t st) {
+  Ctx::SapTuned &best = sap_tuned(c, mode, nsys);
+  if (best.vbh == c.g.vbh) return 0;
   bool fits = false;
   for (int i = 0; i < kNEo; i++) {
     for (int m = 0; m < 3; m++)
@@ -909,28 +922,37 @@ static int sap_autotune(Ctx &c, int mode, cudaStream_t st) {
     fits |= eo_threads(kEo[i], c.g.vbh) != 0;
   }
   if (!fits) return fail("sap: block too large for shared memory");
+  if (&best == &sap_tuned(c, mode, 1)) nsys = 1;
   const size_t nb = spinor_bytes(c, 32);
-  void *psi = nullptr, *rho = nullptr, *phi = nullptr;
-  if (cudaMallocAsync(&psi, nb, st) != cudaSuccess || cudaMallocAsync(&rho, nb, st) != cudaSuccess ||
-      cudaMallocAsync(&phi, nb, st) != cudaSuccess)
-    return fail("sap: out of device memory (autotuning)");
-  cudaMemsetAsync(psi, 0, nb, st);
+  char *fld = nullptr;   // psi, rho and phi of every system
+  while (cudaMallocAsync(&fld, 3 * nb * nsys, st) != cudaSuccess) {
+    cudaGetLastError();
+    fld = nullptr;
+    if (nsys == 1) return fail("sap: out of device memory (autotuning)");
+    nsys = (nsys + 1) / 2;
+  }
+  cudaMemsetAsync(fld, 0, nb * nsys, st);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  int best = -1;
-  float best_ms = 0.0f;
+  int win = -1;
+  float win_ms = 0.0f;
+  SapArgs a = sap_args(c, 0.0f, 4, mode, fld, nullptr, nullptr);
+  a.nsys = nsys;
+  for (int r = 0; r < nsys; r++) {
+    a.psi[r] = (float4 *)(fld + nb * r);
+    a.rho[r] = (float4 *)(fld + nb * (nsys + r));
+    a.phi[r] = (float4 *)(fld + nb * (2 * nsys + r));
+  }
   for (int i = 0; i < kNEo; i++) {
     if (!eo_threads(kEo[i], c.g.vbh)) continue;
-    c.sap_variant[mode] = i;
-    SapArgs a = sap_args(c, 0.0f, 4, mode, psi, rho, phi);
     float tot = 0.0f;
     for (int rep = 0; rep < 4; rep++) {
-      gen_uniform_spinor32(c, rho, 977ull + rep, st);
+      for (int r = 0; r < nsys; r++) gen_uniform_spinor32(c, a.rho[r], 977ull + rep, st);
       cudaEventRecord(e0, st);
       for (int ic = 0; ic < 2; ic++) {
         a.colour = ic;
-        launch_blocks(c, a, 1, mode, st);
+        launch_eo(c, a, i, mode, st);
       }
       cudaEventRecord(e1, st);
       cudaEventSynchronize(e1);
@@ -939,25 +961,28 @@ static int sap_autotune(Ctx &c, int mode, cudaStream_t st) {
       if (rep > 0) tot += ms;   // the first run warms up
     }
     if (cudaGetLastError() != cudaSuccess) continue;   // a variant that cannot launch is skipped
-    if (best < 0 || tot < best_ms) {
-      best = i;
-      best_ms = tot;
+    if (win < 0 || tot < win_ms) {
+      win = i;
+      win_ms = tot;
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaFreeAsync(psi, st);
-  cudaFreeAsync(rho, st);
-  cudaFreeAsync(phi, st);
-  if (best < 0) return fail("sap: no block-kernel variant fits this block size");
-  best = dd_rank0(c, best);   // every rank runs rank 0's choice (the same arithmetic everywhere)
-  c.sap_variant[mode] = best;
-  c.sap_tuned_vbh[mode] = c.g.vbh;
-  c.sap_tuned_ms[mode] = best_ms / 3.0f;
+  cudaFreeAsync(fld, st);
+  if (win < 0) return fail("sap: no block-kernel variant fits this block size");
+  best.variant = dd_rank0(c, win);   // every rank runs rank 0's choice (the same arithmetic everywhere)
+  best.vbh = c.g.vbh;
+  best.ms = win_ms / 3.0f;
   return cudaStreamSynchronize(st) == cudaSuccess ? 0 : fail("sap: CUDA error while autotuning");
 }
 
-int sap_variant_threads(const Ctx &c, int slot) { return eo_threads(kEo[c.sap_variant[slot]], c.g.vbh); }
+// the choice for launches of one system, null if there is none yet
+const Ctx::SapTuned *sap_tuned_one(const Ctx &c, int slot, int *threads) {
+  const Ctx::SapTuned &t = sap_tuned(const_cast<Ctx &>(c), slot, 1);
+  if (t.vbh != c.g.vbh) return nullptr;
+  *threads = eo_threads(kEo[t.variant], c.g.vbh);
+  return &t;
+}
 
 // Fix the launch variant of the even-odd block kernel for the current block
 // size and storage mode (-1: tune again on the next use).
@@ -965,19 +990,17 @@ int sap_set_variant(Ctx &c, int v) {
   const int mode = sap_mode(c, 1, c.stream);
   if (mode < 0) return -1;
   if (v < 0) {
-    c.sap_tuned_vbh[mode] = 0;
+    for (auto &t : c.sap_tuned[mode]) t.vbh = 0;
     return 0;
   }
   if (v >= kNEo || !eo_threads(kEo[v], c.g.vbh))
     return fail("sap: this launch variant does not fit the block size");
   cudaFuncSetAttribute(kEo[v].k[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, SAP_SMEM_MAX);
-  c.sap_variant[mode] = v;
-  c.sap_tuned_vbh[mode] = c.g.vbh;
-  c.sap_tuned_ms[mode] = 0.0f;
+  for (auto &t : c.sap_tuned[mode]) t = {v, c.g.vbh, 0.0f};
   return 0;
 }
 
-int sap_prepare(Ctx &c, cudaStream_t st) {
+int sap_prepare(Ctx &c, cudaStream_t st, int nsys) {
   int ns;
   if (!pick_threads(c.g.vbh, ns)) return fail("sap: block volume too large (at most 1536 sites)");
   static bool attrs = false;
@@ -990,7 +1013,7 @@ int sap_prepare(Ctx &c, cudaStream_t st) {
   if (c.sap_prec == 16 && sap_half_fields(c, st)) return -1;
   const int mode = sap_mode(c, 1, st);
   if (mode < 0) return -1;
-  return sap_autotune(c, mode, st);
+  return sap_autotune(c, mode, nsys, st);
 }
 
 // storage mode in use (for reports): 0 FP32, 1 FP16, 2 FP32 with 12-real links
@@ -999,10 +1022,10 @@ int sap_storage_mode(Ctx &c) { return sap_mode(c, 1, c.stream); }
 // Everything a SAP cycle needs before its launches (storage mode, derived
 // link/SW copies, autotuned variant), done outside any stream capture.
 // Returns the storage mode or -1.
-static int sap_ready(Ctx &c, int isolv, cudaStream_t st) {
+static int sap_ready(Ctx &c, int isolv, cudaStream_t st, int nsys = 1) {
   const int mode = sap_mode(c, isolv, st);
   if (mode < 0) return -1;
-  if (isolv && c.sap_tuned_vbh[mode] != c.g.vbh && sap_prepare(c, st)) return -1;
+  if (isolv && sap_tuned(c, mode, nsys).vbh != c.g.vbh && sap_prepare(c, st, nsys)) return -1;
   if (mode == 1 && !c.h16_valid && sap_half_fields(c, st)) return -1;
   int ns;
   if (!pick_threads(c.g.vbh, ns) || (!isolv && (size_t)48 * c.g.vbh * sizeof(float) > (size_t)SAP_SMEM_MAX))
@@ -1069,10 +1092,10 @@ int sap_cycles_multi(Ctx &c, int n, float mu, int isolv, int nmr, int ncy, void 
       if (sap_cycles(c, mu, isolv, nmr, ncy, psi[r], rho[r], phi_blk[r], st)) return -1;
     return 0;
   }
-  const int mode = sap_ready(c, isolv, st);
-  if (mode < 0) return -1;
+  int mode = 0;
   for (int r0 = 0; r0 < n; r0 += SAP_MS) {
     const int m = n - r0 < SAP_MS ? n - r0 : SAP_MS;
+    if ((mode = sap_ready(c, isolv, st, m)) < 0) return -1;
     SapArgs a = sap_args(c, mu, nmr, mode, psi[r0], rho[r0], phi_blk[r0]);
     a.nsys = m;
     for (int r = 0; r < m; r++) {
@@ -1129,7 +1152,7 @@ int sap_mop(Ctx &c, float mu, int isolv, int nmr, int ncy, const void *rh, void 
   key.tag = 0x5a9;
   key.isolv = isolv;
   key.mode = mode;
-  key.variant = c.sap_variant[mode];
+  key.variant = sap_tuned(c, mode, 1).variant;
   key.ncy = ncy;
   key.a = sap_args(c, mu, nmr, mode, spsi, srho, sphi);
   if (base == srho) return fail("sap_mop: an input in the SAP input field needs a separate base");
@@ -1190,17 +1213,17 @@ int sap_mop_multi(Ctx &c, int ns, const float *mu, int isolv, int nmr, int ncy, 
     return 0;
   }
   const size_t fb = spinor_bytes(c, 32);
-  const int mode = sap_ready(c, isolv, st);
-  if (mode < 0) return -1;
   const size_t n = (size_t)c.g.vol * 6;   // float4 of a field
   for (int r0 = 0; r0 < ns; r0 += SAP_MS) {
     const int m = ns - r0 < SAP_MS ? ns - r0 : SAP_MS;
+    const int mode = sap_ready(c, isolv, st, m);
+    if (mode < 0) return -1;
     SapKey key;
     std::memset(&key, 0, sizeof(key));
     key.tag = 0x5aa;
     key.isolv = isolv;
     key.mode = mode;
-    key.variant = c.sap_variant[mode];
+    key.variant = sap_tuned(c, mode, m).variant;
     key.ncy = ncy;
     key.a = sap_args(c, mu[r0], nmr, mode, c.sap_mfld[0], c.sap_mfld[1], c.sap_mfld[2]);
     key.a.nsys = m;

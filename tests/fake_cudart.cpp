@@ -19,6 +19,8 @@ std::map<char *, size_t> g_mem;        // live allocations, device and page-lock
 std::map<char *, size_t> g_dev;        // the device ones
 std::map<const void *, std::string> g_name;
 std::map<std::string, int> g_count;    // launches by kernel
+std::string g_fast, g_last_kernel;
+int g_fast_ctas, g_last_ctas;
 std::vector<Watch> g_watch;
 int g_allocs, g_fail_at, g_legacy, g_null, g_launches, g_bad_frees;
 cudaError_t g_last;
@@ -71,6 +73,8 @@ int fake_allocs() { return g_allocs; }
 int fake_live() { return (int)g_mem.size(); }
 int fake_legacy() { return g_legacy; }
 int fake_launches() { return g_launches; }
+// the times that events measure: half as long after a launch of this kernel with up to so many CTAs
+void fake_fast(const char *kernel, int ctas) { g_fast = kernel, g_fast_ctas = ctas; }
 void fake_watch(const char *kernel, int arg, int n) { g_watch.push_back({kernel, arg, n}); }
 int fake_launched(const char *kernel) {
   int n = 0;
@@ -149,7 +153,10 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return *e = nul
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.0f, cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
+  *ms = !g_fast.empty() && g_last_kernel.find(g_fast) != std::string::npos && g_last_ctas <= g_fast_ctas ? 0.5f : 1.0f;
+  return cudaSuccess;
+}
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { return *g = nullptr, cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long long) {
@@ -178,6 +185,8 @@ cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **args, size_t,
   if (!g.x || !g.y || !g.z || !b.x || b.x * b.y * b.z > 1024) return err(cudaErrorInvalidConfiguration);
   const std::string &name = g_name[f];
   g_count[name]++;
+  g_last_kernel = name;
+  g_last_ctas = g.x;
   for (const Watch &w : g_watch)
     if (name.find(w.kernel) != std::string::npos)
       for (int i = 0; i < w.n; i++) g_null += ((void **)args[w.arg])[i] == nullptr;
