@@ -271,9 +271,11 @@ int b200_set_dw_staged(int mode);
  * keeps the fastest and returns it. */
 int b200_set_block_order(int kind);
 /* Fix the launch variant of the even-odd SAP block kernel for the current
- * block size (the index of the autotuner's candidate list, 0..3), so that
- * separate runs use the same arithmetic; -1 lets the autotuner choose again
- * (no reference counterpart). */
+ * block size (the index of the autotuner's candidate list, 0..4), so that
+ * separate runs use the same arithmetic; -1 lets the autotuner choose again.
+ * 0 and 4 are refused for blocks of more than 512 and 640 sites; 1 to 3 stand
+ * for the variant of the largest blocks where their own is too small (no
+ * reference counterpart). */
 int b200_set_sap_variant(int variant);
 /* Block-shape autotuner (no reference counterpart).  For each candidate
  * SAP block shape cand[4 i .. 4 i + 3] (i < ncand) that fits the lattice,
@@ -322,8 +324,9 @@ int b200_pipeline_used(void);
 int b200_pipeline_plan(const int L[4], const int bs[4], const int *ipt, int *npieces, int *nslabs);
 int b200_graphs_cached(void);
 /* Launch variant of the SAP block kernel picked by the autotuner for the
- * current block size (prec 32, 16, or 12 for the 12-real links): index,
- * threads per block, time of one cycle's block sweeps in ms. */
+ * current block size and launches of one system (prec 32, 16, or 12 for the
+ * 12-real links): index, threads per block, time of one cycle's block sweeps
+ * in ms. */
 int b200_sap_tuning(int prec, int *variant, int *threads, float *ms);
 
 /* ------------------------------------------------------------- forces.h */

@@ -754,6 +754,7 @@ static const EoVariant kEo[] = {
     {1, 768, EO_KERNELS(1, 768, 1)}, {2, 320, EO_KERNELS(2, 320, 2)},
 };
 static const int kNEo = sizeof(kEo) / sizeof(kEo[0]);
+static const int kEoLarge = 2;   // the variant for every block that the shared memory holds
 
 static size_t eo_smem(int vbh) { return (size_t)(((vbh + 7) & ~7) + 8) * 2 * EO_SREC * sizeof(float4); }
 // threads of a variant, 0 if it does not fit the block size
@@ -993,6 +994,9 @@ int sap_set_variant(Ctx &c, int v) {
     for (auto &t : c.sap_tuned[mode]) t.vbh = 0;
     return 0;
   }
+  // numbers 1 to 3 have always been good for large blocks: where their own
+  // form is too small, they stand for the one with three sites per lane pair
+  if (v > 0 && v < 4 && !eo_threads(kEo[v], c.g.vbh)) v = kEoLarge;
   if (v >= kNEo || !eo_threads(kEo[v], c.g.vbh))
     return fail("sap: this launch variant does not fit the block size");
   cudaFuncSetAttribute(kEo[v].k[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, SAP_SMEM_MAX);

@@ -61,3 +61,31 @@ def test_choice_by_launch_size(qb, L, nr, many, graphs):
     qb.set_cuda_graphs(0)
     qb.set_cuda_graphs(graphs)
     assert run(nr) > 0
+
+
+# sites per parity of the blocks, variants that do not fit them
+REFUSED = [((4, 4, 4, 4), []), ((4, 4, 8, 4), []), ((4, 4, 6, 6), [0]), ((4, 8, 4, 6), [0, 4]), ((6, 6, 6, 6), [0, 4]),
+           ((8, 8, 4, 6), [0, 4])]
+
+
+@pytest.mark.parametrize("bs,refused", REFUSED, ids=["x".join(map(str, b)) for b, _ in REFUSED])
+def test_fixed_variants(qb, bs, refused):
+    """the numbers that were good for a block size are: 0 up to 256 sites per
+    parity, 1 to 3 for every size"""
+    L = tuple(2 * b for b in bs)
+    qb.geometry(L, bs, qb.even_first_ipt(L))
+    qb.set_parms(1.5, 0.0, 0)
+    qb.random_ud(0.3, 1)
+    qb.sw_term()
+    qb.set_sap_parms(bs, 1, 4, 2)
+    x = [qb.DevField(32) for _ in range(2)]
+    for v in range(5):
+        if v in refused:
+            with pytest.raises(qb.B200Error):
+                qb.set_sap_variant(v)
+            continue
+        qb.set_sap_variant(v)
+        qb.dev_sap(0.0, 1, 4, 1, *x)
+        assert qb.sap_tuning(12)[1] >= 32 * ((bs[0] * bs[1] * bs[2] * bs[3] // 2 + 47) // 48)
+    with pytest.raises(qb.B200Error):
+        qb.set_sap_variant(5)
