@@ -67,6 +67,49 @@ __device__ __forceinline__ void pair_load_sw(const void *m, int chunk, int half,
 __device__ __forceinline__ void pair_load_sw(const void *m, int chunk, int half, int s, int vbh, double (&a)[36]) {
   load_pauli_cs((const double2 *)m, chunk, half, s, vbh, a);
 }
+// the sums up, lo of a role's four hops of t around site (p, blk, si)
+template <class LP, int DD, typename R = typename LP::R, typename E = typename Prec<R>::E>
+__device__ __forceinline__ void role_hops(const Geom &g, const DDGeom &dg, const Site &x, int p, int blk, int si,
+                                          const EoRole &ro, const E *__restrict__ t, const void *__restrict__ u,
+                                          Pair3<R> &up, Pair3<R> &lo) {
+  const int vbh = g.vbh, chunk = p * g.nbl + blk;
+  // the two directions of the role: coordinates and blocks
+  const int ya = ro.role ? x.y[2] : x.y[0], yb = ro.role ? x.y[1] : x.y[3];
+  const int na = ro.role ? x.n[2] : x.n[0], nba = ro.role ? g.nb[2] : g.nb[0], bsta = ro.role ? g.bstr[2] : g.bstr[0];
+  const int nb = ro.role ? x.n[1] : x.n[3], nbb = ro.role ? g.nb[1] : g.nb[3], bstb = ro.role ? g.bstr[1] : 1;
+  auto fwd = [&](int y, int n, int nbk, int bstr, int bs, int str, int &c2, int &s2) {
+    const bool in = y + 1 < bs;
+    s2 = (in ? x.l + str : x.l - (bs - 1) * str) >> 1;
+    c2 = (1 - p) * g.nbl + blk + (in ? 0 : (n + 1 < nbk ? bstr : -(nbk - 1) * bstr));
+  };
+  auto bwd = [&](int y, int n, int nbk, int bstr, int bs, int str, int &c2, int &s2) {
+    const bool in = y > 0;
+    s2 = (in ? x.l - str : x.l + (bs - 1) * str) >> 1;
+    c2 = (1 - p) * g.nbl + blk + (in ? 0 : (n > 0 ? -bstr : (nbk - 1) * bstr));
+  };
+  // global time coordinate: the time links at x0 = N0-1 carry the boundary sign
+  const int x0 = (DD ? dg.x0off : 0) + x.n[0] * g.bs[0] + x.y[0], xlast = (DD ? dg.N0 : g.L[0]) - 1;
+  pair_zero(up);
+  pair_zero(lo);
+  int c2, s2;
+  if (DD && ro.role == 0 && na + 1 == nba && ya + 1 == ro.bsa) {
+    eo_face_fwd<LP>(dg.hup, face_sites(g), face_index_of(g, x.n, x.y), u, vbh, chunk, si, x0 == xlast, up, lo);
+  } else {
+    fwd(ya, na, nba, bsta, ro.bsa, ro.stra, c2, s2);
+    eo_field_hop<0, 0, LP>(ro, t, u, vbh, c2, s2, chunk, ro.mua, si, (R)ro.s, ro.role == 0 && x0 == xlast, up, lo);
+  }
+  if (DD && ro.role == 0 && na == 0 && ya == 0) {
+    eo_face_bwd(dg.hdn, face_sites(g), face_index_of(g, x.n, x.y), up, lo);
+  } else {
+    bwd(ya, na, nba, bsta, ro.bsa, ro.stra, c2, s2);
+    eo_field_hop<0, 1, LP>(ro, t, u, vbh, c2, s2, c2, ro.mua, s2, (R)-ro.s, ro.role == 0 && x0 == 0, up, lo);
+  }
+  fwd(yb, nb, nbb, bstb, ro.bsb, ro.strb, c2, s2);
+  eo_field_hop<1, 0, LP>(ro, t, u, vbh, c2, s2, chunk, ro.mub, si, (R)ro.t, false, up, lo);
+  bwd(yb, nb, nbb, bstb, ro.bsb, ro.strb, c2, s2);
+  eo_field_hop<1, 1, LP>(ro, t, u, vbh, c2, s2, c2, ro.mub, s2, (R)-ro.t, false, up, lo);
+}
+
 template <int OPS, int PAR, class LP, int DD, typename R = typename LP::R, typename E = typename Prec<R>::E>
 __device__ __forceinline__ void pair_body(const Geom &g, const DDGeom &dg, int w, const E *__restrict__ s,
                                           const E *__restrict__ t, E *r, const void *__restrict__ u,
@@ -88,42 +131,8 @@ __device__ __forceinline__ void pair_body(const Geom &g, const DDGeom &dg, int w
   const size_t own = ((size_t)chunk * 2 + ro.role) * Prec<R>::NP * vbh + si;   // this role's chirality of a field
   cpx<R> acc[6], h[6];
   if (OPS & (OP_HOP | OP_HOPSUB)) {
-    // the two directions of the role: coordinates and blocks
-    const int ya = ro.role ? x.y[2] : x.y[0], yb = ro.role ? x.y[1] : x.y[3];
-    const int na = ro.role ? x.n[2] : x.n[0], nba = ro.role ? g.nb[2] : g.nb[0], bsta = ro.role ? g.bstr[2] : g.bstr[0];
-    const int nb = ro.role ? x.n[1] : x.n[3], nbb = ro.role ? g.nb[1] : g.nb[3], bstb = ro.role ? g.bstr[1] : 1;
-    auto fwd = [&](int y, int n, int nbk, int bstr, int bs, int str, int &c2, int &s2) {
-      const bool in = y + 1 < bs;
-      s2 = (in ? x.l + str : x.l - (bs - 1) * str) >> 1;
-      c2 = (1 - p) * g.nbl + blk + (in ? 0 : (n + 1 < nbk ? bstr : -(nbk - 1) * bstr));
-    };
-    auto bwd = [&](int y, int n, int nbk, int bstr, int bs, int str, int &c2, int &s2) {
-      const bool in = y > 0;
-      s2 = (in ? x.l - str : x.l + (bs - 1) * str) >> 1;
-      c2 = (1 - p) * g.nbl + blk + (in ? 0 : (n > 0 ? -bstr : (nbk - 1) * bstr));
-    };
-    // global time coordinate: the time links at x0 = N0-1 carry the boundary sign
-    const int x0 = (DD ? dg.x0off : 0) + x.n[0] * g.bs[0] + x.y[0], xlast = (DD ? dg.N0 : g.L[0]) - 1;
     Pair3<R> up, lo;
-    pair_zero(up);
-    pair_zero(lo);
-    int c2, s2;
-    if (DD && ro.role == 0 && na + 1 == nba && ya + 1 == ro.bsa) {
-      eo_face_fwd<LP>(dg.hup, face_sites(g), face_index_of(g, x.n, x.y), u, vbh, chunk, si, x0 == xlast, up, lo);
-    } else {
-      fwd(ya, na, nba, bsta, ro.bsa, ro.stra, c2, s2);
-      eo_field_hop<0, 0, LP>(ro, t, u, vbh, c2, s2, chunk, ro.mua, si, (R)ro.s, ro.role == 0 && x0 == xlast, up, lo);
-    }
-    if (DD && ro.role == 0 && na == 0 && ya == 0) {
-      eo_face_bwd(dg.hdn, face_sites(g), face_index_of(g, x.n, x.y), up, lo);
-    } else {
-      bwd(ya, na, nba, bsta, ro.bsa, ro.stra, c2, s2);
-      eo_field_hop<0, 1, LP>(ro, t, u, vbh, c2, s2, c2, ro.mua, s2, (R)-ro.s, ro.role == 0 && x0 == 0, up, lo);
-    }
-    fwd(yb, nb, nbb, bstb, ro.bsb, ro.strb, c2, s2);
-    eo_field_hop<1, 0, LP>(ro, t, u, vbh, c2, s2, chunk, ro.mub, si, (R)ro.t, false, up, lo);
-    bwd(yb, nb, nbb, bstb, ro.bsb, ro.strb, c2, s2);
-    eo_field_hop<1, 1, LP>(ro, t, u, vbh, c2, s2, c2, ro.mub, s2, (R)-ro.t, false, up, lo);
+    role_hops<LP, DD>(g, dg, x, p, blk, si, ro, t, u, up, lo);
     if (DD) __syncwarp();
     eo_exchange(ro.role, up, lo, h);
 #pragma unroll
@@ -192,6 +201,63 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 3 : DW_MINB32)
   pair_body<OPS, PAR, LP, 1>(g, dg, pair_warp(blockIdx.x), s, t, r, u, sw, swinv, mu_e, mu_o, sched, (const E *)nullptr);
 }
 
+// Hops alone in FP32 (OP_HOP, or OP_HOPSUB | OP_ACC) with one lane per site,
+// which goes through the two roles one after the other: the same sums in the
+// same order as with two lanes.  Without SW matrices there is little to do per
+// byte, and what counts are the bytes that the gathers have in flight; a lane's
+// eight neighbours and links are twice those of a lane of a pair.  Dwoe with
+// 12-real links on 32^3x64 145 us with two lanes, 113 with one (its 288 bytes
+// per site take 92), on 48x24^3 with 6^4 blocks 51.7 and 41.9 us; Dweo 156 and
+// 135 us, 53.5 and 49.2 us; on 32^3x64 with 18-real links 158 and 137 us, 170 and
+// 161 us.
+template <int OPS, int PAR, class LP, int DD, typename R = typename LP::R, typename E = typename Prec<R>::E>
+__device__ __forceinline__ void site_body(const Geom &g, const DDGeom &dg, int n, const E *__restrict__ t, E *r,
+                                          const void *__restrict__ u, const int *__restrict__ sched) {
+  const int i = blockIdx.x * 128 + threadIdx.x, vbh = g.vbh;
+  if (i >= n) return;
+  int blk = i / vbh;
+  const int si = i - blk * vbh;
+  if (sched) blk = __ldg(sched + blk);
+  Site x;
+  site_decode(g, PAR, blk, si, x);
+  Pair3<R> up[2], lo[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) role_hops<LP, DD>(g, dg, x, PAR, blk, si, eo_role(g, k), t, u, up[k], lo[k]);
+  E *own = r + ((size_t)PAR * g.nbl + blk) * 2 * Prec<R>::NP * vbh + si;
+  const R sg = (OPS & OP_HOP) ? (R)-0.5 : (R)0.5;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    cpx<R> h[6];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const auto ar = k ? mk2(lo[1].re[c].y, lo[1].re[c].x) : up[0].re[c], br = k ? lo[0].re[c] : up[1].re[c];
+      const auto ai = k ? mk2(lo[1].im[c].y, lo[1].im[c].x) : up[0].im[c], bi = k ? lo[0].im[c] : up[1].im[c];
+      h[c] = mk<R>(fm(sg, ar.x + br.x, (R)0), fm(sg, ai.x + bi.x, (R)0));   // (no negative zeros, as in pair_body)
+      h[3 + c] = mk<R>(fm(sg, ar.y + br.y, (R)0), fm(sg, ai.y + bi.y, (R)0));
+    }
+    E *o = own + (size_t)k * Prec<R>::NP * vbh;
+    if (OPS & OP_ACC) {
+      cpx<R> v[6];
+      eo_load((const E *)o, vbh, v);
+#pragma unroll
+      for (int j = 0; j < 6; j++) h[j] = mk<R>(h[j].re + v[j].re, h[j].im + v[j].im);
+    }
+    eo_store(o, vbh, h);
+  }
+}
+template <int OPS, int PAR, class LP, int MINB, typename E = typename Prec<typename LP::R>::E>
+__global__ void __launch_bounds__(128, MINB)
+    dirac_site_kernel(Geom g, int n, const E *__restrict__ t, E *r, const void *__restrict__ u,
+                      const int *__restrict__ sched) {
+  site_body<OPS, PAR, LP, 0>(g, DDGeom{0, 0, nullptr, nullptr}, n, t, r, u, sched);
+}
+template <int OPS, int PAR, class LP, typename E = typename Prec<typename LP::R>::E>
+__global__ void __launch_bounds__(128, DW_MINB32)
+    dirac_site_dd_kernel(Geom g, DDGeom dg, int n, const E *__restrict__ t, E *r, const void *__restrict__ u,
+                         const int *__restrict__ sched) {
+  site_body<OPS, PAR, LP, 1>(g, dg, n, t, r, u, sched);
+}
+
 // Several systems of the batched solvers (SAP_MS at most): r_j = sub_j -
 // Dw(mu_j) s_j, FP32, in one launch whose CTAs of one tile of sites
 // are adjacent (CTA x: tile x / n, system x % n), so the links and SW
@@ -239,6 +305,22 @@ static void launch_pairs(const Ctx &c, const DDGeom *dg, const void *s, const vo
   const void *swinv = F64 ? (const void *)c.swd_inv : (const void *)c.sw32_inv;
   const E *es = (const E *)s, *et = (const E *)t, *eb = (const E *)sub;
   E *er = (E *)r;
+  if constexpr (!F64 && !(OPS & (OP_SW | OP_INV))) {
+    // hops alone: one lane per site, unless that leaves half of the warp slots
+    // empty (8^4: 6.2 us with one lane, 4.2 with two; 16^4: 6.2 and 6.2 to 6.9).
+    // CTAs per SM: Dwoe 4 (3 are 8 % slower on 32^3x64, 5 are 5 %).  Dweo,
+    // which reads its output too, 3 with 18-real links (161 us on 32^3x64; 4:
+    // 168), with 12-real ones 5 (135 us; 4: 137, 3: 143), or 3 if the launch is
+    // one wave then (16^4: 6.2 us; 4: 7.2, 5: 8.2)
+    const int n = nblk * c.g.vbh, ns = (n + 127) / 128;
+    if (nb > 2 * 148) {
+      constexpr int MINB = OPS & OP_ACC ? (LP::NRAW == 12 ? 5 : 3) : 4;
+      if (dg) dirac_site_dd_kernel<OPS, PAR, LP><<<ns, 128, 0, st>>>(c.g, *dg, n, et, er, u, sched);
+      else if (ns > 3 * 148) dirac_site_kernel<OPS, PAR, LP, MINB><<<ns, 128, 0, st>>>(c.g, n, et, er, u, sched);
+      else dirac_site_kernel<OPS, PAR, LP, MINB == 5 ? 3 : MINB><<<ns, 128, 0, st>>>(c.g, n, et, er, u, sched);
+      return;
+    }
+  }
   if constexpr (!(OPS & OP_SUB)) {
     if (dg) {
       dirac_pair_dd_kernel<OPS, PAR, LP><<<nb, 128, 0, st>>>(c.g, *dg, es, et, er, u, sw, swinv, mu_e, mu_o, sched);

@@ -1,7 +1,8 @@
 """The FP32 operators with two lanes per site on blocks whose sites do not
 fill a warp's 16 pairs, with 12-real and 18-real links: every operator, the
 residual-update form, and the host pipeline's block lists, against the CPU
-restatement (oracle/qcd_oracle.c, modules/dirac/Dw.c:973)."""
+restatement (oracle/qcd_oracle.c, modules/dirac/Dw.c:973).  Dwoe and Dweo on
+lattices with one lane per site in their two forms."""
 import numpy as np
 import pytest
 
@@ -48,5 +49,37 @@ def test_fp32_operators(L, bs, eoflg):
             assert np.array_equal(np.array(hr.a), qb.dirac_ref("Dw", 32, MU, s))
             hs.free()
             hr.free()
+    finally:
+        qb.set_sap_link12(1)
+
+
+# up to 444 CTAs of one lane per site, and more
+@pytest.mark.parametrize("L,bs", [((16, 12, 16, 12), (4, 6, 4, 6)), ((24, 24, 24, 12), (6, 6, 6, 6))],
+                         ids=["4x6x4x6", "6x6x6x6"])
+def test_fp32_hops_large(L, bs):
+    ipt = qb.even_first_ipt(L)
+    V = ipt.size
+    qb.geometry(L, bs, ipt)
+    qb.set_parms(1.5, 0.0, 0)
+    qb.random_ud(0.4, 99)
+    assert qb.sw_term() == 0
+    U = O.links_ref2lex(qb.download_ud(V), ipt, L)
+    sw = O.pauli_ref2lex(qb.download_swd(V), ipt)
+    g = np.random.default_rng(3)
+    s, r0 = (g.standard_normal(24 * V).astype(np.float32) for _ in range(2))
+    try:
+        for op in ("Dwoe", "Dweo"):
+            ref = O.spinor_lex2ref(O.dirac(L, OPS.index(op), MU, 0, U, sw, sw, O.spinor_ref2lex(s, ipt),
+                                           O.spinor_ref2lex(r0, ipt)), ipt)
+            for l12 in (1, 0):
+                qb.set_sap_link12(l12)
+                assert site_rel_err(qb.dirac_ref(op, 32, MU, s, r0), ref, V) <= TOL, (op, l12)
+        # the operator as a whole, which has two lanes per site, in its pieces
+        qb.set_sap_link12(1)
+        z = np.zeros_like(s)
+        even = qb.dirac_ref("Dweo", 32, MU, -s, qb.dirac_ref("Dwee", 32, MU, s, z))
+        odd = qb.dirac_ref("Dwoo", 32, MU, s, z) + qb.dirac_ref("Dwoe", 32, MU, s, z)
+        h = 12 * V
+        assert site_rel_err(np.concatenate([even[:h], odd[h:]]), qb.dirac_ref("Dw", 32, MU, s), V) <= TOL
     finally:
         qb.set_sap_link12(1)
