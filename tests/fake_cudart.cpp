@@ -14,6 +14,7 @@ namespace {
 struct Watch {
   std::string kernel;
   int arg, n;   // n pointers from the start of argument arg
+  size_t room;  // bytes that have to be left in their allocations
 };
 std::map<char *, size_t> g_mem;        // live allocations, device and page-locked
 std::map<char *, size_t> g_dev;        // the device ones
@@ -22,7 +23,7 @@ std::map<std::string, int> g_count;    // launches by kernel
 std::string g_fast, g_last_kernel;
 int g_fast_ctas, g_last_ctas;
 std::vector<Watch> g_watch;
-int g_allocs, g_fail_at, g_legacy, g_null, g_launches, g_bad_frees;
+int g_allocs, g_fail_at, g_legacy, g_null, g_launches, g_bad_frees, g_short;
 cudaError_t g_last;
 
 cudaError_t err(cudaError_t e) {
@@ -75,7 +76,10 @@ int fake_legacy() { return g_legacy; }
 int fake_launches() { return g_launches; }
 // the times that events measure: half as long after a launch of this kernel with up to so many CTAs
 void fake_fast(const char *kernel, int ctas) { g_fast = kernel, g_fast_ctas = ctas; }
-void fake_watch(const char *kernel, int arg, int n) { g_watch.push_back({kernel, arg, n}); }
+void fake_watch(const char *kernel, int arg, int n) { g_watch.push_back({kernel, arg, n, 0}); }
+void fake_watch_room(const char *kernel, int arg, size_t room) { g_watch.push_back({kernel, arg, 1, room}); }
+void fake_unwatch() { g_watch.clear(); }
+int fake_short_args() { return g_short; }
 int fake_launched(const char *kernel) {
   int n = 0;
   for (const auto &k : g_count)
@@ -189,7 +193,11 @@ cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **args, size_t,
   g_last_ctas = g.x;
   for (const Watch &w : g_watch)
     if (name.find(w.kernel) != std::string::npos)
-      for (int i = 0; i < w.n; i++) g_null += ((void **)args[w.arg])[i] == nullptr;
+      for (int i = 0; i < w.n; i++) {
+        const void *p = ((void **)args[w.arg])[i];
+        g_null += p == nullptr;
+        g_short += room(p) < w.room;
+      }
   return cudaSuccess;
 }
 void **__cudaRegisterFatBinary(void *) {

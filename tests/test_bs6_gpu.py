@@ -41,24 +41,6 @@ def test_dirac_dble(setup, op):
     assert site_rel_err(out, ref, setup.vol) <= 1e-13
 
 
-@pytest.mark.parametrize("op", OPS)
-def test_staged_equals_direct(setup, op):
-    """The FP64 operators with bulk-staged SW matrices (648-site chunks:
-    five tiles of 128 sites and a partial one) against the direct-read
-    kernel: the same arithmetic."""
-    s = setup.source(13)
-    r0 = setup.source(14)
-    prev = qb.set_dw_staged(0)
-    try:
-        out = []
-        for mode in (0, 1):
-            qb.set_dw_staged(mode)
-            out.append(qb.dirac_ref(op, 64, 0.137, s, r0))
-    finally:
-        qb.set_dw_staged(prev)
-    assert site_rel_err(out[1], out[0], setup.vol) <= 1e-15
-
-
 @pytest.mark.parametrize("op", ["Dw", "Dwhat"])
 def test_dirac_fp32(setup, op):
     s = setup.source(23).astype(np.float32)

@@ -44,18 +44,6 @@ def test_c2_dw_dble(c2, mu):
     assert err <= TOL64, "Dw_dble mu=%g on 32^3x64: per-site rel err %.3e" % (mu, err)
 
 
-def test_c2_dw_dble_unstaged(c2):
-    """the direct-read FP64 kernel (SW matrices not staged) on the same case"""
-    s = c2.source(102)
-    r_ref = c2.ref.dirac_dble(0, 0.0, s)
-    prev = qb.set_dw_staged(0)
-    try:
-        r_dev = qb.dirac_ref("Dw", 64, 0.0, s)
-    finally:
-        qb.set_dw_staged(prev)
-    assert site_rel_err(r_dev, r_ref, c2.vol) <= TOL64
-
-
 def test_c2_dwhat_dble(c2):
     s = c2.source(103)
     r0 = c2.source(104)

@@ -2,6 +2,8 @@
 stand-in for the CUDA runtime that lets a chosen allocation fail: the call
 reports it, leaves nothing half made, and the next call starts afresh, without
 a null pointer among its kernels' arguments."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -151,3 +153,37 @@ def test_subspace_generation_restores_the_mass():
                 qb.sw_term()
     total, seen = _every_failure(prepare, call, [])
     assert seen == total >= 20
+
+
+def test_larger_lattice_after_smaller():
+    """what a call keeps is sized anew with the geometry: fields in copies,
+    conversions, block solves and updates hold the new lattice"""
+    qb = hostlib.load()
+    qb.lib().fake_watch_room.argtypes = [C.c_char_p, C.c_int, C.c_size_t]
+    for L in ((8, 8, 8, 8), (16, 8, 8, 8)):
+        V = int(np.prod(L))
+        qb.geometry(L, BS, qb.even_first_ipt(L))
+        qb.lib().fake_unwatch()
+        for kernel, args, site in ((b"k_copy_dd", (1, 2), 192), (b"k_copy_ff", (1, 2), 96), (b"k_sap_out", (1, 2, 3), 96),
+                                   (b"k_fupd", (0, 1), 96), (b"k_scale_d", (1,), 192)):
+            for a in args:
+                qb.lib().fake_watch_room(kernel, a, V * site)
+        qb.set_parms(1.5, 0.0, 0)
+        qb.random_ud(0.3, 1)
+        qb.sw_term()
+        qb.set_sap_parms(BS, 1, 4, 2)
+        s = np.ones(24 * V)
+        qb.dirac_ref("Dwhat", 64, 0.1, s)
+        qb.sap_ref(0.1, 1, 4, s.astype(np.float32), s.astype(np.float32))
+        qb.sap_gcr(2, 2, 0, 1e-10, 0.0, s)
+        qb.tmcg(128, 0, 1e-8, 0.1, s)
+        nv = qb.set_dfl_parms(BS, NS)
+        qb.set_dfl_pro_parms(2, 2, 1e-2, 2, 1e-2)
+        for l in range(NS):
+            qb.dfl_set_basis(l, np.ones(24 * V, np.float32))
+        qb.dfl_s2vd_multi([s.astype(np.float32)] * 3, nv)
+        E, P = ([qb.DevField(64) for _ in range(3)] for _ in range(2))
+        for dfl in (False, True):
+            qb.dev_gcr_batch(2, 2, 0, 1e-10, [0.0] * 3, E, P, dfl=dfl)
+        assert qb.lib().b200_last_error() == b"" and qb.lib().fake_bad_frees() == 0
+        assert qb.lib().fake_short_args() == 0

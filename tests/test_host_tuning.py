@@ -20,7 +20,8 @@ def qb():
 
 
 def _batch(qb, L, nr):
-    """launches of the 255-register variant by a first and a second batch"""
+    """a function that runs a batch of n systems and returns its launches of the
+    variant above, after a first batch of nr"""
     qb.geometry(L, BS, qb.even_first_ipt(L))
     qb.set_parms(1.5, 0.0, 0)
     qb.random_ud(0.3, 1)

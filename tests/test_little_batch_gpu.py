@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("L,ns,nkv,res", [((8, 8, 8, 8), 2, 2, 1e-1), ((8, 8, 8, 8), 8, 16, 1e-6),
-                                          ((16, 8, 8, 8), 20, 32, 1e-6)])
+                                          ((16, 8, 8, 8), 20, 32, 1e-9)])
 def test_little_sums(L, ns, nkv, res):
     bs = (4, 4, 4, 4)
     ipt = qb.even_first_ipt(L)

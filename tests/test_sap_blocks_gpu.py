@@ -37,21 +37,21 @@ def test_sap_blocks(L, bs):
     psi, rho = np.zeros_like(eta), O.spinor_ref2lex(eta, ipt)
     for _ in range(2):
         psi, rho = O.sap(L, bs, MU, 1, 3, 0, U, sw[0], sw[1], psi, rho)
-    tried = 0
+    half = int(np.prod(bs)) // 2
+    refused = [v for v, most in ((0, 256), (4, 320)) if half > most] + [5]
     try:
         for l12 in (1, 0):
             qb.set_sap_link12(l12)
-            for v in range(-1, 8):
-                try:
-                    qb.set_sap_variant(v)
-                except qb.B200Error:
+            for v in range(-1, 6):
+                if v in refused:
+                    with pytest.raises(qb.B200Error):
+                        qb.set_sap_variant(v)
                     continue
+                qb.set_sap_variant(v)
                 p, r = qb.DevField(32), qb.DevField(32).from_ref(eta)
                 qb.dev_sap(MU, 1, 3, 2, p, r)
                 for x, y in ((p, psi), (r, rho)):
                     d = O.spinor_ref2lex(x.to_ref(V), ipt)
                     assert np.linalg.norm(d - y) <= TOL * np.linalg.norm(y), (l12, v)
-                tried += 1
     finally:
         qb.set_sap_link12(1)
-    assert tried >= 4
