@@ -27,23 +27,17 @@ namespace qcd {
 
 enum { OP_SW = 1, OP_HOP = 2, OP_HOPSUB = 4, OP_INV = 8, OP_ACC = 16, OP_SUB = 32 };
 
-// L2 residency: the SW matrices are read once per application and the
+// L2 residency in FP64: the SW matrices are read once per application and the
 // output is not read back by the launch, so both go through L2 with the
-// evict-first policy (ld.global.cs / st.global.cs, or a cache hint on the
-// bulk copies).  The neighbour spinors and links, read by several CTAs at
-// different times (block faces), then stay in L2 longer.
-#ifndef DW_NO_HINTS
-#define DW_HINTS 1
-#else
-#define DW_HINTS 0
-#endif
-
+// evict-first policy (ld.global.cs, and st.global.cs in eo_store).  The
+// neighbour spinors and links, read by several CTAs at different times (block
+// faces), then stay in L2 longer.  FP32 reads and writes with the default policy.
 __device__ __forceinline__ void load_pauli_cs(const double2 *base, int chunk, int half, int s, int vbh,
                                               double u[36]) {
   const double2 *p = base + ((size_t)chunk * 36 + 18 * half) * vbh + s;
 #pragma unroll
   for (int k = 0; k < 18; k++) {
-    const double2 v = DW_HINTS ? __ldcs(p + (size_t)k * vbh) : __ldg(p + (size_t)k * vbh);
+    const double2 v = __ldcs(p + (size_t)k * vbh);
     u[2 * k] = v.x;
     u[2 * k + 1] = v.y;
   }
@@ -58,9 +52,7 @@ __device__ __forceinline__ void load_pauli_cs(const double2 *base, int chunk, in
 // TB/s of the 672 algorithmic bytes per site), on 48x24^3 with 6^4 blocks 107.6
 // -> 94.5 us, on 8^4 8.2 -> 4.1 us; five CTAs per SM (96 registers) 312 and
 // 98.8 us, six (80) 294 and 94.3 us.
-#ifndef DW_MINB32
-#define DW_MINB32 4
-#endif
+constexpr int DW_MINB32 = 4;
 __device__ __forceinline__ void pair_load_sw(const void *m, int chunk, int half, int s, int vbh, float (&a)[36]) {
   Store<float>::load_pauli(m, chunk, half, s, vbh, a);
 }
@@ -182,9 +174,13 @@ static unsigned pair_grid(const Geom &g, int par, int nblk) {
 }
 __device__ __forceinline__ int pair_warp(int cta) { return cta * 4 + (threadIdx.x >> 5); }
 
-// CTAs per SM: FP32 4 of 128 registers (see above); FP64 3 of 168, which ran
-// faster than 2 of 255 (664 against 636 us for Dw on 32^3x64) and than 4 of 128
-// (672 us), unless the launch fits the chip in one wave of 4 and not of 3.
+// CTAs per SM: FP32 4 of 128 registers (see above); FP64 with hops 3 of 168,
+// which run faster than 2 of up to 226 (620 against 696 us for Dw on 32^3x64,
+// 42.8 and 46.9 us on 32x16^3) and than 4 of 128 (666 and 46.1 us), unless the
+// launch fits the chip in one wave of 4 and not of 3: Dwhat on 16^4 (512 CTAs)
+// 26.6 us with 3, 24.6 with 4, on 24^2x16x8 (576) 28.7 and 25.3 us; beyond that
+// wave, on 32x16^3 (1024), 56.3 and 57.9 us.  Without hops the kernel has 120
+// registers anyway.
 template <int OPS, int PAR, class LP, int MINB, typename R = typename LP::R, typename E = typename Prec<R>::E>
 __global__ void __launch_bounds__(128, MINB)
     dirac_pair_kernel(Geom g, const E *__restrict__ s, const E *__restrict__ t, E *r, const void *__restrict__ u,
@@ -327,19 +323,19 @@ static void launch_pairs(const Ctx &c, const DDGeom *dg, const void *s, const vo
       return;
     }
   }
-  if (!F64 || (nb > 3 * 148 && nb <= 4 * 148))
-    dirac_pair_kernel<OPS, PAR, LP, DW_MINB32><<<nb, 128, 0, st>>>(c.g, es, et, er, u, sw, swinv, mu_e, mu_o, sched, eb);
-  else
-    dirac_pair_kernel<OPS, PAR, LP, F64 ? 3 : DW_MINB32><<<nb, 128, 0, st>>>(c.g, es, et, er, u, sw, swinv, mu_e, mu_o,
-                                                                            sched, eb);
+  if constexpr (F64 && (OPS & (OP_HOP | OP_HOPSUB))) {
+    if (nb <= 3 * 148 || nb > 4 * 148) {
+      dirac_pair_kernel<OPS, PAR, LP, 3><<<nb, 128, 0, st>>>(c.g, es, et, er, u, sw, swinv, mu_e, mu_o, sched, eb);
+      return;
+    }
+  }
+  dirac_pair_kernel<OPS, PAR, LP, 4><<<nb, 128, 0, st>>>(c.g, es, et, er, u, sw, swinv, mu_e, mu_o, sched, eb);
 }
 
 // With domain decomposition the operators that hop (all but Dwee, Dwoo)
 // first exchange the x0-faces of the field they hop on.
 template <typename R, int OPS, int PAR>
-static void launch(const Ctx &c, const void *s, const void *t, void *r, R mu_e, R mu_o, bool inv,
-                   cudaStream_t st) {
-  (void)inv;
+static void launch(const Ctx &c, const void *s, const void *t, void *r, R mu_e, R mu_o, cudaStream_t st) {
   constexpr bool HOPS = (OPS & (OP_HOP | OP_HOPSUB)) != 0;
   const void *u = sizeof(R) == 8 ? (const void *)c.ud : (const void *)c.u32;
   const void *u12 = nullptr;
@@ -362,14 +358,14 @@ template <typename R>
 int dirac_op(const Ctx &c, int op, R mu, const void *s, void *r, void *tmp, cudaStream_t st) {
   R muo = c.eoflg ? (R)0 : mu;
   switch (op) {
-    case 0: launch<R, OP_SW | OP_HOP, 2>(c, s, s, r, mu, muo, false, st); break;
-    case 1: launch<R, OP_SW, 0>(c, s, s, r, mu, mu, false, st); break;
-    case 2: launch<R, OP_SW, 1>(c, s, s, r, muo, muo, false, st); break;
-    case 3: launch<R, OP_HOP, 1>(c, s, s, r, mu, mu, false, st); break;
-    case 4: launch<R, OP_HOPSUB | OP_ACC, 0>(c, s, s, r, mu, mu, false, st); break;
+    case 0: launch<R, OP_SW | OP_HOP, 2>(c, s, s, r, mu, muo, st); break;
+    case 1: launch<R, OP_SW, 0>(c, s, s, r, mu, mu, st); break;
+    case 2: launch<R, OP_SW, 1>(c, s, s, r, muo, muo, st); break;
+    case 3: launch<R, OP_HOP, 1>(c, s, s, r, mu, mu, st); break;
+    case 4: launch<R, OP_HOPSUB | OP_ACC, 0>(c, s, s, r, mu, mu, st); break;
     case 5:
-      launch<R, OP_HOP | OP_INV, 1>(c, s, s, tmp, (R)0, (R)0, true, st);
-      launch<R, OP_SW | OP_HOPSUB, 0>(c, s, tmp, r, mu, mu, false, st);
+      launch<R, OP_HOP | OP_INV, 1>(c, s, s, tmp, (R)0, (R)0, st);
+      launch<R, OP_SW | OP_HOPSUB, 0>(c, s, tmp, r, mu, mu, st);
       break;
     default: return -1;
   }

@@ -189,8 +189,9 @@ struct Ctx {
   double2 *gcr_rec = nullptr, *h_gcr_rec = nullptr;   // products of a GCR step, device and page-locked
   int gcr_n = 0;
   cudaStream_t stream = nullptr;
-  // error flag of bounded waits in the operator kernels: page-locked host
-  // memory mapped into the device (h_kerr host view, d_kerr device view)
+  // error flag of bounded waits that b200_sync reports: page-locked host memory
+  // mapped into the device (h_kerr host view, d_kerr device view).  Set by the
+  // self-check's kernel; the batched deflation kernels have their own (dfl.kerr)
   int *h_kerr = nullptr, *d_kerr = nullptr;
   int dw_staged = 1;            // b200_set_dw_staged's mode (without effect)
   // repeated launch sequences (the SAP preconditioner) run as CUDA graphs,

@@ -242,7 +242,8 @@ __device__ __forceinline__ void eo_load(const double2 *f, int vbh, cpx<double> (
     v[j] = mk<double>(q.x, q.y);
   }
 }
-// (evict first: the operators' output is not read back by the launch)
+// (evict first: the operators' output is not read back by the launch; Dwhat's
+// odd intermediate, which its second launch reads, goes the same way)
 __device__ __forceinline__ void eo_store(double2 *f, int vbh, const cpx<double> (&v)[6]) {
 #pragma unroll
   for (int j = 0; j < 6; j++) __stcs(f + (size_t)j * vbh, make_double2(v[j].re, v[j].im));

@@ -36,12 +36,10 @@ namespace qcd {
 struct SapArgs {
   Geom g;
   int colour;
-  float mu;             // system 0
   int nmr;
   int eoflg;
   float4 *psi[SAP_MS], *rho[SAP_MS], *phi[SAP_MS];
-  const void *u;        // links as the block solver's policy reads them
-  const void *ub;       // links for the block-boundary hops (as u, but 18-real FP32 in the FP32 mode)
+  const void *u;        // links, as the storage mode's policy reads them
   const void *sw, *swinv;
   int nsys;
   float mus[SAP_MS];
@@ -90,7 +88,6 @@ __device__ __forceinline__ int block_of_colour(const Geom &g, int h, int colour)
 // and cost half as many GCR iterations again.)
 struct SapF32 {
   using T = float;
-  static constexpr int NP = 24;
   __device__ __forceinline__ static spinor<float> sm_load(const float *sm, int ld, int s) {
     const float4 *p = reinterpret_cast<const float4 *>(sm);
     spinor<float> r;
@@ -200,16 +197,17 @@ __device__ __forceinline__ void block_allreduce3(double (&v)[3], double *red) {
 // ------------------------------------------------------------------------
 // The even-odd block solver, two lanes per site (pairs.cuh).  In shared
 // memory a site's spinor is 9 float4 (144 bytes, free of bank conflicts for 8
-// consecutive sites): for each colour k the pairs (c1 c2), (c3 c4) and
+// consecutive sites; with 6^4 blocks, whose rows have three sites, a quarter of
+// the load wavefronts are conflicts): for each colour k the pairs (c1 c2), (c3 c4) and
 // (c4 c3), real parts then imaginary parts; the swapped copy lets both roles
 // load their lower components in the order of their projector.
 //
-// What bounds it: the shared-memory and L1 data path (half busy) and the
-// latency of the link and SW reads, at 8 to 16 warps per SM; HBM is far from
-// busy.  Against one thread per site (the form this replaces) a block of 4^4
+// What bounds it: the shared-memory and L1 data path (52 % busy with 4^4 blocks
+// on 32^4, 41 % with 6^4 blocks on 48x24^3; issue 52 and 37 %) and the latency of
+// the link and SW reads, at 8 to 16 warps per SM; HBM is far from busy.  Against one thread per site (the form this replaces) a block of 4^4
 // has 8 warps instead of 4 and each works through half the chain.  One cycle
 // (nmr = 4: two launches each of this and the boundary kernel): 8^4 lattice 120
-// -> 70 us, 16^4 126 -> 78 us, 32^4 841 -> 760 us (4^4 blocks); 48x24^3 (6^4
+// -> 66 us, 16^4 126 -> 70 us, 32^4 841 -> 760 us (4^4 blocks); 48x24^3 (6^4
 // blocks) 701 -> 664 us.  Tried and dropped: the links of the block copied into
 // shared memory at the start (their reads compete with the spinors' for the
 // same data path: 90.8 against 81.2 us on 8^4); the two half spinors as packed
@@ -359,10 +357,10 @@ __device__ __forceinline__ bool eo_cross(const SapArgs &a, const DDGeom &dg, con
   int c2, s2;
   if (fa) {
     if (DD && ro.role == 0 && na + 1 == nba) {
-      eo_face_fwd<LP>(dg.hup, face_sites(g), face_index_of(g, x.n, x.y), a.ub, g.vbh, chunk, s, x0 == xlast, up, lo);
+      eo_face_fwd<LP>(dg.hup, face_sites(g), face_index_of(g, x.n, x.y), a.u, g.vbh, chunk, s, x0 == xlast, up, lo);
     } else {
       across(na, nba, bsta, ro.bsa, ro.stra, +1, c2, s2);
-      eo_field_hop<0, 0, LP>(ro, phi, a.ub, g.vbh, c2, s2, chunk, ro.mua, s, ro.s, ro.role == 0 && x0 == xlast, up, lo);
+      eo_field_hop<0, 0, LP>(ro, phi, a.u, g.vbh, c2, s2, chunk, ro.mua, s, ro.s, ro.role == 0 && x0 == xlast, up, lo);
     }
   }
   if (ba) {
@@ -370,16 +368,16 @@ __device__ __forceinline__ bool eo_cross(const SapArgs &a, const DDGeom &dg, con
       eo_face_bwd(dg.hdn, face_sites(g), face_index_of(g, x.n, x.y), up, lo);
     } else {
       across(na, nba, bsta, ro.bsa, ro.stra, -1, c2, s2);
-      eo_field_hop<0, 1, LP>(ro, phi, a.ub, g.vbh, c2, s2, c2, ro.mua, s2, -ro.s, ro.role == 0 && x0 == 0, up, lo);
+      eo_field_hop<0, 1, LP>(ro, phi, a.u, g.vbh, c2, s2, c2, ro.mua, s2, -ro.s, ro.role == 0 && x0 == 0, up, lo);
     }
   }
   if (fb) {
     across(nb_, nbb, bstb, ro.bsb, ro.strb, +1, c2, s2);
-    eo_field_hop<1, 0, LP>(ro, phi, a.ub, g.vbh, c2, s2, chunk, ro.mub, s, ro.t, false, up, lo);
+    eo_field_hop<1, 0, LP>(ro, phi, a.u, g.vbh, c2, s2, chunk, ro.mub, s, ro.t, false, up, lo);
   }
   if (bb) {
     across(nb_, nbb, bstb, ro.bsb, ro.strb, -1, c2, s2);
-    eo_field_hop<1, 1, LP>(ro, phi, a.ub, g.vbh, c2, s2, c2, ro.mub, s2, -ro.t, false, up, lo);
+    eo_field_hop<1, 1, LP>(ro, phi, a.u, g.vbh, c2, s2, c2, ro.mub, s2, -ro.t, false, up, lo);
   }
   __syncwarp();
   eo_exchange(ro.role, up, lo, o);
@@ -690,7 +688,7 @@ __global__ void k_sap_dd_pack(SapArgs a, DDGeom dg, void *dn, void *up) {
   face_site(g, side, f, chunk, s, n, y);
   const spinor<float> v = Store<float>::load_spinor(a.phi[0], chunk, s, g.vbh);
   vec3<float> h0, h1;
-  eo_face_send<LP>(side, v, a.ub, g.vbh, chunk, s, dg.x0off + g.L[0] - 1 == dg.N0 - 1, h0, h1);
+  eo_face_send<LP>(side, v, a.u, g.vbh, chunk, s, dg.x0off + g.L[0] - 1 == dg.N0 - 1, h0, h1);
   Half<float>::store(side == 0 ? dn : up, F, f, h0, h1);
 }
 
@@ -734,7 +732,7 @@ static int pick_threads(int vbh, int &ns) {
 // Which one wins, in us per cycle of four MR steps:
 //   ns maxt (registers)   8^4, 4^4 blocks  32^4, 4^4  4x4x6x4   48x24^3, 6^4  8x4x6x8
 //   1   512 (128)               72            769        -              -             -
-//   1   256 (255)               66            958        -              -             -
+//   1   256 (230)               66            958        -              -             -
 //   3   512 (128)              130            987        -             666           364
 //   1   768 (80)                80            797       132            -             -
 //   2   320 (96, two CTAs/SM)  111            941       379            -             -
@@ -864,7 +862,7 @@ static int sap_mode(Ctx &c, int isolv, cudaStream_t st) {
 
 // The choice for launches of nsys systems.  One CTA per SM at most, or more:
 // with several systems the first can become the second, and the variant that
-// wins one (one CTA of 255 registers per SM) loses the other: six GCR steps of
+// wins one (one CTA of 230 registers per lane on an SM) loses the other: six GCR steps of
 // four systems on 16^4 with 4^4 blocks 9.24 ms with the one-system choice,
 // 8.11 ms with its own; on 24^2x16x8 with 4x6x8x4 blocks 11.77 and 10.61 ms.
 static Ctx::SapTuned &sap_tuned(Ctx &c, int mode, int nsys) { return c.sap_tuned[mode][c.g.nbl / 2 * nsys > 148]; }
@@ -894,7 +892,6 @@ static SapArgs sap_args(Ctx &c, float mu, int nmr, int mode, void *psi, void *rh
   const bool half = mode == 1;
   a.g = c.g;
   a.colour = 0;
-  a.mu = mu;
   a.nmr = nmr;
   a.eoflg = c.eoflg;
   a.psi[0] = (float4 *)psi;
@@ -903,7 +900,6 @@ static SapArgs sap_args(Ctx &c, float mu, int nmr, int mode, void *psi, void *rh
   a.nsys = 1;
   a.mus[0] = mu;
   a.u = half ? (const void *)c.u16 : (mode == 2 ? (const void *)c.u12 : (const void *)c.u32);
-  a.ub = half ? (const void *)c.u16 : (mode == 2 ? (const void *)c.u12 : (const void *)c.u32);
   a.sw = half ? (const void *)c.sw16 : (const void *)c.sw32;
   a.swinv = half ? (const void *)c.sw16_inv : (const void *)c.sw32_inv;
   return a;

@@ -1,5 +1,6 @@
-// Self-check of the bounded-wait path that the bulk-copy kernels rely on
-// (b200_selfcheck_bounded_wait, no counterpart in the reference).
+// Self-check of a bounded wait on bulk copies, of the kind the batched
+// deflation kernels have, that runs out (b200_selfcheck_bounded_wait, no
+// counterpart in the reference).
 //
 // One CTA arms an mbarrier that no copy and no thread will ever complete and
 // waits on it with a caller-given iteration limit.  The wait gives up,
