@@ -608,7 +608,7 @@ def sustained_dw(qb, n, chunk=20):
 
 def scan_block_orders(qb):
     """Dw_dble on 32^3x64 under each block traversal order: first two
-    launches per order (the launches a 10-launch ncu capture of
+    launches per order (the launches that a 10-launch ncu capture of the
     Dw_dble kernel sees), then 3 x 20 timed launches per order."""
     L = LATTICE
     qb.geometry(L, BS, qb.even_first_ipt(L))

@@ -197,13 +197,14 @@ __device__ __forceinline__ void block_allreduce3(double (&v)[3], double *red) {
 // ------------------------------------------------------------------------
 // The even-odd block solver, two lanes per site (pairs.cuh).  In shared
 // memory a site's spinor is 9 float4 (144 bytes, free of bank conflicts for 8
-// consecutive sites; with 6^4 blocks, whose rows have three sites, a quarter of
-// the load wavefronts are conflicts): for each colour k the pairs (c1 c2), (c3 c4) and
-// (c4 c3), real parts then imaginary parts; the swapped copy lets both roles
-// load their lower components in the order of their projector.
+// consecutive sites; neighbours' rows are shorter, and a fifth of the load
+// wavefronts are conflicts with 4^4 and with 6^4 blocks): for each colour k the
+// pairs (c1 c2), (c3 c4) and (c4 c3), real parts then imaginary parts; the
+// swapped copy lets both roles load their lower components in the order of
+// their projector.
 //
 // What bounds it: the shared-memory and L1 data path (52 % busy with 4^4 blocks
-// on 32^4, 41 % with 6^4 blocks on 48x24^3; issue 52 and 37 %) and the latency of
+// on 32^4, 39 % with 6^4 blocks on 48x24^3; issue 55 and 45 %) and the latency of
 // the link and SW reads, at 8 to 16 warps per SM; HBM is far from busy.  Against one thread per site (the form this replaces) a block of 4^4
 // has 8 warps instead of 4 and each works through half the chain.  One cycle
 // (nmr = 4: two launches each of this and the boundary kernel): 8^4 lattice 120
