@@ -1,9 +1,11 @@
 """The part of reflib.RefLib's interface that the CPU restatement
 (oracle/qcd_oracle.c) covers, for machines without the reference's sources:
-gauge fields and SW term, the Dirac operators, SAP cycles and sap_gcr.  The
-fields are its own (numpy's generators), drawn with the reference's
-distributions; everything else goes through missing().  Test infrastructure
-only."""
+gauge fields and SW term, the Dirac operators, SAP cycles and sap_gcr, and on
+top of them, in numpy, the deflation: block basis, restriction and
+prolongation, the little operators as dense matrices, and the deflated
+solver.  The fields are its own (numpy's generators), drawn with the
+reference's distributions; everything else goes through missing().  Test
+infrastructure only."""
 import numpy as np
 
 import oracle as O
@@ -134,3 +136,147 @@ class Restated:
         return self._call(np.float64, lambda e: O.sap_gcr(self.L, bs, isolv, nmr, ncy, self.eoflg, self.U, self.sw,
                                                           self.sw.astype(np.float32), self.swi.astype(np.float32),
                                                           nkv, nmx, istop, res, mu, e), eta)
+
+    # --------------------------------------------------------------- deflation
+    # Little vectors: Ns numbers per block, the blocks of colour 0 first, each
+    # colour in lexicographic order (modules/block/blk_grid.c:20-32).
+    def dfl_init(self, bs, Ns, nkv=16, nmx=256, res=1e-2, nmx_gcr=24, res_gcr=1e-2, kappa=0.125, mu=0.0,
+                 ninv=5, nmr=4, ncy=4):
+        n = self._x // np.array(bs).reshape(4, 1)
+        nb = [l // b for l, b in zip(self.L, bs)]
+        lex = np.ravel_multi_index(n, nb)
+        nbl = int(np.prod(nb))
+        colour = np.indices(nb).reshape(4, -1).sum(axis=0) & 1
+        order = np.lexsort((np.arange(nbl), colour))
+        place = np.empty(nbl, dtype=int)
+        place[order] = np.arange(nbl)
+        sites = np.argsort(place[lex], kind="stable")       # of block 0, of block 1, ...
+        self._blocks = sites.reshape(nbl, -1)
+        self.Ns, self.nbl, self.nv = Ns, nbl, Ns * nbl
+        self._little_of = None
+        return self.nv
+
+    def _by_block(self, s, dt=np.complex128):
+        """storage order -> [block, component of the block's sites]"""
+        f = np.asarray(s).reshape(self.vol, 24)[self.ipt()[self._blocks]]
+        return np.ascontiguousarray(f.reshape(self.nbl, -1)).view(np.complex64 if f.dtype == np.float32
+                                                                   else np.complex128).astype(dt)
+
+    def _from_block(self, f, dt):
+        out = np.empty((self.vol, 24), dtype=dt)
+        out[self.ipt()[self._blocks]] = np.ascontiguousarray(f).view(np.float64).reshape(self.nbl, -1, 24)
+        return out.reshape(-1)
+
+    def dfl_subspace(self, modes):
+        """the block orthonormal basis of the modes (dfl_subspace.c:171): Q of
+        their QR decomposition with a positive diagonal of R"""
+        M = np.stack([self._by_block(m) for m in modes], axis=-1)       # block, component, mode
+        Q, R = np.linalg.qr(M)
+        d = np.einsum("nll->nl", R)
+        self._Q = (Q * (d / np.abs(d))[:, None, :]).astype(np.complex64).astype(np.complex128)
+        self._little_of = None
+
+    def dfl_modes(self, seed):
+        """a subspace of random fields smoothed by one, two and three SAP cycles
+        (dfl_modes.c:283-300), without the inverse iteration"""
+        g = np.random.default_rng(seed)
+        modes = []
+        for _ in range(self.Ns):
+            m = (g.random(24 * self.vol) - 0.5).astype(np.float32)
+            for n in (1, 2, 3):
+                m = self.sap(0.0, 1, 4, n, np.zeros_like(m), m)[0]
+            modes.append(m)
+        self.dfl_subspace(modes)
+        return 0, [0, 0]
+
+    def dfl_get_basis(self, l):
+        return self._from_block(self._Q[:, :, l], np.float32)
+
+    def _restrict(self, s):
+        return np.einsum("ncl,nc->nl", self._Q.conj(), self._by_block(s)).reshape(-1)
+
+    def _prolong(self, v, dt):
+        return self._from_block(np.einsum("ncl,nl->nc", self._Q, v.reshape(self.nbl, self.Ns)), dt)
+
+    def dfl_s2vd(self, s):
+        return self._restrict(np.asarray(s, dtype=np.float32)).view(np.float64)
+
+    def dfl_vd2s(self, vd):
+        return self._prolong(np.ascontiguousarray(vd, dtype=np.float64).view(np.complex128), np.float32)
+
+    def _Aw(self, mu):
+        """the little operator as a matrix (Aw_ops.c:186): products of the basis
+        with Dw on it and with i gamma5"""
+        if self._little_of is None:
+            A, G = (np.empty((self.nv, self.nv), dtype=np.complex128) for _ in range(2))
+            e = np.zeros(self.nv, dtype=np.complex128)
+            g5 = np.repeat([1.0, -1.0], 12)
+            for j in range(self.nv):
+                e[:] = 0.0
+                e[j] = 1.0
+                b = self._prolong(e, np.float64)
+                A[:, j] = self._restrict(self.dirac_dble(0, 0.0, b))
+                G[:, j] = 1j * self._restrict((b.reshape(-1, 24) * g5).reshape(-1))
+            self._little_of = A, G
+        A, G = self._little_of
+        return A + mu * G
+
+    def little(self, which, mu, v, w=None):
+        """Aw, Awhat, Aweeinv, Awooinv, Awoe, Aweo (Aw_dble.c:122-361)"""
+        v = np.ascontiguousarray(v, dtype=np.float64).view(np.complex128)
+        w = np.zeros_like(v) if w is None else np.array(w, dtype=np.float64, copy=True).view(np.complex128)
+        A, h = self._Aw(mu), self.nv // 2
+        ee, oo = A[:h, :h].copy(), A[h:, h:].copy()
+        for M in (ee, oo):                     # the diagonal blocks; blocks of one colour do not touch
+            M[np.kron(np.eye(self.nbl // 2), np.ones((self.Ns, self.Ns))) == 0] = 0.0
+        if which == 0:
+            w = A @ v
+        elif which == 1:
+            w[:h] = v[:h] - np.linalg.solve(ee, A[:h, h:] @ np.linalg.solve(oo, A[h:, :h] @ v[:h]))
+        elif which == 2:
+            w[:h] = np.linalg.solve(ee, v[:h])
+        elif which == 3:
+            w[h:] = np.linalg.solve(oo, v[h:])
+        elif which == 4:
+            w[h:] = A[h:, :h] @ v[:h]
+        elif which == 5:
+            w[:h] -= A[:h, h:] @ v[h:]
+        else:
+            self.missing("little operator %d" % which)
+        return w.view(np.float64), 0
+
+    def little32(self, which, mu, v, w=None):
+        w = None if w is None else np.asarray(w, dtype=np.float64)
+        return self.little(which, mu, np.asarray(v, dtype=np.float64), w)[0].astype(np.float32)
+
+    def ltl_gcr(self, mu, eta):
+        """the solution itself; the steps it takes are not restated"""
+        e = np.ascontiguousarray(eta, dtype=np.float64).view(np.complex128)
+        return np.linalg.solve(self._Aw(mu), e).view(np.float64), 0.0, 0, [1, 1]
+
+    def dfl_sap_gcr(self, nkv, nmx, istop, res, mu, eta):
+        """GCR with the preconditioner of dfl_sap_gcr.c:212-241 (an exact little
+        solve), in double precision, restarted after nkv steps"""
+        bs, isolv, nmr, ncy = self.sap_parms
+        A = np.linalg.inv(self._Aw(mu))
+        psi, r = np.zeros_like(eta), np.array(eta)
+        tol, steps = res * np.linalg.norm(eta), 0
+        while np.linalg.norm(r) > tol and steps < nmx:
+            chi = []
+            while len(chi) < nkv and np.linalg.norm(r) > tol and steps < nmx:
+                p = self._prolong(A @ self._restrict(r), np.float64)
+                q = r - self.dirac_dble(0, mu, p)
+                d = self.sap(mu, isolv, nmr, ncy, np.zeros(q.size, np.float32), q.astype(np.float32))[0]
+                p = (p + d).view(np.complex128)
+                q = self.dirac_dble(0, mu, p.view(np.float64)).view(np.complex128)
+                for a, b in chi:
+                    z = np.vdot(b, q)
+                    p, q = p - z * a, q - z * b
+                n = np.linalg.norm(q)
+                p, q = p / n, q / n
+                z = np.vdot(q, r.view(np.complex128))
+                psi, r = psi + (z * p).view(np.float64), r - (z * q).view(np.float64)
+                chi.append((p, q))
+                steps += 1
+            r = eta - self.dirac_dble(0, mu, psi)
+        return psi, np.linalg.norm(r), 0 if np.linalg.norm(r) <= tol * 1.0001 else -1, [steps, 1, 0]

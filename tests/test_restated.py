@@ -66,9 +66,36 @@ def test_solver(r):
 
 def test_what_it_does_not_cover(r):
     with pytest.raises(NotImplementedError):
-        r.dfl_modes(1)
+        r.tmcg(1)
     with pytest.raises(NotImplementedError):
         r.init(isw=1)
+
+
+def test_deflation():
+    r = restated.Restated((8, 8, 8, 8))
+    r.init(csw=1.5, m0=-0.2)
+    r.gen_links(0.4, 5)
+    r.sw_term()
+    r.set_sap_parms((4, 4, 4, 4), 1, 4, 5)
+    nv = r.dfl_init((4, 4, 4, 4), 4)
+    assert nv == 64 and r.dfl_modes(7)[0] == 0
+    g = np.random.default_rng(1)
+    v = g.standard_normal(2 * nv)
+    assert np.abs(r.dfl_s2vd(r.dfl_vd2s(v)) - v).max() <= 1e-5          # an orthonormal block basis
+    # the little operator through fields, and the even-odd pieces through it
+    s = r._prolong(v.view(complex), np.float64)
+    assert np.allclose(r.little(0, 0.03, v)[0], r._restrict(r.dirac_dble(0, 0.03, s)).view(float), rtol=0, atol=1e-12)
+    w = r.little(5, 0.03, v, r.little(0, 0.03, v)[0])[0][:nv]           # Aee v_e
+    assert np.allclose(r.little(2, 0.03, np.concatenate([w, v[nv:]]))[0][:nv], v[:nv], rtol=0, atol=1e-10)
+    x = r.little(1, 0.03, v)[0][:nv]
+    y = r.little(3, 0.03, r.little(4, 0.03, v)[0])[0]
+    z = r.little(2, 0.03, r.little(5, 0.03, y)[0])[0][:nv]              # -Aee^-1 Aeo Aoo^-1 Aoe v_e
+    assert np.allclose(x, v[:nv] + z, rtol=0, atol=1e-12)
+    assert np.allclose(r.little(0, 0.03, r.ltl_gcr(0.03, v)[0])[0], v, rtol=0, atol=1e-10)
+    eta = r.random_sd(3)
+    psi, rho, ifail, status = r.dfl_sap_gcr(16, 64, 0, 1e-10, 0.0, eta)
+    assert ifail == 0 and status[0] < r.sap_gcr(16, 64, 0, 1e-10, 0.0, eta)[3] + 2
+    assert np.linalg.norm(eta - r.dirac_dble(0, 0.0, psi)) <= 1.0001e-10 * np.linalg.norm(eta)
 
 
 class _Device:
@@ -100,7 +127,7 @@ def test_without_the_reference(monkeypatch):
     st = helpers.Setup((8, 8, 8, 8))
     assert st.vol == 4096 and st.ud.size == 4 * 4096 * 18 and st.source(1).size == 24 * 4096
     with pytest.raises(pytest.skip.Exception):
-        st.ref.dfl_modes(1)
+        st.ref.tmcg(1)
     ref.init(csw=1.5, m0=0.0)
     ref.gen_links(0.4, 1234)
     ref.sw_term()
