@@ -28,9 +28,10 @@ class Restated:
         return self.missing(name)
 
     def init(self, bc=3, seed=1234, csw=1.5, m0=0.0, eoflg=0, isw=0, theta=None):
-        if bc != 3 or isw != 0 or (theta is not None and np.any(theta)):
-            self.missing("boundary conditions other than type 3, exponential SW term or phase angles")
+        if bc != 3 or isw != 0:
+            self.missing("boundary conditions other than type 3 or exponential SW term")
         self.csw, self.m0, self.eoflg = csw, m0, eoflg
+        self.theta = (0.0, 0.0, 0.0) if theta is None else theta
 
     def set_sw_parms(self, m0):
         self.m0 = m0
@@ -56,7 +57,8 @@ class Restated:
     def gen_links(self, eps, seed):
         """U = exp(eps X), X distributed as by random_alg
         (modules/linalg/liealg.c:41-65); bc type 3 flips the sign of the time
-        links of the last plane (modules/uflds/uflds.c:307-335)"""
+        links of the last plane (modules/uflds/uflds.c:307-335), and phase
+        angles multiply U(x,k) by exp(i theta[k-1] / N[k]) (uflds.c:249-300)"""
         g = np.random.default_rng(seed).standard_normal((8, self.vol, 4)) / np.sqrt(2.0)
         a, b = (np.sqrt(3.0) + 1.0) / 6.0, (np.sqrt(3.0) - 1.0) / 6.0
         x1, x2 = a * g[0] + b * g[1], a * g[1] + b * g[0]
@@ -69,6 +71,8 @@ class Restated:
         w, v = np.linalg.eigh(-1j * eps * X)
         U = (v * np.exp(1j * w)[..., None, :]) @ v.conj().swapaxes(-1, -2)
         U[self._x[0] == self.L[0] - 1, 0] *= -1.0
+        for k in range(3):
+            U[:, k + 1] *= np.exp(1j * self.theta[k] / self.L[k + 1])
         self.U = np.ascontiguousarray(U).view(np.float64).reshape(-1)
 
     def ud(self):
@@ -101,9 +105,74 @@ class Restated:
         out[self.ipt()] = np.where(inv[:, None], self.swi.reshape(-1, 72), self.sw.reshape(-1, 72))
         return out.reshape(-1)
 
+    def plaq_sum(self):
+        """sum of Re tr of the plaquettes (modules/uflds/plaq_sum.c:161)"""
+        U = self.U.view(np.complex128).reshape(self.L + (4, 3, 3)).copy()
+        U[-1, :, :, :, 0] *= -1.0
+        for k in range(3):
+            U[..., k + 1, :, :] *= np.exp(-1j * self.theta[k] / self.L[k + 1])
+
+        def up(a, mu):
+            return np.roll(a, -1, axis=mu)
+        out = 0.0
+        for mu in range(4):
+            for nu in range(mu):
+                a, b = U[..., mu, :, :], U[..., nu, :, :]
+                out += np.einsum("...ij,...jk,...lk,...il", a, up(b, mu), up(a, nu).conj(), b.conj(), optimize=True).real.sum()
+        return out
+
     def random_sd(self, seed, sigma=1.0):
         """|s|^2 / sigma^2 distributed as by random_sd (modules/sflds/sflds.c)"""
         return np.random.default_rng(seed).standard_normal(24 * self.vol) * (sigma / np.sqrt(2.0))
+
+    # ------------------------------------------------------- sums and matrices
+    def spinor_prod_dble(self, s, r):
+        a, b = (np.asarray(x, dtype=np.longdouble).reshape(-1, 2) for x in (s, r))
+        z = (np.sum(a * b), np.sum(a[:, 0] * b[:, 1] - a[:, 1] * b[:, 0]))
+        return np.array([f(x) for x in z for f in (float, lambda x: float(x - np.longdouble(float(x))))])
+
+    def norm_square_dble(self, s):
+        return self.spinor_prod_dble(s, s)[:2]
+
+    def spinor_prod(self, s, r):
+        return self.spinor_prod_dble(s, r)[::2].astype(np.float32)
+
+    def norm_square(self, s):
+        return np.float32(self.norm_square_dble(s)[0])
+
+    @staticmethod
+    def _pauli(m):
+        """packed 6x6 matrices (modules/sw_term/pauli.c:953) -> full ones"""
+        m = np.asarray(m, dtype=np.float64).reshape(-1, 36)
+        out = np.zeros((len(m), 6, 6), dtype=np.complex128)
+        out[:, range(6), range(6)] = m[:, :6]
+        for k, (i, j) in enumerate((i, j) for i in range(6) for j in range(i + 1, 6)):
+            out[:, i, j] = m[:, 6 + 2 * k] + 1j * m[:, 7 + 2 * k]
+            out[:, j, i] = out[:, i, j].conj()
+        return out
+
+    def _sw_matrices(self, vol, mu, m):
+        out = self._pauli(m)[:2 * vol]
+        out[0::2, range(6), range(6)] += 1j * mu
+        out[1::2, range(6), range(6)] -= 1j * mu
+        return out
+
+    def apply_sw_dble(self, vol, mu, m, s):
+        s = np.ascontiguousarray(s, dtype=np.float64)
+        w = s.view(np.complex128).reshape(-1, 6)[:2 * vol]
+        return np.einsum("nij,nj->ni", self._sw_matrices(vol, mu, m), w).reshape(-1).view(np.float64)
+
+    def apply_sw(self, vol, mu, m, s):
+        return self.apply_sw_dble(vol, mu, m, s).astype(np.float32)
+
+    def apply_swinv_dble(self, vol, mu, m, s):
+        """and whether the Frobenius condition number of any matrix exceeds 100
+        (modules/sw_term/pauli_dble.c:55-59)"""
+        A = self._sw_matrices(vol, mu, m)
+        inv = np.linalg.inv(A)
+        w = np.ascontiguousarray(s, dtype=np.float64).view(np.complex128).reshape(-1, 6)[:2 * vol]
+        cond = np.linalg.norm(A, axis=(1, 2)) * np.linalg.norm(inv, axis=(1, 2))
+        return np.einsum("nij,nj->ni", inv, w).reshape(-1).view(np.float64), int(cond.max() > 100.0)
 
     # --------------------------------------------------------------- operators
     def _call(self, dt, f, *fields):

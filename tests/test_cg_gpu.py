@@ -64,6 +64,35 @@ def test_tmcg_zero_source(setup):
     assert rho == 0.0 and f == 0 and not psi.any()
 
 
+@pytest.mark.parametrize("bs", [(4, 4, 4, 4), (2, 4, 4, 2)], ids=["4x4x4x4", "2x4x4x2"])
+def test_true_residuals(setup, bs):
+    """the three solvers by their residuals alone, also on blocks that do not
+    fill the operators' warps"""
+    eta = setup.source(23)
+    n = setup.vol // 2 * 24
+    try:
+        qb.geometry(L, bs, setup.ipt)
+        qb.set_parms(1.5, -0.1, 0)
+        qb.upload_ud(setup.ud)
+        assert qb.upload_swd(setup.swd) == 0
+        psi, rho, f, st = qb.tmcg(2000, 0, 1e-10, 0.05, eta)
+        r = np.linalg.norm(eta - normal_op(setup, 0.05, psi))
+        assert f == 0 and st > 10 and r <= 1.05e-10 * np.linalg.norm(eta) and abs(r - rho) <= 1e-2 * r
+        psi, rho, f, st = qb.tmcg(2000, 0, 1e-10, 0.02, eta, eo=True)
+        r = np.linalg.norm((eta - normal_eo(setup, 0.02, psi))[:n])
+        assert f == 0 and st > 10 and r <= 1.05e-10 * np.linalg.norm(eta[:n]) and abs(r - rho) <= 1e-2 * r
+        mus = [0.05, 0.0, 0.2]
+        ps, f, st = qb.tmcgm(2000, 0, [1e-10] * 3, mus, eta)
+        assert f == 0
+        for mu, p in zip(mus, ps):
+            assert np.linalg.norm((eta - normal_eo(setup, mu, p))[:n]) <= 1.05e-10 * np.linalg.norm(eta[:n])
+    finally:
+        qb.geometry(L, (4, 4, 4, 4), setup.ipt)
+        qb.set_parms(1.5, -0.1, 0)
+        qb.upload_ud(setup.ud)
+        qb.upload_swd(setup.swd)
+
+
 # ------------------------------------------------------------ multi-shift CG
 def normal_eo(setup, mu, psi):
     """(Dwhat(mu)^dag Dwhat(mu) psi) on the even sites, with the reference

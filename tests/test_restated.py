@@ -57,6 +57,31 @@ def test_inverted_sw_term(r):
     r.sw_term(0)
 
 
+def test_sums_and_matrices(r):
+    s, t = r.random_sd(1), r.random_sd(2)
+    z = r.spinor_prod_dble(s, t)
+    assert abs(z[0] + 1j * z[2] - np.vdot(s.view(complex), t.view(complex))) <= 1e-12 * abs(np.vdot(s, s))
+    # Dwee + Dwoo on all sites is the SW term
+    d = r.dirac_dble(1, 0.2, s)
+    h = 12 * r.vol
+    assert np.allclose(r.apply_sw_dble(r.vol, 0.2, r.swd(), s)[:h], d[:h], rtol=0, atol=1e-13)
+    w = r.apply_sw_dble(r.vol, 0.2, r.swd(), s)
+    assert np.allclose(r.apply_swinv_dble(r.vol, 0.2, r.swd(), w)[0], s, rtol=0, atol=1e-12)
+    # 1 - <Re tr U_p> / 3 = 4 x 2 eps^2 / 3 up to O(eps^4) for independent links
+    assert abs(1.0 - r.plaq_sum() / (18 * r.vol) - 8 * 0.3 ** 2 / 3) <= 0.06
+
+
+def test_phase_angles():
+    """the SW term and the plaquette do not see them, the links do"""
+    a, b = (restated.Restated((4, 4, 4, 4)) for _ in range(2))
+    for x, theta in ((a, None), (b, (0.5, -0.8, 1.3))):
+        x.init(csw=1.5, m0=0.0, theta=theta)
+        x.gen_links(0.3, 5)
+        x.sw_term()
+    assert np.abs(a.U - b.U).max() > 0.1
+    assert np.abs(a.sw - b.sw).max() <= 1e-13 and abs(a.plaq_sum() - b.plaq_sum()) <= 1e-10
+
+
 def test_solver(r):
     r.set_sap_parms((4, 4, 4, 4), 1, 4, 3)
     eta = r.random_sd(3)
