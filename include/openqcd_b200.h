@@ -271,9 +271,9 @@ int b200_set_dw_staged(int mode);
  * keeps the fastest and returns it. */
 int b200_set_block_order(int kind);
 /* Fix the launch variant of the even-odd SAP block kernel for the current
- * block size (the index of the autotuner's candidate list, 0..4), so that
+ * block size (the index of the autotuner's candidate list, 0..5), so that
  * separate runs use the same arithmetic; -1 lets the autotuner choose again.
- * 0 and 4 are refused for blocks of more than 512 and 640 sites; 1 to 3 stand
+ * 0, 4 and 5 are refused for blocks of more than 512, 640 and 256 sites; 1 to 3 stand
  * for the variant of the largest blocks where their own is too small (no
  * reference counterpart). */
 int b200_set_sap_variant(int variant);

@@ -163,12 +163,12 @@ struct Ctx {
   void *u16 = nullptr, *sw16 = nullptr, *sw16_inv = nullptr;
   bool h16_valid = false;
   // SAP block-kernel launch variant chosen by the autotuner, per storage mode
-  // (0: FP32, 1: FP16, 2: FP32 with 12-real links) and size of launch (0: one
-  // CTA per SM at most, 1: more), for the block size it was tuned on
+  // (0: FP32, 1: FP16, 2: FP32 with 12-real links) and size of launch (one CTA
+  // per SM at most, two, more), for the block size it was tuned on
   struct SapTuned {
     int variant = 0, vbh = 0;
     float ms = 0.0f;
-  } sap_tuned[3][2];
+  } sap_tuned[3][3];
   // 12-real FP32 links for the SAP block solver (first two rows; the third
   // is rebuilt), used when every link passes the SU(3) check
   int sap_link12 = 1;

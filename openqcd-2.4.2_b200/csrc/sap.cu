@@ -737,6 +737,7 @@ static int pick_threads(int vbh, int &ns) {
 //   3   512 (128)              130            987        -             666           364
 //   1   768 (80)                80            797       132            -             -
 //   2   320 (96, two CTAs/SM)  111            941       379            -             -
+//   2   128 (128, four CTAs/SM)  for launches of three and more CTAs per SM (below)
 // Few blocks leave one CTA to an SM: what counts is a lane's chain, and
 // registers shorten it; many blocks want warps.  A block shared by a cluster
 // of 2, 4 or 8 CTAs, each writing its sites into the others' shared memory,
@@ -750,7 +751,7 @@ struct EoVariant {
    k_sap_blocks_eo<NS, EoTwoRow, SapF32, MAXT, MINB>}
 static const EoVariant kEo[] = {
     {1, 512, EO_KERNELS(1, 512, 1)}, {1, 256, EO_KERNELS(1, 256, 1)}, {3, 512, EO_KERNELS(3, 512, 1)},
-    {1, 768, EO_KERNELS(1, 768, 1)}, {2, 320, EO_KERNELS(2, 320, 2)},
+    {1, 768, EO_KERNELS(1, 768, 1)}, {2, 320, EO_KERNELS(2, 320, 2)}, {2, 128, EO_KERNELS(2, 128, 4)},
 };
 static const int kNEo = sizeof(kEo) / sizeof(kEo[0]);
 static const int kEoLarge = 2;   // the variant for every block that the shared memory holds
@@ -861,12 +862,16 @@ static int sap_mode(Ctx &c, int isolv, cudaStream_t st) {
   return c.u12_ok ? 2 : 0;
 }
 
-// The choice for launches of nsys systems.  One CTA per SM at most, or more:
-// with several systems the first can become the second, and the variant that
-// wins one (one CTA of 230 registers per lane on an SM) loses the other: six GCR steps of
-// four systems on 16^4 with 4^4 blocks 9.24 ms with the one-system choice,
-// 8.11 ms with its own; on 24^2x16x8 with 4x6x8x4 blocks 11.77 and 10.61 ms.
-static Ctx::SapTuned &sap_tuned(Ctx &c, int mode, int nsys) { return c.sap_tuned[mode][c.g.nbl / 2 * nsys > 148]; }
+// The choice for launches of nsys systems: at most one CTA per SM, at most two,
+// or more.  Several systems make a larger launch, where another variant wins.
+// Six GCR steps on 16^4 with 4^4 blocks, ms: one system (128 CTAs) 2.37 with one
+// CTA of 230 registers per lane on an SM, 2.60 with two of 128; two systems (256
+// CTAs) 4.53 and 4.09, and 4.54 with four of two sites per lane pair; four (512)
+// 9.19, 8.09 and 7.74.
+static Ctx::SapTuned &sap_tuned(Ctx &c, int mode, int nsys) {
+  const int n = c.g.nbl / 2 * nsys;
+  return c.sap_tuned[mode][n <= 148 ? 0 : n <= 2 * 148 ? 1 : 2];
+}
 
 static void launch_eo(const Ctx &c, const SapArgs &a, int variant, int mode, cudaStream_t st) {
   const EoVariant &v = kEo[variant];

@@ -65,8 +65,8 @@ def test_choice_by_launch_size(qb, L, nr, many, graphs):
 
 
 # sites per parity of the blocks, variants that do not fit them
-REFUSED = [((4, 4, 4, 4), []), ((4, 4, 8, 4), []), ((4, 4, 6, 6), [0]), ((4, 8, 4, 6), [0, 4]), ((6, 6, 6, 6), [0, 4]),
-           ((8, 8, 4, 6), [0, 4])]
+REFUSED = [((4, 4, 4, 4), []), ((4, 4, 8, 4), [5]), ((4, 4, 6, 6), [0, 5]), ((4, 8, 4, 6), [0, 4, 5]),
+           ((6, 6, 6, 6), [0, 4, 5]), ((8, 8, 4, 6), [0, 4, 5])]
 
 
 @pytest.mark.parametrize("bs,refused", REFUSED, ids=["x".join(map(str, b)) for b, _ in REFUSED])
@@ -80,7 +80,7 @@ def test_fixed_variants(qb, bs, refused):
     qb.sw_term()
     qb.set_sap_parms(bs, 1, 4, 2)
     x = [qb.DevField(32) for _ in range(2)]
-    for v in range(5):
+    for v in range(6):
         if v in refused:
             with pytest.raises(qb.B200Error):
                 qb.set_sap_variant(v)
@@ -89,4 +89,4 @@ def test_fixed_variants(qb, bs, refused):
         qb.dev_sap(0.0, 1, 4, 1, *x)
         assert qb.sap_tuning(12)[1] >= 32 * ((bs[0] * bs[1] * bs[2] * bs[3] // 2 + 47) // 48)
     with pytest.raises(qb.B200Error):
-        qb.set_sap_variant(5)
+        qb.set_sap_variant(6)

@@ -38,11 +38,11 @@ def test_sap_blocks(L, bs):
     for _ in range(2):
         psi, rho = O.sap(L, bs, MU, 1, 3, 0, U, sw[0], sw[1], psi, rho)
     half = int(np.prod(bs)) // 2
-    refused = [v for v, most in ((0, 256), (4, 320)) if half > most] + [5]
+    refused = [v for v, most in ((0, 256), (4, 320), (5, 128)) if half > most] + [6]
     try:
         for l12 in (1, 0):
             qb.set_sap_link12(l12)
-            for v in range(-1, 6):
+            for v in range(-1, 7):
                 if v in refused:
                     with pytest.raises(qb.B200Error):
                         qb.set_sap_variant(v)
